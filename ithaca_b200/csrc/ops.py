@@ -79,6 +79,10 @@ _SIGNATURES = {
     "ik_gemm_bf16_mma_batched": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, ctypes.c_longlong, ctypes.c_longlong, ctypes.c_longlong, _vp],
     "ik_gemm_bf16_mma": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _vp],
     "ik_gemm_tcgen05": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _i, _vp, _vp],
+    "ik_gemm_wide": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _i, _vp, _vp],
+    "ik_gemm_wide_grouped": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp],
+    "ik_gemm_qkv_rope_wide": [_vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp],
+    "ik_gemm_wide_take_wait_record": [_vp],
     "ik_gemm_tcgen05_tile": [_i],
     "ik_gemm_tcgen05_tile_width": [_i, _i],
     "ik_gemm_tcgen05_stream_k_bytes": [],
@@ -477,6 +481,15 @@ def tcgen05_splits(M: int, N: int, K: int) -> int:
     return 1
 
 
+def wide_takes(M: int, N: int, K: int) -> bool:
+    """Whether a product runs on pairs of SMs (gemm_wide.cu) instead of one tile per SM (gemm_tcgen05.cu).  It needs about half
+    the pairs busy with its narrowest tiles of 256 tokens x 128 features.  Measured on B200, other kernel / this one
+    (us): 36 tiles' worth and more: 4096 x 4096 at 300 tokens 20.0 / 19.1, 28672 x 4096 at 200 80 / 60, 16384 x 2048 at
+    130 29 / 23, 4096 x 14336 at 512 67 / 58, 2048 x 8192 at 768 34 / 32; below: 6144 x 4096 at 130 17.5 / 20.1, 4096 x 14336 at 256
+    49 / 57, 2048 x 8192 at 512 27.5 / 30.5.  Up to 128 tokens the other kernel's slices of K win."""
+    return M > 128 and M * N >= 36 * 256 * 128
+
+
 _pairs_lib = None
 PAIRS = os.environ.get("IK_PAIRS", "1") != "0"
 
@@ -501,9 +514,13 @@ def pairs_lib():
 def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, out_dtype=torch.float32,
                  accumulate: bool = False, splits: Optional[int] = None,
                  status: Optional[torch.Tensor] = None, swiglu: bool = False, pairs: Optional[bool] = None,
-                 glu=None, act: Optional[str] = None) -> Optional[torch.Tensor]:
+                 glu=None, act: Optional[str] = None, wide: Optional[bool] = None, wide_tile: int = 0) -> Optional[torch.Tensor]:
     """bfloat16 operands on the tcgen05 tensor cores (TMA-fed, accumulators in TMEM).  Returns None
     when the kernel does not take these sizes (K not a multiple of 8, unaligned rows).
+
+    Which kernel: ``wide`` = the one of gemm_wide.cu (two SMs to a tile of 256 tokens; where it does not take the call, the others
+    do), None = where ``wide_takes`` says so and neither ``splits`` nor ``pairs`` asks for another; ``pairs`` = the pair mode of
+    gemm_tcgen05.cu, None = for more than 256 tokens.  ``wide_tile``: features of a tile (128, 192, 256; 0 = chosen).
 
     ``w`` is a weight: launched early, the kernel asks for its first tiles of ``w`` before it waits for the
     kernel before it in the stream, so ``w`` must not be what that kernel writes (``x`` and ``out`` may be)."""
@@ -523,12 +540,19 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] =
     _need(out, "out", contiguous=False)
     if out.shape != (M, n_out) or out.stride(1) != 1:
         raise KernelError("gemm: the output has the wrong shape")
-    if splits is None:
-        splits = tcgen05_splits(M, N, K)
     # ``glu`` = (alpha, limit, shift): the gate with parameters; ``act``: an ungated activation on every result
     join = (2 if glu is not None else 1) if swiglu else _act_code(act, swiglu)
     tag = (' +swiglu' if swiglu else '') + (' +' + act if act else '')
     ga, gl, gs = glu if glu is not None else (1.0, 0.0, 0.0)
+    if wide or (wide is None and splits is None and pairs is None and wide_takes(M, N, K)):
+        _work(f"gemm_wide{tag} {M}x{N}x{K}", 2 * (M * K + N * K) + M * n_out * out.element_size(), 2 * M * N * K)
+        st = lib().ik_gemm_wide(_ptr(x), _ptr(w), _ptr(out), _code(out), M, N, K, x.stride(0), w.stride(0), out.stride(0),
+                                1 if accumulate else 0, join, ga, gl, gs, wide_tile, _ptr(status), _stream())
+        if st != -2:
+            _check(st, "gemm_wide")
+            return out
+    if splits is None:
+        splits = tcgen05_splits(M, N, K)
     if splits == 1 and M > 256 and pairs is not False:
         pl = pairs_lib()
         if pl is None and pairs:
@@ -601,6 +625,11 @@ def gemm_qkv_rope(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, k_pages
         st = lib().ik_gemm_qkv_rope_mma(_ptr(x), _ptr(w), M, N, K, x.stride(0), w.stride(0), ctypes.byref(rs), _stream())
         kernels = 1
     else:
+        if splits is None and wide_takes(M, N, K):
+            st = lib().ik_gemm_qkv_rope_wide(_ptr(x), _ptr(w), M, N, K, x.stride(0), w.stride(0), 0, _ptr(status), ctypes.byref(rs), _stream())
+            if st != -2:
+                _check(st, "gemm_qkv_rope (wide)")
+                return True
         if splits is None:
             splits = tcgen05_splits(M, N, K)
         pl = pairs_lib() if splits == 1 and M > 256 else None
@@ -922,6 +951,13 @@ def gemm_tcgen05_grouped(x: torch.Tensor, w: torch.Tensor, plan: MoEPaddedPlan, 
     used = min(M, plan.rows)
     _work(f"gemm_tcgen05 grouped{' +swiglu' if swiglu else ''} {used}x{N}x{K}", 2 * (used * K + min(plan.n_experts, plan.n_tiles) * N * K) + used * n_out * out.element_size(),
           2 * used * N * K)
+    if plan.bn in (128, 256):
+        st = lib().ik_gemm_wide_grouped(_ptr(x), _ptr(w), _ptr(out), _code(out), _ptr(plan.tile_group), plan.n_experts, plan.bn,
+                                        M, N, K, x.stride(0), w.stride(0), out.stride(0), 1 if swiglu else _act_code(act),
+                                        _ptr(status), _stream())
+        if st != -2:
+            _check(st, "gemm_wide_grouped")
+            return out
     st = lib().ik_gemm_tcgen05_grouped(_ptr(x), _ptr(w), _ptr(out), _code(out), _ptr(plan.tile_group), plan.n_experts, plan.bn,
                                        M, N, K, x.stride(0), w.stride(0), out.stride(0), 1 if swiglu else _act_code(act),
                                        _ptr(status), _stream())
@@ -962,7 +998,7 @@ def wait_records() -> str:
     error message, empty if none did."""
     found = []
     rec = (ctypes.c_int * 4)()
-    takers = [("matrix product", lib().ik_gemm_tcgen05_take_wait_record), ("state-space duality", lib().ik_ssd_take_wait_record)]
+    takers = [("matrix product", lib().ik_gemm_tcgen05_take_wait_record), ("matrix product (wide)", lib().ik_gemm_wide_take_wait_record), ("state-space duality", lib().ik_ssd_take_wait_record)]
     from . import attention_bf16
     for hd, m in attention_bf16._modules.items():
         takers.append((f"attention (head size {hd})", m.ik_attn_take_wait_record))
