@@ -430,72 +430,82 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
 
+    // The two issuing warps stay together and elect the lane that issues (see elect_one).
+    auto wait_all = [&](uint64_t* bar, uint32_t parity, int site, int i) {
+        return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, IK_WAIT_LIMIT_NS, site, i)) != 0;
+    };
     if (warp == 0) {
-        if (lane == 0) {
+        auto load_page = [&](unsigned char* dst, const CUtensorMap* map, int row, uint64_t* bar, uint32_t bytes) {
+            mbar_expect_tx(bar, bytes);
+            for (int bx = 0; bx < TC_BOXES; bx++) tma_load_2d(dst + bx * (PAGE * 128), map, bx * 64, row, bar);
+        };
+        if (elect_one()) {
             mbar_expect_tx(q_full, TC_Q_BYTES);
             for (int bx = 0; bx < TC_BOXES; bx++)
                 tma_load_2d(Qs + bx * (TC_BM * 128), &map_q, h * HD + bx * 64, q_begin + row0, q_full);
-            auto page_row = [&](int i) -> int {
-                int page = table[(size_t)b * table_stride + page_at(i, n_kept, p_lo)];
-                if (page < 0 || page >= n_pages) { ik_set_status(status, IK_STATUS_READ_NO_PAGE); page = 0; }
-                return (page * nkv + kvh) * PAGE;
-            };
-            // rows that are keys and values: one ring, a stage is free once O += P V has read it
-            for (int i = 0; ONE_ROW && i < n_iter; i++) {
-                const int s = i % TC_NS;
-                if (!mbar_wait(k_free + s, ((i / TC_NS) & 1) ^ 1, abort_flag, status, IK_WAIT_LIMIT_NS, 11, i)) break;
-                const int row = page_row(i);
-                mbar_expect_tx(k_full + s, TC_KV_BYTES + PAGE * 4);
-                for (int bx = 0; bx < TC_BOXES; bx++)
-                    tma_load_2d(Ks + s * TC_KV_BYTES + bx * (PAGE * 128), &map_k, bx * 64, row, k_full + s);
+        }
+        __syncwarp();
+        auto page_row = [&](int i) -> int {
+            int page = table[(size_t)b * table_stride + page_at(i, n_kept, p_lo)];
+            if (page < 0 || page >= n_pages) { ik_set_status(status, IK_STATUS_READ_NO_PAGE); page = 0; }
+            return (page * nkv + kvh) * PAGE;
+        };
+        // rows that are keys and values: one ring, a stage is free once O += P V has read it
+        for (int i = 0; ONE_ROW && i < n_iter; i++) {
+            const int s = i % TC_NS;
+            if (!wait_all(k_free + s, ((i / TC_NS) & 1) ^ 1, 11, i)) break;
+            const int row = page_row(i);
+            if (elect_one()) {
+                load_page(Ks + s * TC_KV_BYTES, &map_k, row, k_full + s, TC_KV_BYTES + PAGE * 4);
                 bulk_load(Cs + s * PAGE, key_scales + row, PAGE * 4, k_full + s);
             }
-            // keys of page i, then values of page i - 1
-            for (int i = 0; !ONE_ROW && i <= n_iter; i++) {
-                if (i < n_iter) {
-                    const int s = i % TC_NS;
-                    if (!mbar_wait(k_free + s, ((i / TC_NS) & 1) ^ 1, abort_flag, status, IK_WAIT_LIMIT_NS, 11, i)) break;
-                    const int row = page_row(i);
-                    mbar_expect_tx(k_full + s, TC_KV_BYTES);
-                    for (int bx = 0; bx < TC_BOXES; bx++)
-                        tma_load_2d(Ks + s * TC_KV_BYTES + bx * (PAGE * 128), &map_k, bx * 64, row, k_full + s);
-                }
-                if (i > 0) {
-                    const int s = (i - 1) % TC_NS;
-                    if (!mbar_wait(v_free + s, (((i - 1) / TC_NS) & 1) ^ 1, abort_flag, status, IK_WAIT_LIMIT_NS, 12, i)) break;
-                    const int row = page_row(i - 1);
-                    mbar_expect_tx(v_full + s, TC_KV_BYTES);
-                    for (int bx = 0; bx < TC_BOXES; bx++)
-                        tma_load_2d(Vs + s * TC_KV_BYTES + bx * (PAGE * 128), &map_v, bx * 64, row, v_full + s);
-                }
+            __syncwarp();
+        }
+        // keys of page i, then values of page i - 1
+        for (int i = 0, row = 0, row_before = 0; !ONE_ROW && i <= n_iter; i++, row_before = row) {
+            if (i < n_iter) {
+                const int s = i % TC_NS;
+                if (!wait_all(k_free + s, ((i / TC_NS) & 1) ^ 1, 11, i)) break;
+                row = page_row(i);
+                if (elect_one()) load_page(Ks + s * TC_KV_BYTES, &map_k, row, k_full + s, TC_KV_BYTES);
+                __syncwarp();
+            }
+            if (i > 0) {
+                const int s = (i - 1) % TC_NS;
+                if (!wait_all(v_free + s, (((i - 1) / TC_NS) & 1) ^ 1, 12, i)) break;
+                if (elect_one()) load_page(Vs + s * TC_KV_BYTES, &map_v, row_before, v_full + s, TC_KV_BYTES);
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc_qk = umma_idesc(PAGE), idesc_pv = umma_idesc(HD, 1);
-            const uint32_t q_addr = smem_u32(Qs);
-            bool ok = mbar_wait(q_full, 0, abort_flag, status, IK_WAIT_LIMIT_NS, 13, 0);
-            auto issue_qk = [&](int i) -> bool {
-                const int s = i % TC_NS;
-                if (!mbar_wait(k_full + s, (i / TC_NS) & 1, abort_flag, status, IK_WAIT_LIMIT_NS, 14, i)) return false;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t k_addr = smem_u32(Ks + s * TC_KV_BYTES);
+        const uint32_t idesc_qk = umma_idesc(PAGE), idesc_pv = umma_idesc(HD, 1);
+        const uint32_t q_addr = smem_u32(Qs);
+        bool ok = wait_all(q_full, 0, 13, 0);
+        auto issue_qk = [&](int i) -> bool {
+            const int s = i % TC_NS;
+            if (!wait_all(k_full + s, (i / TC_NS) & 1, 14, i)) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t k_addr = smem_u32(Ks + s * TC_KV_BYTES);
+            if (elect_one()) {
                 #pragma unroll
                 for (int j = 0; j < HD / 16; j++)
                     umma(tmem + (i & 1) * PAGE, umma_desc(q_addr + (j / 4) * (TC_BM * 128) + (j % 4) * 32),
                          umma_desc(k_addr + (j / 4) * (PAGE * 128) + (j % 4) * 32), idesc_qk, j != 0);
                 umma_commit(s_full + (i & 1));
                 if (!ONE_ROW) umma_commit(k_free + s);     // the key stage is free once these products have read it
-                return true;
-            };
-            if (ok) ok = issue_qk(0);
-            for (int i = 0; i < n_iter && ok; i++) {
-                if (i + 1 < n_iter) { ok = issue_qk(i + 1); if (!ok) break; }     // runs while page i is in the softmax
-                const int s = i % TC_NS;
-                ok = mbar_wait(p_ready + (i & 1), (i >> 1) & 1, abort_flag, status, IK_WAIT_LIMIT_NS, 15, i) && (ONE_ROW || mbar_wait(v_full + s, (i / TC_NS) & 1, abort_flag, status, IK_WAIT_LIMIT_NS, 16, i));
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t v_addr = smem_u32(Vs + s * TC_KV_BYTES);
+            }
+            __syncwarp();
+            return true;
+        };
+        if (ok) ok = issue_qk(0);
+        for (int i = 0; i < n_iter && ok; i++) {
+            if (i + 1 < n_iter) { ok = issue_qk(i + 1); if (!ok) break; }     // runs while page i is in the softmax
+            const int s = i % TC_NS;
+            ok = wait_all(p_ready + (i & 1), (i >> 1) & 1, 15, i) && (ONE_ROW || wait_all(v_full + s, (i / TC_NS) & 1, 16, i));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t v_addr = smem_u32(Vs + s * TC_KV_BYTES);
+            if (elect_one()) {
                 #pragma unroll
                 for (int j = 0; j < PAGE / 16; j++)
                     umma_ts(tmem + TC_O_COL, tmem + (i & 1) * PAGE + j * 8, umma_desc_mn(v_addr + j * 2048, PAGE * 128),
@@ -503,8 +513,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 umma_commit(ONE_ROW ? k_free + s : v_free + s);
                 umma_commit(pv_done);
             }
-            if (ok) umma_commit(o_done);
+            __syncwarp();
         }
+        if (ok && elect_one()) umma_commit(o_done);
+        __syncwarp();
     } else {
         const int quarter = warp & 3, r = quarter * 32 + lane;
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);

@@ -309,17 +309,22 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     float* const pieces = stream_k ? partial + SK_FLAG_INTS : nullptr;  // stream-K: [block][BN][128] raw sums of a piece
 
     if (warp == 0) {
-        if (lane == 0) {
-            int it = 0, armed = 0;
-            bool ok = true;
-            Walk walk = walk_init;
-            for (Work w; ok && walk.next(w);) {
-                const int n0 = w.nt * BM + w.group * N, m0 = w.mt * bn, kb0 = w.kb0, nkb = w.nkb;       // n0: the weight tile's first row in W
-                for (int i = 0; i < nkb; i += KSUB, it++) {
-                    const int s = it % NST, n_sub = min(KSUB, nkb - i);
-                    unsigned char* a = tiles + s * STAGE;
-                    if (it >= pre_issued) {             // the first stages are armed and their weights asked for already
-                        if (!mbar_wait(empty + s, ((it / NST) & 1) ^ 1, abort_flag, status, IK_WAIT_LIMIT_NS, 1, it)) { ok = false; break; }
+        // The two issuing roles keep their warp together and elect a lane where they issue (see elect_one).
+        int it = 0;
+        bool ok = true;
+        const int n_pre = __shfl_sync(0xffffffffu, pre_issued, 0);
+        Walk walk = walk_init;
+        for (Work w; ok && walk.next(w);) {
+            const int n0 = w.nt * BM + w.group * N, m0 = w.mt * bn, kb0 = w.kb0, nkb = w.nkb;       // n0: the weight tile's first row in W
+            for (int i = 0; i < nkb; i += KSUB, it++) {
+                const int s = it % NST, n_sub = min(KSUB, nkb - i);
+                unsigned char* a = tiles + s * STAGE;
+                if (it >= n_pre) {                      // the first stages are armed and their weights asked for already
+                    ok = __all_sync(0xffffffffu, mbar_wait(empty + s, ((it / NST) & 1) ^ 1, abort_flag, status, IK_WAIT_LIMIT_NS, 1, it));
+                    if (!ok) break;
+                }
+                if (elect_one()) {
+                    if (it >= n_pre) {
                         mbar_expect_tx(full + s, n_sub * block_bytes);
                         for (int sub = 0; sub < n_sub; sub++)
                             tma_load_2d(a + sub * C::A_BYTES, &map_w, (kb0 + i + sub) * BK, n0, full + s);
@@ -332,40 +337,39 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                         for (int sub = 0; sub < n_sub; sub++)
                             tma_load_2d(a + KSUB * C::A_BYTES + sub * C::B_BYTES, &map_x, (kb0 + i + sub) * BK, m0, full + s);
                     }
-                    armed = it + 1;
                 }
+                __syncwarp();
             }
-            if (*abort_flag) {
-                // leave no copy of this block in flight: wait (bounded) for the stages that were armed last
-                for (int i = max(0, armed - NST); i < armed; i++) {
-                    const long long c0 = wait_clock();
-                    while (!mbar_test(full + i % NST, (i / NST) & 1) && !wait_ran_out(c0, 2000000ull)) {}
-                }
+        }
+        if (*abort_flag && lane == 0) {
+            // leave no copy of this block in flight: wait (bounded) for the stages that were armed last
+            for (int i = max(0, it - NST); i < it; i++) {
+                const long long c0 = wait_clock();
+                while (!mbar_test(full + i % NST, (i / NST) & 1) && !wait_ran_out(c0, 2000000ull)) {}
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // With the loads compiled out, a K block of four products and a commit takes this thread 0.27-0.3 us whether
-            // the token tile is 64, 128 or 256 wide (see MODE 3 above), so what it does besides is kept short: stage and
-            // phase are counted, not divided, and the descriptors are one addition away.
-            const uint32_t idesc = umma_idesc(bn), desc_hi = umma_desc_hi(), a_lo0 = umma_desc_lo(smem_u32(tiles));
-            int it = 0, lt = 0, s = 0;                     // s = it % NST, phase = (it / NST) & 1
-            uint32_t phase = 0;
-            bool ok = true;
-            Walk walk = walk_init;
-            for (Work w; ok && walk.next(w); lt++) {
-                const int nkb = w.nkb;
-                const int buf = lt & 1;
-                ok = mbar_wait(acc_empty + buf, ((lt >> 1) & 1) ^ 1, abort_flag, status, IK_WAIT_LIMIT_NS, 2, lt);   // drained by the epilogue
+        // What the issuing thread does besides is kept short: stage and phase are counted, not divided, and the descriptors
+        // are one addition away.
+        const uint32_t idesc = umma_idesc(bn), desc_hi = umma_desc_hi(), a_lo0 = umma_desc_lo(smem_u32(tiles));
+        int it = 0, lt = 0, s = 0;                     // s = it % NST, phase = (it / NST) & 1
+        uint32_t phase = 0;
+        bool ok = true;
+        Walk walk = walk_init;
+        for (Work w; ok && walk.next(w); lt++) {
+            const int nkb = w.nkb;
+            const int buf = lt & 1;
+            ok = __all_sync(0xffffffffu, mbar_wait(acc_empty + buf, ((lt >> 1) & 1) ^ 1, abort_flag, status, IK_WAIT_LIMIT_NS, 2, lt));   // drained by the epilogue
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t acc = tmem_base + buf * C::ACC_COLS;
+            for (int i = 0; i < nkb; i += KSUB, it++, s = s + 1 == NST ? 0 : s + 1, phase ^= (uint32_t)(s == 0)) {
+                ok = __all_sync(0xffffffffu, mbar_wait(full + s, phase, abort_flag, status, IK_WAIT_LIMIT_NS, 3, it));
                 if (!ok) break;
+                if (it == 0 && lane == 0) IK_STAMP(3);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t acc = tmem_base + buf * C::ACC_COLS;
-                for (int i = 0; i < nkb; i += KSUB, it++, s = s + 1 == NST ? 0 : s + 1, phase ^= (uint32_t)(s == 0)) {
-                    ok = mbar_wait(full + s, phase, abort_flag, status, IK_WAIT_LIMIT_NS, 3, it);
-                    if (!ok) break;
-                    if (it == 0) IK_STAMP(3);
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a_lo = a_lo0 + (uint32_t)s * (STAGE >> 4), b_lo = a_lo + ((KSUB * C::A_BYTES) >> 4);
+                const uint32_t a_lo = a_lo0 + (uint32_t)s * (STAGE >> 4), b_lo = a_lo + ((KSUB * C::A_BYTES) >> 4);
+                if (elect_one()) {
                     #pragma unroll
                     for (int sub = 0; sub < KSUB; sub++) {
                         if (sub > 0 && i + sub >= nkb) break;      // an odd number of K blocks: the last stage holds one
@@ -377,9 +381,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     if (PAIRS) umma_commit_pair(empty + s);    // ... in both blocks, whose copies fill each other's stages
                     else umma_commit(empty + s);             // the stage is free once these MMAs have read it
                 }
-                if (ok) umma_commit(acc_full + buf);
-                IK_STAMP(4);
+                __syncwarp();
             }
+            if (ok && elect_one()) umma_commit(acc_full + buf);
+            __syncwarp();
+            if (lane == 0) IK_STAMP(4);
         }
     } else {
         // epilogue: warp w owns TMEM lanes 32 * (w % 4) .. + 31
