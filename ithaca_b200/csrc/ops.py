@@ -123,7 +123,8 @@ _SIGNATURES = {
     "ik_scale_softcap": [_vp, _u64, _f, _f, _vp],
     "ik_glu_act": [_vp, _vp, _i, _i, _i, _i, _f, _f, _f, _vp],
     "ik_causal_conv": [_vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
-    "ik_selective_scan": [_vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
+    "ik_selective_scan": [_vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp],
+    "ik_selective_scan_scratch": [_i, _i, _i, _i, _i, _i, _i],
     "ik_ssd": [_i, _vp, _i, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
     "ik_ssd_tcgen05": [_vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp],
     "ik_ssd_take_wait_record": [_vp],
@@ -258,6 +259,7 @@ def lib():
             fn = getattr(l, name)
             fn.argtypes = sig
             fn.restype = _i
+        l.ik_selective_scan_scratch.restype = ctypes.c_longlong
         _lib = l
     return timed(_lib)
 
@@ -1195,10 +1197,14 @@ def selective_scan(u: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[torc
     out = torch.empty((T, inner), dtype=out_dtype, device=u.device)
     _work(f"selective_scan {T}x{inner}x{N}", T * inner * (u.element_size() + 8 + out.element_size()) + 8 * ctx.n_seqs * inner * N,
           9 * T * inner * N)
+    max_new = getattr(ctx, "max_new", 0)                  # a caller that does not say gets every sequence token by token
+    need = lib().ik_selective_scan_scratch(_code(u), T, ctx.n_seqs, max_new, inner, N, 1 if ctx.is_decode else 0)
+    scratch = torch.empty(need, dtype=torch.float32, device=u.device) if need else None
     st = lib().ik_selective_scan(_ptr(u), _code(u), _ptr(dt_raw), _ptr(dt_bias), _ptr(A), _ptr(bc), bc.stride(0), b_off, c_off,
                                  _ptr(D), _ptr(z), ldz, _ptr(state), _ptr(ctx.slots), _ptr(ctx.cu_seqlens), _ptr(ctx.kv_lens),
-                                 _ptr(out), _code(out), T, ctx.n_seqs, inner, N, 1 if ctx.is_decode else 0, _stream())
-    _check(st, "selective_scan")
+                                 _ptr(out), _code(out), T, ctx.n_seqs, inner, N, 1 if ctx.is_decode else 0, max_new, _ptr(scratch),
+                                 _stream())
+    _check(st, "selective_scan", kernels=3 if need else 1)
     return out
 
 

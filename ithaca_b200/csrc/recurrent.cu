@@ -254,13 +254,29 @@ template <bool FAST> __device__ __forceinline__ float ik_scan_step(float S, floa
     return (float)fma(exp((double)dt * (double)a), (double)S, (double)dt * (double)x * (double)B);
 }
 
-template <typename TU, typename TO, bool FAST, int NPT, int L, int TT>
+// Prompts of the 16-bit path are cut into pieces of `piece` tokens that run side by side (token by token a prompt is a chain:
+// with one sequence there are hardly two warps a scheduler, each waiting for itself).  MODE 1 runs every piece but a sequence's
+// last from a zero state and leaves its end state and the sum of its step sizes in scratch; scan_carry_kernel turns the end
+// states into the pieces' states at entry, S <- exp(a * sum dt) S + S_piece; MODE 2 runs the pieces from there and writes the
+// results.  MODE 0: whole sequences.  Pieces have flat numbers: piece j of sequence b is cu_seqlens[b] / piece + b + j, of
+// which there are at most T / piece + B.
+// Measured on B200: a scan layer 2,048 wide (4,096 channels of 16 states) over two prompts of 3,000 and fewer tokens 1,411 -> 646 us,
+// 765 us of it in this kernel's place; what bounds the pieces is the exponential (one per state and token in either pass).
+struct ScanPieces {
+    int piece;                                        // tokens; 0 = whole sequences
+    int n_seqs;
+    float* states;                                    // [flat piece][inner][N]: end states, then states at entry
+    float* sums;                                      // [flat piece][inner]: sums of the step sizes
+};
+__device__ __forceinline__ int scan_piece_base(const int* cu_seqlens, int b, int piece) { return cu_seqlens[b] / piece + b; }
+
+template <typename TU, typename TO, bool FAST, int NPT, int L, int TT, int MODE>
 __global__ void __launch_bounds__(128)
 selective_scan_kernel(const TU* __restrict__ u, const float* __restrict__ dt_raw, const float* __restrict__ dt_bias,
                       const float* __restrict__ A, const float* __restrict__ bc, int ldbc, int b_off, int c_off,
                       const float* __restrict__ Dv, const float* __restrict__ z, int ldz, float* __restrict__ state,
                       const int* __restrict__ slots, const int* __restrict__ cu_seqlens, const int* __restrict__ kv_lens,
-                      TO* __restrict__ out, int inner, int N) {
+                      TO* __restrict__ out, int inner, int N, ScanPieces pieces) {
     constexpr int CH = 128 / L, NPAD = L * NPT, W = 3 * CH + 2 * NPAD, PER_TILE = TT * W;
     constexpr int KX = (TT * CH + 127) / 128, KB = (TT * 2 * NPAD + 127) / 128;      // staged values a thread
     extern __shared__ __align__(16) float sm[];      // [2][TT][W]: x, dt, silu(z) per channel; B (padded), C (padded)
@@ -273,13 +289,25 @@ selective_scan_kernel(const TU* __restrict__ u, const float* __restrict__ dt_raw
     IK_AFTER_WAIT(cu_seqlens);
     IK_AFTER_WAIT(kv_lens);
     ik_pdl_launch_dependents();
-    const int b = blockIdx.y;
+    int b = blockIdx.y;
+    if (MODE != 0) {                                         // the sequence of this flat piece: the last whose first piece is not behind it
+        int low = 0, high = pieces.n_seqs - 1;
+        while (low < high) {
+            const int mid = (low + high + 1) >> 1;
+            if (scan_piece_base(cu_seqlens, mid, pieces.piece) <= (int)blockIdx.y) low = mid;
+            else high = mid - 1;
+        }
+        b = low;
+    }
     const int l = threadIdx.x & (L - 1), ch = threadIdx.x / L;
     const int c0 = blockIdx.x * CH, c = c0 + ch;
     const bool live = c < inner;
     const int cc = live ? c : inner - 1;                     // idle lanes follow along (the shuffles need them)
-    const int lo = cu_seqlens[b], hi = cu_seqlens[b + 1], end = kv_lens[b], start = end - (hi - lo);
-    if (hi <= lo) return;
+    const int seq_lo = cu_seqlens[b], seq_hi = cu_seqlens[b + 1], end = kv_lens[b], start = end - (seq_hi - seq_lo);
+    const int lo = MODE == 0 ? seq_lo : seq_lo + ((int)blockIdx.y - scan_piece_base(cu_seqlens, b, pieces.piece)) * pieces.piece;
+    const int hi = MODE == 0 ? seq_hi : min(seq_hi, lo + pieces.piece);
+    if (hi <= lo || (MODE == 1 && hi == seq_hi)) return;
+    float* const carried = MODE == 0 ? nullptr : pieces.states + ((size_t)blockIdx.y * inner + cc) * N;
     float* st_in = state + ((size_t)slots[b] * 2 + ((start - 1) & 1)) * inner * N + (size_t)cc * N;
     float* st_out = state + ((size_t)slots[b] * 2 + ((end - 1) & 1)) * inner * N + (size_t)cc * N;
     float S[NPT], a[NPT];
@@ -287,8 +315,10 @@ selective_scan_kernel(const TU* __restrict__ u, const float* __restrict__ dt_raw
     for (int r = 0; r < NPT; r++) {
         const int n = l * NPT + r;
         a[r] = n < N ? A[(size_t)cc * N + n] : 0.f;
-        S[r] = (n < N && start > 0) ? st_in[n] : 0.f;
+        if (MODE == 0) S[r] = (n < N && start > 0) ? st_in[n] : 0.f;
+        else S[r] = MODE == 2 && n < N ? carried[n] : 0.f;
     }
+    float dt_sum = 0.f;
     const float dskip = Dv ? Dv[cc] : 0.f;
     typename IkRaw<TU>::type rx[KX];
     float rd[KX], rz[KX], rb[KB], bias_k[KX];
@@ -307,7 +337,7 @@ selective_scan_kernel(const TU* __restrict__ u, const float* __restrict__ dt_raw
             if (tt < TT && col < inner) {
                 rx[k] = ik_ld_now(u + (size_t)t * inner + col);
                 rd[k] = ik_ld_now(dt_raw + (size_t)t * inner + col);
-                if (z) rz[k] = ik_ld_now(z + (size_t)t * ldz + col);
+                if (MODE != 1 && z) rz[k] = ik_ld_now(z + (size_t)t * ldz + col);
             }
         }
         #pragma unroll
@@ -315,7 +345,7 @@ selective_scan_kernel(const TU* __restrict__ u, const float* __restrict__ dt_raw
             const int e = threadIdx.x + k * 128, tt = e / (2 * NPAD), n2 = e % (2 * NPAD), n = n2 % NPAD;
             const int t = min(t0 + tt, hi - 1);
             rb[k] = 0.f;
-            if (tt < TT && n < N) rb[k] = ik_ld_now(bc + (size_t)t * ldbc + (n2 < NPAD ? b_off : c_off) + n);
+            if (tt < TT && n < N && (MODE != 1 || n2 < NPAD)) rb[k] = ik_ld_now(bc + (size_t)t * ldbc + (n2 < NPAD ? b_off : c_off) + n);
         }
     };
     auto store = [&](int buf) {
@@ -326,7 +356,7 @@ selective_scan_kernel(const TU* __restrict__ u, const float* __restrict__ dt_raw
             if (tt < TT) {
                 tile[tt * W + w] = ik_raw_float(rx[k]);
                 tile[tt * W + CH + w] = ik_softplus_as<FAST>(rd[k] + bias_k[k]);
-                tile[tt * W + 2 * CH + w] = ik_silu_as<FAST>(rz[k]);
+                if (MODE != 1) tile[tt * W + 2 * CH + w] = ik_silu_as<FAST>(rz[k]);
             }
         }
         #pragma unroll
@@ -368,20 +398,40 @@ selective_scan_kernel(const TU* __restrict__ u, const float* __restrict__ dt_raw
                 #pragma unroll
                 for (int r = 0; r < NPT; r++) {
                     S[r] = ik_scan_step<FAST>(S[r], dt, x, a[r], bv[r]);
+                    if (MODE == 1) continue;
                     if (r & 1) a1 = fmaf(S[r], cv[r], a1);
                     else a0 = fmaf(S[r], cv[r], a0);
                 }
+                if (MODE == 1) dt_sum += dt;
             }
             acc[tt] = a0 + a1;
         }
+        // Sums over a channel's lanes, L tokens at a time: each exchange halves what a lane still holds, so that lane i ends with
+        // token i's sum (the same additions as a butterfly per token, a quarter of the shuffles) and finishes that token.
+        constexpr int GRP = TT % L == 0 ? L : 1;
         #pragma unroll
-        for (int tt = 0; tt < TT; tt++) {
-            float v = acc[tt];
+        for (int t4 = 0; MODE != 1 && t4 < TT; t4 += GRP) {
+            float v[GRP];
             #pragma unroll
-            for (int o = L >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (l == 0 && live && tt < n_here) {
+            for (int i = 0; i < GRP; i++) v[i] = acc[t4 + i];
+            if (GRP == L) {
+                #pragma unroll
+                for (int o = L >> 1; o > 0; o >>= 1) {
+                    const bool upper = l & o;
+                    #pragma unroll
+                    for (int i = 0; i < o; i++) {
+                        const float theirs = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[(i + o) % GRP], o);
+                        v[i] = (upper ? v[(i + o) % GRP] : v[i]) + theirs;
+                    }
+                }
+            } else {
+                #pragma unroll
+                for (int o = L >> 1; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+            }
+            const int tt = GRP == L ? t4 + l : t4;
+            if ((GRP == L || l == 0) && live && tt < n_here) {
                 const float* row = tile + tt * W;
-                float y = fmaf(dskip, row[ch], v);
+                float y = fmaf(dskip, row[ch], v[0]);
                 if (z) y *= row[2 * CH + ch];
                 ik_st(out, (size_t)(t0 + tt) * inner + c, y);
             }
@@ -389,11 +439,42 @@ selective_scan_kernel(const TU* __restrict__ u, const float* __restrict__ dt_raw
         if (t0 + TT < hi) store(buf ^ 1);
         __syncthreads();
     }
-    if (live) {
+    if (live && (MODE != 2 || hi == seq_hi)) {
         #pragma unroll
         for (int r = 0; r < NPT; r++) {
             const int n = l * NPT + r;
-            if (n < N) st_out[n] = S[r];
+            if (n < N) (MODE == 1 ? carried : st_out)[n] = S[r];
+        }
+        if (MODE == 1 && l == 0) pieces.sums[(size_t)blockIdx.y * inner + c] = dt_sum;
+    }
+}
+
+// The states with which a sequence's pieces begin, one thread per channel and state.
+__global__ void __launch_bounds__(256)
+scan_carry_kernel(const float* __restrict__ A, const float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ cu_seqlens,
+                  const int* __restrict__ kv_lens, int inner, int N, ScanPieces pieces) {
+    ik_pdl_wait();
+    ik_pdl_launch_dependents();
+    const int b = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x, all = inner * N;
+    if (i >= all) return;
+    const int n_new = cu_seqlens[b + 1] - cu_seqlens[b], start = kv_lens[b] - n_new, f0 = scan_piece_base(cu_seqlens, b, pieces.piece);
+    const int n = (n_new + pieces.piece - 1) / pieces.piece, c = i / N;
+    const float a = A[i];
+    float S = start > 0 && n > 0 ? state[((size_t)slots[b] * 2 + ((start - 1) & 1)) * all + i] : 0.f;
+    float* mine = pieces.states + (size_t)f0 * all + i;
+    const float* sums = pieces.sums + (size_t)f0 * inner + c;
+    for (int j0 = 0; j0 < n; j0 += 8) {                      // eight pieces' loads in flight together
+        float own[8], sum[8];
+        #pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const bool has = j0 + j + 1 < n;                 // the last piece leaves nothing
+            own[j] = has ? mine[(size_t)(j0 + j) * all] : 0.f;
+            sum[j] = has ? sums[(size_t)(j0 + j) * inner] : 0.f;
+        }
+        #pragma unroll
+        for (int j = 0; j < 8; j++) {
+            if (j0 + j < n) mine[(size_t)(j0 + j) * all] = S;
+            S = fmaf(__expf(a * sum[j]), S, own[j]);
         }
     }
 }
@@ -450,25 +531,57 @@ selective_scan_decode_kernel(const TU* __restrict__ u, const float* __restrict__
     }
 }
 
+// Tokens of a piece, 0 = whole sequences: pieces pay where the longest sequence is several of them.  As long as about
+// twelve blocks an SM come together (each piece costs scratch), of 64 to 512 tokens.  A grid's second dimension ends at 65,535.
+static int scan_piece_tokens(int T, int B, int max_new, int inner, int N) {
+    if (N > 64 || max_new < 192) return 0;
+    int piece = 512;
+    const long long across = (inner + 31) / 32;
+    while (piece > 64 && across * (T / piece) < 12LL * ik_sm_count()) piece /= 2;
+    return max_new >= 3 * piece && T / piece + B <= 65535 ? piece : 0;
+}
+
 template <typename TU, typename TO, bool FAST>
 static int launch_scan(const void* u, const float* dt_raw, const float* dt_bias, const float* A, const float* bc, int ldbc, int b_off,
                        int c_off, const float* Dv, const float* z, int ldz, float* state, const int* slots, const int* cu_seqlens,
-                       const int* kv_lens, void* out, int B, int inner, int N, int one_token_each, cudaStream_t stream) {
+                       const int* kv_lens, void* out, int T, int B, int inner, int N, int one_token_each, int max_new, float* scratch,
+                       cudaStream_t stream) {
     // four states a thread (eight from 65 states on), as many lanes a channel as that takes, tiles as long as a thread's
     // staging registers allow
+#define IK_SCAN_AT(NPT, L, TT, MODE, ROWS)                                                                                      \
+    IK_RETURN_IF_ERROR(ik_launch(selective_scan_kernel<TU, TO, FAST, NPT, L, TT, MODE>, dim3((inner + 128 / (L) - 1) / (128 / (L)), ROWS), 128, \
+                                 (size_t)2 * (TT) * (3 * (128 / (L)) + 2 * (L) * (NPT)) * sizeof(float), stream,                \
+                                 (const TU*)u, dt_raw, dt_bias, A, bc, ldbc, b_off, c_off, Dv, z, ldz, state, slots, cu_seqlens,  \
+                                 kv_lens, (TO*)out, inner, N, pieces))
 #define IK_SCAN(NPT, L, TT)                                                                                                     \
     do {                                                                                                                        \
-        constexpr int CH = 128 / (L), W = 3 * CH + 2 * (L) * (NPT);                                                             \
-        const dim3 grid((inner + CH - 1) / CH, B);                                                                              \
         if (one_token_each)                                                                                                     \
-            IK_RETURN_IF_ERROR(ik_launch(selective_scan_decode_kernel<TU, TO, FAST, NPT, L>, grid, 128, 0, stream, (const TU*)u, dt_raw,   \
+            IK_RETURN_IF_ERROR(ik_launch(selective_scan_decode_kernel<TU, TO, FAST, NPT, L>, dim3((inner + 128 / (L) - 1) / (128 / (L)), B), 128, 0, stream, (const TU*)u, dt_raw,   \
                                          dt_bias, A, bc, ldbc, b_off, c_off, Dv, z, ldz, state, slots, cu_seqlens, kv_lens, (TO*)out,    \
                                          inner, N));                                                                            \
-        else                                                                                                                    \
-        IK_RETURN_IF_ERROR(ik_launch(selective_scan_kernel<TU, TO, FAST, NPT, L, TT>, grid, 128, (size_t)2 * (TT) * W * sizeof(float), stream, \
-                                     (const TU*)u, dt_raw, dt_bias, A, bc, ldbc, b_off, c_off, Dv, z, ldz, state, slots, cu_seqlens,  \
-                                     kv_lens, (TO*)out, inner, N));                                                             \
+        else IK_SCAN_AT(NPT, L, TT, 0, B);                                                                                      \
     } while (0)
+#define IK_SCAN_PIECES(NPT, L, TT)                                                                                              \
+    do {                                                                                                                        \
+        const int rows = T / pieces.piece + B;                                                                                  \
+        IK_SCAN_AT(NPT, L, TT, 1, rows);                                                                                        \
+        IK_RETURN_IF_ERROR(ik_launch(scan_carry_kernel, dim3((inner * N + 255) / 256, B), 256, 0, stream, A, (const float*)state, slots, \
+                                     cu_seqlens, kv_lens, inner, N, pieces));                                                   \
+        IK_SCAN_AT(NPT, L, TT, 2, rows);                                                                                        \
+    } while (0)
+    ScanPieces pieces = {0, B, nullptr, nullptr};
+    if constexpr (FAST) {
+        const int piece = one_token_each || !scratch ? 0 : scan_piece_tokens(T, B, max_new, inner, N);
+        if (piece > 0) {
+            pieces.piece = piece;
+            pieces.states = scratch;
+            pieces.sums = scratch + (size_t)(T / piece + B) * inner * N;
+            if (N <= 16) IK_SCAN_PIECES(4, 4, 16);
+            else if (N <= 32) IK_SCAN_PIECES(4, 8, 16);
+            else IK_SCAN_PIECES(4, 16, 16);
+            IK_LAUNCH_STATUS();
+        }
+    }
     // up to 16 states, 16-bit path: two states a thread while four would leave the SMs with fewer than two warps a scheduler
     // (one 4,096-token prompt, 4,096 channels: 1.01 -> 0.88 ms).  The float32 path keeps one shape whatever the batch, so
     // that its sums never depend on what else a step brings.
@@ -484,14 +597,23 @@ static int launch_scan(const void* u, const float* dt_raw, const float* dt_bias,
     IK_LAUNCH_STATUS();
 }
 
+// Floats of scratch that ik_selective_scan wants for these sizes (0: none): bfloat16 inputs in several pieces.
+IK_EXPORT long long ik_selective_scan_scratch(int u_dtype, int T, int B, int max_new, int inner, int N, int one_token_each) {
+    if (u_dtype != IK_BF16 || one_token_each || T <= 0 || B <= 0) return 0;
+    const int piece = scan_piece_tokens(T, B, max_new, inner, N);
+    return piece ? (long long)(T / piece + B) * inner * (N + 1) : 0;
+}
+
+// scratch: ik_selective_scan_scratch floats, or null (every sequence is then run token by token).  max_new: the longest sequence's tokens.
 IK_EXPORT int ik_selective_scan(const void* u, int u_dtype, const float* dt_raw, const float* dt_bias, const float* A,
                                 const float* bc, int ldbc, int b_off, int c_off, const float* Dv, const float* z, int ldz,
                                 float* state, const int* slots, const int* cu_seqlens, const int* kv_lens, void* out,
-                                int out_dtype, int T, int B, int inner, int N, int one_token_each, cudaStream_t stream) {
+                                int out_dtype, int T, int B, int inner, int N, int one_token_each, int max_new, float* scratch,
+                                cudaStream_t stream) {
     if (T < 0 || B < 0 || inner <= 0 || N <= 0 || !state || b_off < 0 || c_off < 0 || ldbc < N) return IK_BAD_ARGUMENT;
     if (T == 0 || B == 0) return IK_OK;
     if (one_token_each && T != B) return IK_BAD_ARGUMENT;
-#define IK_ARGS u, dt_raw, dt_bias, A, bc, ldbc, b_off, c_off, Dv, z, ldz, state, slots, cu_seqlens, kv_lens, out, B, inner, N, one_token_each, stream
+#define IK_ARGS u, dt_raw, dt_bias, A, bc, ldbc, b_off, c_off, Dv, z, ldz, state, slots, cu_seqlens, kv_lens, out, T, B, inner, N, one_token_each, max_new, scratch, stream
     if (u_dtype == IK_F32 && out_dtype == IK_F32) return launch_scan<float, float, false>(IK_ARGS);
     if (u_dtype == IK_BF16 && out_dtype == IK_BF16) return launch_scan<__nv_bfloat16, __nv_bfloat16, true>(IK_ARGS);
     if (u_dtype == IK_F32 && out_dtype == IK_BF16) return launch_scan<float, __nv_bfloat16, false>(IK_ARGS);
