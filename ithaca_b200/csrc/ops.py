@@ -95,6 +95,8 @@ _SIGNATURES = {
     "ik_plain_act": [_vp, _vp, _i, _u64, _i, _vp],
     "ik_delta_prepare": [_vp, _i, _i, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _f, _f, _vp],
     "ik_delta_rule": [_vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
+    "ik_delta_chunks": [_vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
+    "ik_delta_chunks_scratch": [_i, _i, _i, _i, _i, _i],
     "ik_head_norm_gate": [_vp, _vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _f, _i, _i, _vp],
     "ik_latent_prepare": [_vp, _i, _i, _i, _vp, _f, _vp, _vp, _i, _vp, _i, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i,
                           _vp, _vp],
@@ -259,7 +261,7 @@ def lib():
             fn = getattr(l, name)
             fn.argtypes = sig
             fn.restype = _i
-        l.ik_selective_scan_scratch.restype = ctypes.c_longlong
+        l.ik_selective_scan_scratch.restype = l.ik_delta_chunks_scratch.restype = ctypes.c_longlong
         _lib = l
     return timed(_lib)
 
@@ -1401,10 +1403,13 @@ def delta_prepare(u: torch.Tensor, q_off: int, k_off: int, p: torch.Tensor, b_of
 
 
 def delta_rule(u: torch.Tensor, q_off: int, k_off: int, v_off: int, bg: torch.Tensor, state: torch.Tensor, ctx, n_heads: int,
-               n_qk_heads: int, dk: int, dv: int) -> torch.Tensor:
+               n_qk_heads: int, dk: int, dv: int, chunks: bool = False) -> torch.Tensor:
     """The gated delta rule over the step's tokens: per head S <- g S; u = b (v - S^T k); S <- S + k u^T; o = S^T q.  q, k
     (``n_qk_heads`` heads, unit vectors) and v are column ranges of ``u`` (float), ``bg`` [T, 2, heads] the steps and decays,
-    ``state`` [max_slots, 2, heads, dv, dk] float (column by column).  Returns float [T, heads * dv]."""
+    ``state`` [max_slots, 2, heads, dv, dk] float (column by column).  Returns float [T, heads * dv].
+
+    ``chunks``: prompts may run 64 tokens at a time (float all the same, but a token's sums then depend on where its chunk
+    begins, so a prompt cut otherwise does not give the same bits: for the 16-bit path)."""
     _need(u, "u", torch.float32)
     _need(bg, "bg", torch.float32)
     _need(state, "state", torch.float32)
@@ -1415,6 +1420,14 @@ def delta_rule(u: torch.Tensor, q_off: int, k_off: int, v_off: int, bg: torch.Te
     out = torch.empty((T, n_heads * dv), dtype=torch.float32, device=u.device)
     _work(f"delta_rule {T}x{n_heads}x{dk}x{dv}", T * (2 * n_qk_heads * dk + 2 * n_heads * dv) * 4 + 8 * ctx.n_seqs * n_heads * dk * dv,
           6 * T * n_heads * dk * dv)
+    need = lib().ik_delta_chunks_scratch(T, ctx.n_seqs, ctx.max_new, n_heads, dk, dv) if chunks and not ctx.is_decode else 0
+    if need:
+        scratch = torch.empty(need, dtype=torch.float32, device=u.device)
+        st = lib().ik_delta_chunks(_ptr(u), u.stride(0), q_off, k_off, v_off, _ptr(bg), _ptr(state), _ptr(ctx.slots), _ptr(ctx.cu_seqlens),
+                                   _ptr(ctx.kv_lens), _ptr(out), _ptr(scratch), T, ctx.n_seqs, n_heads, n_qk_heads, dk, dv, _stream())
+        if st != -2:
+            _check(st, "delta_chunks", kernels=2)
+            return out
     _check(lib().ik_delta_rule(_ptr(u), u.stride(0), q_off, k_off, v_off, _ptr(bg), _ptr(state), _ptr(ctx.slots), _ptr(ctx.cu_seqlens),
                                _ptr(ctx.kv_lens), _ptr(out), T, ctx.n_seqs, n_heads, n_qk_heads, dk, dv, 1 if ctx.is_decode else 0,
                                _stream()), "delta_rule")

@@ -130,7 +130,7 @@ class GatedDeltaRule:
         else:
             bg = ops.delta_prepare(u, 0, self.k_off, p, self.b_off, self.a_off, self.A_log, self.dt_bias, G, dk, H, dk ** -0.5,
                                    self.unit_eps)
-            o = ops.delta_rule(u, 0, self.k_off, self.v_off, bg, cache.state(STATE), ctx, H, G, dk, dv)
+            o = ops.delta_rule(u, 0, self.k_off, self.v_off, bg, cache.state(STATE), ctx, H, G, dk, dv, chunks=rt.dtype == "bfloat16")
         if self.lowrank_gate:
             gate = self.g2(ops.cast(p[:, self.g_off:self.g_off + self.gate_rank], rt.act_dtype), out_dtype=torch.float32)
             mid = ops.head_norm_gate(o, self.norm_w, self.norm_eps, gate, 0, H, rt.act_dtype, gate="sigmoid")

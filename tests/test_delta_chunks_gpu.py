@@ -1,0 +1,85 @@
+"""The gated delta rule of a prompt in chunks of 64 tokens, against float64 and the token-by-token kernel: sequences of several chunks,
+of one, of none, with and without an earlier state, lengths on and off the chunks' edges, decays near 0 and 1."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def make(H, G, dk, dv, new, start, seed, decay):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)
+    T, B = sum(new), len(new)
+    u = rnd(T, 4 + 2 * G * dk + H * dv)
+    for off, mult in ((4, dk ** -0.5), (4 + G * dk, 1.0)):
+        x = u[:, off:off + G * dk].view(T, G, dk)
+        u[:, off:off + G * dk] = (x * torch.rsqrt((x * x).sum(-1, keepdim=True) + 1e-6) * mult).view(T, -1)
+    bg = torch.sigmoid(rnd(T, 2, H))
+    bg[:, 1] = {"usual": 1 - 0.2 * bg[:, 1] ** 2, "near one": 1 - 1e-4 * bg[:, 1], "small": bg[:, 1] ** 8}[decay]
+    if decay == "small":
+        bg[::7, 1] = 0.0
+    state = rnd(B + 1, 2, H, dv, dk)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    cu = [sum(new[:i]) for i in range(B + 1)]
+    slots = list(range(B, 0, -1))
+    ctx = SimpleNamespace(n_seqs=B, max_new=max(new), slots=i32(slots), cu_seqlens=i32(cu), kv_lens=i32([a + b for a, b in zip(new, start)]),
+                          is_decode=False)
+    return u, bg.contiguous(), state, ctx, cu, slots
+
+
+def far(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30))
+
+
+@pytest.mark.parametrize("H,G,dk,dv", [(4, 2, 128, 128), (2, 2, 64, 64), (3, 1, 128, 36), (2, 1, 64, 20), (40, 8, 128, 128)])
+@pytest.mark.parametrize("new,start", [([200], [0]), ([3, 0, 129, 64, 63], [5, 0, 0, 12, 0])])
+@pytest.mark.parametrize("decay", ["usual", "near one", "small"])
+def test_delta_rule_in_chunks(H, G, dk, dv, new, start, decay):
+    from ithaca_b200.csrc import ops
+    u, bg, before, ctx, cu, slots = make(H, G, dk, dv, new, start, dk + dv, decay)
+    assert ops.lib().ik_delta_chunks_scratch(cu[-1], len(new), max(new), H, dk, dv) > 0
+    args = (4, 4 + G * dk, 4 + 2 * G * dk, bg)
+    state, state1 = before.clone(), before.clone()
+    o = ops.delta_rule(u, *args, state, ctx, H, G, dk, dv, chunks=True)
+    o1 = ops.delta_rule(u, *args, state1, ctx, H, G, dk, dv)
+    ud, bd = u.double(), bg.double()
+    for b, (n, first) in enumerate(zip(new, start)):
+        if n == 0:
+            assert torch.equal(state[slots[b]], before[slots[b]])
+            continue
+        S = before[slots[b], (first - 1) & 1].double() if first > 0 else torch.zeros(H, dv, dk, dtype=torch.float64, device=DEV)
+        want = []
+        for t in range(cu[b], cu[b + 1]):
+            q, k = (ud[t, off:off + G * dk].view(G, dk).repeat_interleave(H // G, 0) for off in (4, 4 + G * dk))
+            S = S * bd[t, 1][:, None, None]
+            x = bd[t, 0][:, None] * (ud[t, 4 + 2 * G * dk:].view(H, dv) - torch.einsum("hvk,hk->hv", S, k))
+            S = S + x[:, :, None] * k[:, None, :]
+            want.append(torch.einsum("hvk,hk->hv", S, q).reshape(-1))
+        rows, p = slice(cu[b], cu[b + 1]), (first + n - 1) & 1
+        want = torch.stack(want)
+        # float sums of at most dk + 64 products, carried on by the decays: as far off as token by token, give or take
+        assert far(o[rows], want) < max(1.5 * far(o1[rows], want), 1e-6) and far(o[rows], want) < 5e-6
+        assert far(state[slots[b], p], S) < max(1.5 * far(state1[slots[b], p], S), 1e-6)
+        if (first - 1) & 1 != p:
+            assert torch.equal(state[slots[b], 1 - p], before[slots[b], 1 - p])
+    assert torch.equal(state[0], before[0])
+
+
+@pytest.mark.parametrize("where", ["k", "v", "decay"])
+def test_what_is_not_finite_stays_behind_its_token(where):
+    from ithaca_b200.csrc import ops
+    H, G, dk, dv = 2, 1, 128, 64
+    u, bg, before, ctx, cu, slots = make(H, G, dk, dv, [150], [0], 3, "usual")
+    args = (4, 4 + G * dk, 4 + 2 * G * dk)
+    whole = ops.delta_rule(u, *args, bg, before.clone(), ctx, H, G, dk, dv, chunks=True)
+    bad_u, bad_bg = u.clone(), bg.clone()
+    if where == "decay":
+        bad_bg[101, 1] = float("nan")
+    else:
+        bad_u[101, 4 + G * dk if where == "k" else 4 + 2 * G * dk + 5] = float("inf") if where == "v" else float("nan")
+    got = ops.delta_rule(bad_u, *args, bad_bg, before.clone(), ctx, H, G, dk, dv, chunks=True)
+    assert torch.equal(got[:101], whole[:101])
+    assert not torch.isfinite(got[101]).all() and not torch.isfinite(got[149]).all()
