@@ -95,3 +95,46 @@ def attend(q: torch.Tensor, k_pages: torch.Tensor, ctx, table: torch.Tensor, n_h
                             int(window or 0), 1 if sink else 0, page_size, n_pages, chunk, n_splits, _ptr(status), _stream()),
            "attention latent", kernels=2 if n_splits > 1 else 1)
     return out
+
+
+PROMPT_KEYS_MOST = 1 << 17        # keys of a step whose heads' keys and values are formed: 8 or 16 KB each with 16 or 32 heads
+FORM_KEYS_QUERIES = 64
+
+
+def forms_keys(ctx, k_pages: torch.Tensor, dtype: torch.dtype, dk: int, dr: int, dv: int, rank: int) -> bool:
+    """Whether a step's attention goes over keys and values formed per head (``prompt``) rather than over the cached rows.  Forming
+    them costs heads x rank x (dk + dv) products a key; a query that sees the key then saves 2 rank - dk - dv of the 2 rank + dr
+    products per head (768 of 1,088), and runs on tcgen05.  Measured on B200 (rank 512, one sequence; us for the layer, over the rows /
+    formed): 16 heads, 64 new tokens behind 2,000 190 / 155, 512 behind 2,000 371 / 168, 4,096 from the start 2,056 / 348; 32 heads,
+    64 behind 2,000 228 / 183, 512 behind 2,000 674 / 245; below 64 not measured."""
+    if dtype != torch.bfloat16 or k_pages.dtype != torch.bfloat16 or ctx.is_decode or k_pages.shape[1:3] != (1, 64):
+        return False
+    if dk != 128 or dv != 128 or dr not in (0, 64) or rank % 64 or k_pages.shape[3] != rank + dr:
+        return False
+    lens, new = ctx.host_kv_lens, ctx.host_n_new
+    keys = sum(lens)
+    return len(lens) == ctx.n_seqs and keys <= PROMPT_KEYS_MOST and sum(n * e for n, e in zip(new, lens)) >= FORM_KEYS_QUERIES * keys
+
+
+def prompt(q_plain: torch.Tensor, q_full: torch.Tensor, k_pages: torch.Tensor, w_kv: torch.Tensor, ctx, table: torch.Tensor, n_heads: int,
+           rank: int, scale: float, window: int, status: Optional[torch.Tensor]) -> torch.Tensor:
+    """q_plain [T, heads * 128] and the turning parts in q_full [T, heads * (rank + dr)]; ``w_kv`` [2 * heads * 128, rank]: all heads'
+    key matrices, then their value matrices.  Returns the heads' results [T, heads * 128]."""
+    from . import gemm_bf16
+    n_pages, _, _, hd = k_pages.shape
+    T, B = q_plain.shape[0], ctx.n_seqs
+    n_keys = sum(-(-e // 64) * 64 for e in ctx.host_kv_lens)
+    lib = ops.lib()
+    latents = torch.empty((n_keys, rank), dtype=torch.bfloat16, device=q_plain.device)
+    ops._work(f"latent_gather {n_keys}x{rank}", 2 * ops._nbytes(latents))
+    _check(lib.ik_latent_gather(_ptr(k_pages), _ptr(ctx.kv_lens), _ptr(table), table.stride(0), _ptr(latents), B, ctx.max_kv_len, hd, rank, n_pages,
+                                _ptr(status), _stream()), "latent_gather")
+    kv = gemm_bf16.gemm(latents, w_kv, out_dtype=torch.bfloat16)
+    out = torch.empty((T, n_heads * 128), dtype=torch.bfloat16, device=q_plain.device)
+    if ops.profiling():
+        pairs = sum(min(p + 1, window) if window else p + 1 for n, e in zip(ctx.host_n_new, ctx.host_kv_lens) for p in range(e - n, e))
+        ops._work(f"attention latent prompt {T}x{n_heads}", ops._nbytes(q_plain, out, kv), 2 * pairs * n_heads * (256 + hd - rank))
+    _check(lib.ik_latent_prompt(_ptr(q_plain), _ptr(q_full), _ptr(kv), _ptr(k_pages), _ptr(out), _ptr(ctx.cu_seqlens), _ptr(ctx.kv_lens), _ptr(table),
+                                table.stride(0), T, B, ctx.max_new, n_keys, n_heads, hd, rank, scale, int(window or 0), n_pages, _ptr(status),
+                                _stream()), "attention latent prompt")
+    return out

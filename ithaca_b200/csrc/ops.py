@@ -100,6 +100,9 @@ _SIGNATURES = {
     "ik_head_norm_gate": [_vp, _vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _f, _i, _i, _vp],
     "ik_latent_prepare": [_vp, _i, _i, _i, _vp, _f, _vp, _vp, _i, _vp, _i, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i,
                           _vp, _vp],
+    "ik_latent_gather": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp, _vp],
+    "ik_latent_prompt": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp, _vp],
+    "ik_latent_prompt_take_wait_record": [_vp],
     "ik_layernorm": [_vp, _vp, _vp, _vp, _vp, _i, _vp, _f, _i, _i, _f, _vp],
     "ik_add": [_vp, _vp, _u64, _vp],
     "ik_conv_rope_append": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i,
@@ -1002,7 +1005,8 @@ def wait_records() -> str:
     error message, empty if none did."""
     found = []
     rec = (ctypes.c_int * 4)()
-    takers = [("matrix product", lib().ik_gemm_tcgen05_take_wait_record), ("matrix product (wide)", lib().ik_gemm_wide_take_wait_record), ("state-space duality", lib().ik_ssd_take_wait_record)]
+    takers = [("matrix product", lib().ik_gemm_tcgen05_take_wait_record), ("matrix product (wide)", lib().ik_gemm_wide_take_wait_record), ("state-space duality", lib().ik_ssd_take_wait_record),
+              ("latent attention of prompts", lib().ik_latent_prompt_take_wait_record)]
     from . import attention_bf16
     for hd, m in attention_bf16._modules.items():
         takers.append((f"attention (head size {hd})", m.ik_attn_take_wait_record))

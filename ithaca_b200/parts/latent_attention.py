@@ -7,10 +7,12 @@ position part (all ``rope_dim`` of them); the score is (q_plain . k_plain + q_tu
 window allows; ordinary softmax; the heads side by side times sigmoid(Wg x) (``head_gate: "wide"``) go through the output
 projection.
 
-Only [c | turned key part] is cached, as one key/value head of size kv_rank + rope_dim, and nothing else is ever formed
-for a cached token: q_plain is carried into the latent's space (Wuk^T q_plain, one small product per head), attention
+Only [c | turned key part] is cached, as one key/value head of size kv_rank + rope_dim, and in decode steps nothing else is
+formed for a cached token: q_plain is carried into the latent's space (Wuk^T q_plain, one small product per head), attention
 runs over the cached rows with the latent as key AND value, and the head's weighted sum of latents is brought to value
-space by Wuv (again one small product per head).  Prefill and decode run the same steps.
+space by Wuv (again one small product per head).  Steps with some hundred new tokens behind a key go the other way round on the
+16-bit path: the heads' plain keys and values are formed from the cached rows for the step, and attention runs over those
+(``attention_latent.forms_keys`` says when).
 
 A layer may read the rows that another layer of equal ``kv_rank``, ``rope_dim`` and rotation has written instead of
 making its own (the schedule gives it that layer's cache entry with ``writes_cache=False``): it then has no Wdkv and no
@@ -102,6 +104,8 @@ class LatentAttention:
         self.uv = uv.view(H, dv, rank).contiguous().to(wdt or uv.dtype)
         self.c_norm_w = as_float32(tensors[w["dkv_norm"]], runtime) if self.own_latent else None
         self.runtime = runtime
+        # prompts: one product forms every head's plain keys and values from the rows (see ``attention_latent.prompt``)
+        self.w_kv = torch.cat([uk.to(wdt), uv.to(wdt)], dim=0).contiguous() if wdt is not None and dk == dv == 128 else None
 
     def cache_requests(self) -> List[object]:
         # one key/value head whose rows are [latent | turned key part]; the values are the rows' leading kv_rank columns
@@ -126,6 +130,12 @@ class LatentAttention:
             q_plain = torch.empty((T, H * dk), dtype=rt.act_dtype, device=x.device)
             ops.latent_prepare(p, 0, self.c_off, self.c_norm_w, self.norm_eps, q_plain, q_full, cache.k_pages, ctx.token_seq,
                                ctx.token_pos, table, self.position.inv_freq if dr else None, H, dk, dr, rank, writes_cache, rt.status)
+        if self.w_kv is not None and attention_latent.forms_keys(ctx, cache.k_pages, rt.act_dtype, dk, dr, dv, rank):
+            heads = attention_latent.prompt(q_plain, q_full, cache.k_pages, self.w_kv, ctx, table, H, rank, self.scale, self.window or 0, rt.status)
+            if self.gate:
+                ops.head_gate(heads, p, self.g_off, heads, H, wide=True)
+            self.o(heads, out=residual, accumulate=accumulate)
+            return
         ops.gemm_heads(q_plain.view(T, H, dk), self.uk_t, q_full.view(T, H, hd)[:, :, :rank])
         # [T, H * rank]: the tensor-core kernel whose tile rows are the heads, or (32-bit, other sizes) the CUDA cores
         att = attention_latent.attend(q_full, cache.k_pages, ctx, table, H, self.scale, self.window or 0, rt.status, rank)
