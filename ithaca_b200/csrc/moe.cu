@@ -355,9 +355,16 @@ moe_sort_padded_kernel(const int* __restrict__ chosen, int* __restrict__ row_of,
     for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
     for (int r = threadIdx.x; r < n_tiles * bn; r += blockDim.x) src_token[r] = -1;
     __syncthreads();
-    for (int a = threadIdx.x; a < A; a += blockDim.x) {
-        const int e = chosen[a];
-        if (e >= 0 && e < E) atomicAdd(&cnt[e], 1);
+    // eight assignments a thread at a time, so that their loads are under way together (one at a time the block waited for
+    // memory twice per 1,024 assignments: 35 us for 16,384 of them on B200)
+    constexpr int AT = 8;
+    for (int a0 = threadIdx.x; a0 < A; a0 += AT * 1024) {
+        int e[AT];
+        #pragma unroll
+        for (int i = 0; i < AT; i++) e[i] = a0 + i * 1024 < A ? chosen[a0 + i * 1024] : -1;
+        #pragma unroll
+        for (int i = 0; i < AT; i++)
+            if (e[i] >= 0 && e[i] < E) atomicAdd(&cnt[e[i]], 1);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -369,30 +376,44 @@ moe_sort_padded_kernel(const int* __restrict__ chosen, int* __restrict__ row_of,
         for (; nt < n_tiles; nt++) tile_group[nt] = -1;
     }
     __syncthreads();
-    for (int a = threadIdx.x; a < A; a += blockDim.x) {
-        const int e = chosen[a];
-        if (e < 0 || e >= E) { row_of[a] = 0; continue; }
-        const int r = atomicAdd(&cur[e], 1);
-        row_of[a] = r;
-        if (r < n_tiles * bn) {
-            src_token[r] = a / top;
-            if (src_assign) src_assign[r] = a;            // (read only where src_token is not -1)
+    for (int a0 = threadIdx.x; a0 < A; a0 += AT * 1024) {
+        int e[AT];
+        #pragma unroll
+        for (int i = 0; i < AT; i++) e[i] = a0 + i * 1024 < A ? chosen[a0 + i * 1024] : -2;
+        #pragma unroll
+        for (int i = 0; i < AT; i++) {
+            const int a = a0 + i * 1024;
+            if (a >= A) break;
+            if (e[i] < 0 || e[i] >= E) { row_of[a] = 0; continue; }
+            const int r = atomicAdd(&cur[e[i]], 1);
+            row_of[a] = r;
+            if (r < n_tiles * bn) {
+                src_token[r] = a / top;
+                if (src_assign) src_assign[r] = a;            // (read only where src_token is not -1)
+            }
         }
     }
 }
 
 // xp[r, :] = x[src_token[r], :], zeros where src_token[r] < 0; rows of d bfloat16, d a multiple of 8
-__global__ void moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ src_token, uint4* __restrict__ xp,
-                                  int rows, int d8) {
+// Four rows a block: their tokens' numbers are read once, and four rows' loads are under way together.
+__global__ void __launch_bounds__(256)
+moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ src_token, uint4* __restrict__ xp, int rows, int d8) {
     ik_pdl_wait();
     IK_AFTER_WAIT(x);
     IK_AFTER_WAIT(src_token);
     ik_pdl_launch_dependents();
-    const size_t total = (size_t)rows * d8, stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {
-        const size_t r = idx / d8;
-        const int c = (int)(idx - r * d8), t = src_token[r];
-        xp[idx] = t >= 0 ? x[(size_t)t * d8 + c] : make_uint4(0u, 0u, 0u, 0u);
+    const int r0 = blockIdx.x * 4;
+    int t[4];
+    #pragma unroll
+    for (int i = 0; i < 4; i++) t[i] = r0 + i < rows ? src_token[r0 + i] : -1;
+    for (int c = threadIdx.x; c < d8; c += 256) {
+        uint4 v[4];
+        #pragma unroll
+        for (int i = 0; i < 4; i++) v[i] = t[i] >= 0 ? x[(size_t)t[i] * d8 + c] : make_uint4(0u, 0u, 0u, 0u);
+        #pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (r0 + i < rows) xp[(size_t)(r0 + i) * d8 + c] = v[i];
     }
 }
 
@@ -441,6 +462,51 @@ __global__ void moe_combine_kernel(const float* __restrict__ parts, const float*
         for (int k = 0; k < top; k++) acc = fmaf(weight ? weight[t * top + k] : 1.0f, parts[(size_t)(row_of ? row_of[t * top + k] : t * top + k) * d + i], acc);
         if (extra) acc = fmaf(extra_weight ? extra_weight[t] : 1.0f, extra[idx], acc);
         y[idx] = accumulate ? y[idx] + acc : acc;
+    }
+}
+
+// The same for rows of a multiple of four on 16-byte boundaries, one block per token and four columns a thread: a token's rows and
+// weights are found once, and four rows' loads are under way together (with the gathering four rows a block and the sort eight
+// assignments a thread: a layer of 32 experts, 4 chosen, over 4,096 tokens 2,048 wide 365 -> 329 us on B200).
+__global__ void __launch_bounds__(256)
+moe_combine4_kernel(const float4* __restrict__ parts, const float* __restrict__ weight, const int* __restrict__ row_of, const float4* __restrict__ extra,
+                    const float* __restrict__ extra_weight, float4* __restrict__ y, int top, int d4, int accumulate) {
+    ik_pdl_wait();
+    IK_AFTER_WAIT(parts);
+    IK_AFTER_WAIT(weight);
+    IK_AFTER_WAIT(row_of);
+    IK_AFTER_WAIT(extra);
+    IK_AFTER_WAIT(extra_weight);
+    ik_pdl_launch_dependents();
+    const size_t t = blockIdx.x;
+    const float ew = extra && extra_weight ? extra_weight[t] : 1.0f;
+    for (int c = threadIdx.x; c < d4; c += 256) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k0 = 0; k0 < top; k0 += 4) {
+            float4 v[4];
+            float w[4];
+            #pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (k0 + i < top) {
+                    v[i] = parts[(size_t)(row_of ? row_of[t * top + k0 + i] : (int)t * top + k0 + i) * d4 + c];
+                    w[i] = weight ? weight[t * top + k0 + i] : 1.0f;
+                }
+            #pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (k0 + i < top) {
+                    acc.x = fmaf(w[i], v[i].x, acc.x); acc.y = fmaf(w[i], v[i].y, acc.y);
+                    acc.z = fmaf(w[i], v[i].z, acc.z); acc.w = fmaf(w[i], v[i].w, acc.w);
+                }
+        }
+        if (extra) {
+            const float4 v = extra[t * d4 + c];
+            acc.x = fmaf(ew, v.x, acc.x); acc.y = fmaf(ew, v.y, acc.y); acc.z = fmaf(ew, v.z, acc.z); acc.w = fmaf(ew, v.w, acc.w);
+        }
+        if (accumulate) {
+            const float4 v = y[t * d4 + c];
+            acc = make_float4(v.x + acc.x, v.y + acc.y, v.z + acc.z, v.w + acc.w);
+        }
+        y[t * d4 + c] = acc;
     }
 }
 
@@ -549,8 +615,7 @@ IK_EXPORT int ik_moe_sort_padded(const int* chosen, int* row_of, int* src_token,
 IK_EXPORT int ik_moe_gather(const void* x, const int* src_token, void* xp, int rows, int d, cudaStream_t stream) {
     if (rows < 0 || d <= 0 || d % 8 || ((uintptr_t)x % 16) || ((uintptr_t)xp % 16)) return IK_BAD_ARGUMENT;
     if (rows == 0) return IK_OK;
-    const size_t total = (size_t)rows * (d / 8), want = (total + 255) / 256, cap = (size_t)ik_sm_count() * 16;
-    IK_RETURN_IF_ERROR(ik_launch(moe_gather_kernel, (int)(want < cap ? want : cap), 256, 0, stream, (const uint4*)x, src_token, (uint4*)xp, rows, d / 8));
+    IK_RETURN_IF_ERROR(ik_launch(moe_gather_kernel, (rows + 3) / 4, 256, 0, stream, (const uint4*)x, src_token, (uint4*)xp, rows, d / 8));
     IK_LAUNCH_STATUS();
 }
 
@@ -570,6 +635,12 @@ IK_EXPORT int ik_moe_combine(const float* parts, const float* weight, const int*
                              int T, int top, int d, int accumulate, cudaStream_t stream) {
     if (T < 0 || top <= 0 || d <= 0) return IK_BAD_ARGUMENT;
     if (T == 0) return IK_OK;
+    // few tokens are cut by columns over the SMs (the kernel above's flat grid) instead of by tokens
+    if (d % 4 == 0 && T >= 2 * ik_sm_count() && ((uintptr_t)parts | (uintptr_t)y | (uintptr_t)extra) % 16 == 0) {
+        IK_RETURN_IF_ERROR(ik_launch(moe_combine4_kernel, T, 256, 0, stream, (const float4*)parts, weight, row_of, (const float4*)extra, extra_weight,
+                                     (float4*)y, top, d / 4, accumulate));
+        IK_LAUNCH_STATUS();
+    }
     const size_t total = (size_t)T * d, want = (total + 255) / 256, cap = (size_t)ik_sm_count() * 16;
     IK_RETURN_IF_ERROR(ik_launch(moe_combine_kernel, (int)(want < cap ? want : cap), 256, 0, stream, parts, weight, row_of, extra, extra_weight, y, T, top, d, accumulate));
     IK_LAUNCH_STATUS();
