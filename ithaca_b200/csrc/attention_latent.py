@@ -97,23 +97,24 @@ def attend(q: torch.Tensor, k_pages: torch.Tensor, ctx, table: torch.Tensor, n_h
     return out
 
 
-PROMPT_KEYS_MOST = 1 << 17        # keys of a step whose heads' keys and values are formed: 8 or 16 KB each with 16 or 32 heads
+PROMPT_KEYS_MOST = 1 << 16        # keys of a step whose heads' keys and values are formed: 8 or 16 KB each with 16 or 32 heads, 1 GB at most
 FORM_KEYS_QUERIES = 64
 
 
-def forms_keys(ctx, k_pages: torch.Tensor, dtype: torch.dtype, dk: int, dr: int, dv: int, rank: int) -> bool:
+def forms_keys(ctx, k_pages: torch.Tensor, dtype: torch.dtype, dk: int, dr: int, dv: int, rank: int, window: int = 0) -> bool:
     """Whether a step's attention goes over keys and values formed per head (``prompt``) rather than over the cached rows.  Forming
     them costs heads x rank x (dk + dv) products a key; a query that sees the key then saves 2 rank - dk - dv of the 2 rank + dr
     products per head (768 of 1,088), and runs on tcgen05.  Measured on B200 (rank 512, one sequence; us for the layer, over the rows /
     formed): 16 heads, 64 new tokens behind 2,000 190 / 155, 512 behind 2,000 371 / 168, 4,096 from the start 2,056 / 348; 32 heads,
-    64 behind 2,000 228 / 183, 512 behind 2,000 674 / 245; below 64 not measured."""
+    64 behind 2,000 228 / 183, 512 behind 2,000 674 / 245; below 64 not measured.  Under a window a query sees that many keys at
+    most, while every key is formed."""
     if dtype != torch.bfloat16 or k_pages.dtype != torch.bfloat16 or ctx.is_decode or k_pages.shape[1:3] != (1, 64):
         return False
     if dk != 128 or dv != 128 or dr not in (0, 64) or rank % 64 or k_pages.shape[3] != rank + dr:
         return False
     lens, new = ctx.host_kv_lens, ctx.host_n_new
     keys = sum(lens)
-    return len(lens) == ctx.n_seqs and keys <= PROMPT_KEYS_MOST and sum(n * e for n, e in zip(new, lens)) >= FORM_KEYS_QUERIES * keys
+    return len(lens) == ctx.n_seqs and keys <= PROMPT_KEYS_MOST and sum(n * min(e, window or e) for n, e in zip(new, lens)) >= FORM_KEYS_QUERIES * keys
 
 
 def prompt(q_plain: torch.Tensor, q_full: torch.Tensor, k_pages: torch.Tensor, w_kv: torch.Tensor, ctx, table: torch.Tensor, n_heads: int,
@@ -127,8 +128,8 @@ def prompt(q_plain: torch.Tensor, q_full: torch.Tensor, k_pages: torch.Tensor, w
     lib = ops.lib()
     latents = torch.empty((n_keys, rank), dtype=torch.bfloat16, device=q_plain.device)
     ops._work(f"latent_gather {n_keys}x{rank}", 2 * ops._nbytes(latents))
-    _check(lib.ik_latent_gather(_ptr(k_pages), _ptr(ctx.kv_lens), _ptr(table), table.stride(0), _ptr(latents), B, ctx.max_kv_len, hd, rank, n_pages,
-                                _ptr(status), _stream()), "latent_gather")
+    _check(lib.ik_latent_gather(_ptr(k_pages), _ptr(ctx.cu_seqlens), _ptr(ctx.kv_lens), _ptr(table), table.stride(0), _ptr(latents), B, ctx.max_kv_len,
+                                hd, rank, int(window or 0), n_pages, _ptr(status), _stream()), "latent_gather")
     kv = gemm_bf16.gemm(latents, w_kv, out_dtype=torch.bfloat16)
     out = torch.empty((T, n_heads * 128), dtype=torch.bfloat16, device=q_plain.device)
     if ops.profiling():

@@ -326,14 +326,17 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_qp, const __grid_co
 }
 
 // The cached latents of all sequences' keys, one after another: row key_base(b) + j holds the leading `rank` columns of key j of
-// sequence b, and zeros where the last step of a sequence has no key.
+// sequence b, and zeros where the last step of a sequence has no key.  Pages that lie wholly behind the window of the step's first
+// query are passed over: they may have been given back, and their rows are never read.
 __global__ void __launch_bounds__(256)
-latent_gather_kernel(const bf16* __restrict__ rows, const int* __restrict__ kv_lens, const int* __restrict__ table, int table_stride,
-                     bf16* __restrict__ out, int hd, int rank, int n_pages, int* status) {
+latent_gather_kernel(const bf16* __restrict__ rows, const int* __restrict__ cu_seqlens, const int* __restrict__ kv_lens, const int* __restrict__ table,
+                     int table_stride, bf16* __restrict__ out, int hd, int rank, int window, int n_pages, int* status) {
     ik_pdl_wait();
     ik_pdl_launch_dependents();
     const int b = blockIdx.y, p = blockIdx.x, len = kv_lens[b];
     if (p * PAGE >= len) return;
+    const int first = len - (cu_seqlens[b + 1] - cu_seqlens[b]);               // position of the sequence's first query
+    if (window > 0 && (p + 1) * PAGE <= first + 1 - window) return;
     int page = table[(size_t)b * table_stride + p];
     const bool there = page >= 0 && page < n_pages;
     if (!there) {
@@ -365,13 +368,13 @@ int launch_prompt(const CUtensorMap& qp, const CUtensorMap& qt, const CUtensorMa
 }  // namespace
 
 // Gathers the latents (columns 0 .. rank - 1 of the rows [n_pages][64][hd]) of B sequences' keys into out [sum of lengths rounded up to 64, rank].
-IK_EXPORT int ik_latent_gather(const void* rows, const int* kv_lens, const int* table, int table_stride, void* out, int B, int max_kv_len, int hd,
-                               int rank, int n_pages, int* status, cudaStream_t stream) {
+IK_EXPORT int ik_latent_gather(const void* rows, const int* cu_seqlens, const int* kv_lens, const int* table, int table_stride, void* out, int B,
+                               int max_kv_len, int hd, int rank, int window, int n_pages, int* status, cudaStream_t stream) {
     if (B < 0 || max_kv_len < 0 || rank <= 0 || hd < rank || n_pages <= 0) return IK_BAD_ARGUMENT;
     if (hd % 8 || rank % 8 || ((uintptr_t)rows | (uintptr_t)out) % 16 || B > 65535) return IK_UNSUPPORTED;
     if (B == 0 || max_kv_len == 0) return IK_OK;
-    IK_RETURN_IF_ERROR(ik_launch(latent_gather_kernel, dim3((max_kv_len + PAGE - 1) / PAGE, B), 256, 0, stream, (const bf16*)rows, kv_lens, table,
-                                 table_stride, (bf16*)out, hd, rank, n_pages, status));
+    IK_RETURN_IF_ERROR(ik_launch(latent_gather_kernel, dim3((max_kv_len + PAGE - 1) / PAGE, B), 256, 0, stream, (const bf16*)rows, cu_seqlens,
+                                 kv_lens, table, table_stride, (bf16*)out, hd, rank, window, n_pages, status));
     IK_LAUNCH_STATUS();
 }
 

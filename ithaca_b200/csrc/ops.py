@@ -100,7 +100,7 @@ _SIGNATURES = {
     "ik_head_norm_gate": [_vp, _vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _f, _i, _i, _vp],
     "ik_latent_prepare": [_vp, _i, _i, _i, _vp, _f, _vp, _vp, _i, _vp, _i, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i,
                           _vp, _vp],
-    "ik_latent_gather": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp, _vp],
+    "ik_latent_gather": [_vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp],
     "ik_latent_prompt": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp, _vp],
     "ik_latent_prompt_take_wait_record": [_vp],
     "ik_layernorm": [_vp, _vp, _vp, _vp, _vp, _i, _vp, _f, _i, _i, _f, _vp],

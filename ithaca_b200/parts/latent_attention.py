@@ -130,7 +130,7 @@ class LatentAttention:
             q_plain = torch.empty((T, H * dk), dtype=rt.act_dtype, device=x.device)
             ops.latent_prepare(p, 0, self.c_off, self.c_norm_w, self.norm_eps, q_plain, q_full, cache.k_pages, ctx.token_seq,
                                ctx.token_pos, table, self.position.inv_freq if dr else None, H, dk, dr, rank, writes_cache, rt.status)
-        if self.w_kv is not None and attention_latent.forms_keys(ctx, cache.k_pages, rt.act_dtype, dk, dr, dv, rank):
+        if self.w_kv is not None and attention_latent.forms_keys(ctx, cache.k_pages, rt.act_dtype, dk, dr, dv, rank, self.window or 0):
             heads = attention_latent.prompt(q_plain, q_full, cache.k_pages, self.w_kv, ctx, table, H, rank, self.scale, self.window or 0, rt.status)
             if self.gate:
                 ops.head_gate(heads, p, self.g_off, heads, H, wide=True)

@@ -26,7 +26,11 @@ def test_attention_over_formed_keys(rope, new, start, window):
     for b, e in enumerate(lens):
         for i in range(-(-e // 64)):
             table[b, i] = order.pop()
-    rows, table = rnd(n_pages, 1, 64, hd), table.to(DEV)
+    rows, whole = rnd(n_pages, 1, 64, hd), table.clone().to(DEV)
+    for b, first in enumerate(start):                              # pages behind the window may have been given back
+        if window:
+            table[b, :max(0, first + 1 - window) // 64] = -1
+    table = table.to(DEV)
     q_plain, q_full, w = rnd(T, H * 128), rnd(T, H * hd) * 1.5, (rnd(2 * H * 128, rank).float() * rank ** -0.5).to(torch.bfloat16)
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
     cu = [sum(new[:i]) for i in range(B + 1)]
@@ -39,7 +43,7 @@ def test_attention_over_formed_keys(rope, new, start, window):
     assert torch.equal(got, again)
     for b, (n, e) in enumerate(zip(new, lens)):
         at = torch.arange(e, device=DEV)
-        x = rows[table[b, at // 64].long(), 0, at % 64].double()
+        x = rows[whole[b, at // 64].long(), 0, at % 64].double()
         kv = (x[:, :rank] @ w.double().T).view(e, 2, H, 128)
         k = torch.cat((kv[:, 0], x[:, None, rank:].expand(-1, H, -1)), -1)
         q = torch.cat((q_plain[cu[b]:cu[b + 1]].view(n, H, 128), q_full[cu[b]:cu[b + 1]].view(n, H, hd)[:, :, rank:]), -1).double()
@@ -74,3 +78,5 @@ def test_which_steps_form_keys():
     assert takes(ctx([64], [64])) and not takes(ctx([63], [63])) and not takes(ctx([1, 1], [900, 900], True)) and not takes(ctx([300, 1], [300, 60000]))
     assert not takes(ctx([4096], [4096]), dk=64) and not takes(ctx([4096], [4096]), dr=32) and not takes(ctx([4096], [4096]), dt=torch.float32)
     assert not takes(ctx([200000], [200000]))
+    assert not a.forms_keys(ctx([300], [60000]), rows, torch.bfloat16, 128, 64, 128, 512, 1024)       # a window: most keys would be formed for nothing
+    assert a.forms_keys(ctx([4096], [4096]), rows, torch.bfloat16, 128, 64, 128, 512, 1024)
