@@ -6,10 +6,11 @@
 //   S <- G_end S + K^T ((G_end / G) U).
 // delta_chunk_prepare_kernel forms T and P of every chunk and head side by side; delta_chunk_kernel walks a sequence's chunks with
 // a slice of a head's columns per block: five small products a chunk in place of 64 dependent steps.  The tokens' chain is what
-// bounded the token-by-token kernel (0.45 us a token whatever the batch); the chunks' chain is bound by the multiply-adds of
-// the walk, about 8,200 cycles a chunk and block at full rate.
+// bounded the token-by-token kernel (0.45 us a token whatever the batch); the chunks' chain is bound by the walk's
+// reads from shared memory (half a 16-byte read per four multiply-adds and thread, and an SM returns 128 bytes of reads a cycle)
+// beside its multiply-adds, about 8,200 cycles a chunk and block at full rate.
 // Measured on B200: a layer 2,048 wide with 16 heads of 128 over two prompts of 3,000 and fewer tokens 2,776 -> 790 us (the rule itself
-// 2,240 -> 600: 89 us of T and P, 509 us of the walk, 10.8 us a chunk).
+// 2,240 -> 600: 89 us of T and P, 509 us of the walk, 10.8 us a chunk; with 512 threads, each half the results, the walk took 606).
 #include "common.cuh"
 
 namespace {

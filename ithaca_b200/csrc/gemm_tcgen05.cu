@@ -219,12 +219,13 @@ __device__ unsigned long long ik_timeline[1024][8];
 // MODE 1 (CL): the cluster mode described at the top (n_splits blocks per tile, partial == nullptr, one piece of work
 // per block).  MODE 2 (PAIRS): pairs of blocks share the token tile's copy (whole tiles only; map_x's box is half a tile).
 // MODE 3: as MODE 0 with two K blocks (128 k) per stage, for token tiles up to 128 wide.  Measured with one thread issuing
-// back to back in a kernel that does nothing else (ik_gemm_tcgen05_issue_rate below): a product instruction costs the
-// issuing thread about 75 cycles and a commit about 190, whatever the tile's width, while the tensor core needs 32 / 64 /
+// back to back, inside a branch on its lane, in a kernel that does nothing else (ik_gemm_tcgen05_issue_rate below): a product
+// instruction costs the issuing thread about 75 cycles and a commit about 190, whatever the tile's width, while the tensor core needs 32 / 64 /
 // 128 cycles for 64 / 128 / 256 tokens.  At 256 tokens four products and a commit per K block just keep up (about 490
 // against 512 cycles); below that the issuing thread would be the bound, and eight products per commit make it cheaper.  (Two issuing threads, each with an accumulator of its own,
 // issue twice as fast in that kernel, but did not speed up this one: with stages this large only three or four are in
-// flight, and what a block can take in, 192 KB per load latency, is the bound that is left.)
+// flight, and what a block can take in, 192 KB per load latency, is the bound that is left.)  Since then the issuing warps stay
+// whole and elect the lane, which costs less per instruction (elect_one, tc_common.cuh).
 // A stage holds [W block 0][W block 1][X block 0][X block 1].
 template <int BN, typename TY, int MODE>
 __global__ void __launch_bounds__(THREADS, 1)

@@ -11,7 +11,8 @@
 //
 // Tokens are TMEM lanes, so a thread of the epilogue holds neighbouring features of one token: gate and up, or the two
 // members of a rotary pair, meet in one thread without shuffles, and results leave through shared memory as TMA stores of
-// 32 tokens x 64 or 128 bytes (adding into Y: as TMA reductions, so that Y is never read by the SM).  Eight warps drain an
+// 32 tokens x 64 or 128 bytes (adding into Y: as TMA
+// reductions, one per element, so that Y is never read by the SM; a sum below 2^-126 may become zero).  Eight warps drain an
 // accumulator (each 32 lanes of every other chunk of columns) while the next tile fills the other one.
 //
 // Measured on B200 against gemm_tcgen05.cu's pair mode (us, replayed graphs over weights larger than L2 together; cuBLAS beside):
