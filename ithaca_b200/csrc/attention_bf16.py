@@ -68,6 +68,8 @@ def module(head_dim: int, slopes: bool = False, one_row: bool = False) -> ctypes
         m.ik_attn_prefill.restype = _i
         m.ik_attn_prefill_tc.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _f, _i, _i, _i, _vp, _vp, _vp, _f, _f, _i, _i, _i, _vp, _vp]
         m.ik_attn_prefill_tc.restype = _i
+        m.ik_attn_prefill_two_heads.argtypes = m.ik_attn_prefill_tc.argtypes
+        m.ik_attn_prefill_two_heads.restype = _i
         m.ik_attn_decode.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _f, _i, _i, _i, _vp, _vp, _vp, _f, _f, _i, _i, _i, _i, _i, _i,
                                      _vp, _vp]
         m.ik_attn_decode.restype = _i
@@ -84,8 +86,8 @@ def prefill(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, cu_se
             window: int, status: Optional[torch.Tensor], out: Optional[torch.Tensor] = None,
             kind: str = "auto", work: Optional[Tuple[int, int]] = None, softcap: float = 0.0, sink=False, keep: int = 0,
             key_scales: Optional[torch.Tensor] = None, slopes: Optional[torch.Tensor] = None, reach=None) -> torch.Tensor:
-    """``kind``: "tc" = the tcgen05 kernel (head sizes 64 and 128), "mma" = the warp-level kernel,
-    "auto" = tcgen05 where it applies.  ``softcap``: scores become cap * tanh(score / cap) (0 = no cap).  ``sink``: the
+    """``kind``: "tc" = the tcgen05 kernels (head sizes 64 and 128), "two_heads" = the one with two heads a block, "mma" = the
+    warp-level kernel, "auto" = tcgen05 where it applies.  ``softcap``: scores become cap * tanh(score / cap) (0 = no cap).  ``sink``: the
     softmax's denominator counts one more key of score 0 that carries no value (True), or of a score per head (a float32
     tensor [n_heads], not scaled).  ``key_scales``: the pages' rows are keys and values (``v_pages`` None), and every score is
     multiplied by its key's number.  ``slopes`` [n_heads]: a score loses slope * distance, behind the cap.  ``reach`` = (norm, coef, every): no
@@ -96,15 +98,16 @@ def prefill(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, cu_se
     m = module(hd, slopes is not None, key_scales is not None)
     if out is None:
         out = torch.empty_like(q)
-    if kind == "tc" or (kind == "auto" and hd in (64, 128)):
+    if kind in ("tc", "two_heads") or (kind == "auto" and hd in (64, 128)):
         ops._work(f"attention prefill tcgen05 {q.shape[0]}x{n_heads}", *(work or (0, 0)))
-        st = m.ik_attn_prefill_tc(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(cu_seqlens), _ptr(kv_lens),
+        run = m.ik_attn_prefill_two_heads if kind == "two_heads" else m.ik_attn_prefill_tc
+        st = run(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(cu_seqlens), _ptr(kv_lens),
                                   _ptr(table), table.stride(0), q.shape[0], n_seqs, max_new, n_heads, nkv, scale, softcap, window, keep,
                                   ops.sink_flag(sink), _ptr(ops.sink_values(sink, n_heads)), _ptr(key_scales), _ptr(slopes), *(reach or (0.0, 0.0, 0)), page_size, n_pages, _ptr(status), _stream())
         if st != -2:
             _check(st, "attention prefill (tcgen05)")
             return out
-        if kind == "tc":
+        if kind != "auto":
             raise KernelError("attention prefill (tcgen05): head size or alignment not supported")
     ops._work(f"attention prefill mma {q.shape[0]}x{n_heads}", *(work or (0, 0)))
     _check(m.ik_attn_prefill(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(cu_seqlens), _ptr(kv_lens),
