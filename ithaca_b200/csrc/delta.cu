@@ -89,7 +89,7 @@ template <int L, int R>
 __global__ void __launch_bounds__(256)
 delta_rule_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, int v_off, const float* __restrict__ bg,
                   float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ cu_seqlens,
-                  const int* __restrict__ kv_lens, float* __restrict__ out, int H, int G, int dk, int dv, int TT, int W, int vec) {
+                  const int* __restrict__ kv_lens, float* __restrict__ out, int H, int G, int dk, int dv, int TT, int W, int vec, int below) {
     extern __shared__ __align__(16) float sm[];          // [2][TT][W]: q, k (16 L each), the block's v, step, decay, k . q
     ik_pdl_wait();
     IK_AFTER_WAIT(u);
@@ -107,7 +107,7 @@ delta_rule_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, in
     const int ccol = live ? col : dv - 1;
     const int per_tile = TT * W;
     const int lo = cu_seqlens[b], hi = cu_seqlens[b + 1], end = kv_lens[b], start = end - (hi - lo);
-    if (hi <= lo) return;
+    if (hi <= lo || hi - lo >= below) return;
     const int kvh = h / (H / G);
     const size_t per = (size_t)H * dk * dv;
     const float* st_in = state + ((size_t)slots[b] * 2 + ((start - 1) & 1)) * per + ((size_t)h * dv + ccol) * dk;
@@ -214,7 +214,7 @@ delta_rule_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, in
 template <int L, int R>
 static cudaError_t ik_delta_rule_launch(dim3 grid, int threads, size_t smem, cudaStream_t stream, const float* u, int ldu, int q_off, int k_off,
                                         int v_off, const float* bg, float* state, const int* slots, const int* cu_seqlens,
-                                        const int* kv_lens, float* out, int H, int G, int dk, int dv, int TT, int W, int vec) {
+                                        const int* kv_lens, float* out, int H, int G, int dk, int dv, int TT, int W, int vec, int below) {
     static bool raised = false;
     if (smem > 48 * 1024 && !raised) {
         const cudaError_t e = cudaFuncSetAttribute(delta_rule_kernel<L, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
@@ -222,13 +222,14 @@ static cudaError_t ik_delta_rule_launch(dim3 grid, int threads, size_t smem, cud
         raised = true;
     }
     return ik_launch(delta_rule_kernel<L, R>, grid, dim3(threads), smem, stream, u, ldu, q_off, k_off, v_off, bg, state, slots, cu_seqlens,
-                     kv_lens, out, H, G, dk, dv, TT, W, vec);
+                     kv_lens, out, H, G, dk, dv, TT, W, vec, below);
 }
 
+// below > 0: sequences that bring that many tokens or more are left alone (ik_delta_chunks has run them).
 IK_EXPORT int ik_delta_rule(const float* u, int ldu, int q_off, int k_off, int v_off, const float* bg, float* state, const int* slots,
                             const int* cu_seqlens, const int* kv_lens, float* out, int T, int B, int H, int G, int dk, int dv,
-                            int one_token_each, cudaStream_t stream) {
-    if (T < 0 || B < 0 || H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0 || !state || !bg) return IK_BAD_ARGUMENT;
+                            int one_token_each, int below, cudaStream_t stream) {
+    if (T < 0 || B < 0 || H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0 || below < 0 || !state || !bg) return IK_BAD_ARGUMENT;
     if (T == 0 || B == 0) return IK_OK;
     if (dk > 32 * 16) return IK_UNSUPPORTED;         // 32 lanes of 16 rows
     if (one_token_each && T != B) return IK_BAD_ARGUMENT;
@@ -246,7 +247,7 @@ IK_EXPORT int ik_delta_rule(const float* u, int ldu, int q_off, int k_off, int v
 #define IK_DR(LL)                                                                                                                 \
     case LL:                                                                                                                      \
         IK_RETURN_IF_ERROR(ik_delta_rule_launch<LL, R>(grid, 32 * nwarps, smem, stream, u, ldu, q_off, k_off, v_off, bg, state, slots, \
-                                                       cu_seqlens, kv_lens, out, H, G, dk, dv, TT, W, vec));                     \
+                                                       cu_seqlens, kv_lens, out, H, G, dk, dv, TT, W, vec, below ? below : 0x7fffffff));                     \
         break
     switch (L) {
         IK_DR(1);

@@ -6,7 +6,7 @@
 //   S <- G_end S + K^T ((G_end / G) U).
 // delta_chunk_prepare_kernel forms T and P of every chunk and head side by side; delta_chunk_kernel walks a sequence's chunks with
 // a slice of a head's columns per block: five small products a chunk in place of 64 dependent steps.  The tokens' chain is what
-// bounded the token-by-token kernel (0.45 us a token whatever the batch); the chunks' chain is bound by the walk's
+// bounds the token-by-token kernel (0.37 to 0.4 us a token; which sequences of a step go which way: ops.delta_chunks_from); the chunks' chain is bound by the walk's
 // reads from shared memory (half a 16-byte read per four multiply-adds and thread, and an SM returns 128 bytes of reads a cycle)
 // beside its multiply-adds, about 8,200 cycles a chunk and block at full rate.
 // Measured on B200: a layer 2,048 wide with 16 heads of 128 over two prompts of 3,000 and fewer tokens 2,776 -> 790 us (the rule itself
@@ -19,7 +19,36 @@ constexpr int C = 64;                                    // tokens of a chunk
 constexpr int TLD = C + 4;                               // row stride of T and P in shared memory
 constexpr int VEC = 132;                                 // floats of a chunk's decays: G [64], G_end / G [64], G_end, padding
 
-__device__ __forceinline__ int chunk_base(const int* cu_seqlens, int b) { return cu_seqlens[b] / C + b; }
+// Only sequences of at least `least` (> 0) tokens are walked, and their chunks numbered, in the order of the sequences.
+struct Walked {
+    int b, chunk0;                                       // the sequence (-1: there is none), the number of its first chunk
+};
+// The i-th walked sequence, or (BY_CHUNK) the one that chunk number i belongs to.  Every warp looks by itself, 32 sequences at a time.
+template <bool BY_CHUNK>
+__device__ __forceinline__ Walked walked_sequence(const int* cu_seqlens, int n_seqs, int least, int i) {
+    const int lane = threadIdx.x & 31;
+    for (int b0 = 0, seen = 0, chunks = 0; b0 < n_seqs; b0 += 32) {
+        const int b = b0 + lane, n = b < n_seqs ? cu_seqlens[b + 1] - cu_seqlens[b] : 0;
+        const bool mine = n >= least;
+        const int own = mine ? (n + C - 1) / C : 0;
+        int upto = own;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int before = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += before;
+        }
+        const unsigned all = __ballot_sync(0xffffffffu, mine);
+        const bool it = mine && (BY_CHUNK ? i < chunks + upto && i >= chunks + upto - own : seen + __popc(all & ((1u << lane) - 1)) == i);
+        const unsigned found = __ballot_sync(0xffffffffu, it);
+        if (found) {
+            const int at = __ffs(found) - 1;
+            return {b0 + at, __shfl_sync(0xffffffffu, chunks + upto - own, at)};
+        }
+        seen += __popc(all);
+        chunks += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return {-1, 0};
+}
 
 __device__ __forceinline__ void copy16(float* dst, const float* src, bool there) {           // zeros where there is nothing
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -29,11 +58,11 @@ __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_
 __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ float4 at4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
-// One block per (flat chunk, value head): flat chunk cu_seqlens[b] / 64 + b + j is chunk j of sequence b.
+// One block per (chunk, value head).
 template <int DK>
 __global__ void __launch_bounds__(256)
 delta_chunk_prepare_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, const float* __restrict__ bg, float* __restrict__ scratch,
-                           float* __restrict__ vecs, const int* __restrict__ cu_seqlens, int n_seqs, int H, int G) {
+                           float* __restrict__ vecs, const int* __restrict__ cu_seqlens, int n_seqs, int least, int H, int G) {
     constexpr int LD = DK + 4;
     extern __shared__ __align__(16) float sm[];
     float* const Ks = sm;                                // [64][LD]
@@ -48,14 +77,9 @@ delta_chunk_prepare_kernel(const float* __restrict__ u, int ldu, int q_off, int 
     IK_AFTER_WAIT(cu_seqlens);
     ik_pdl_launch_dependents();
     const int tid = threadIdx.x, h = blockIdx.y, f = blockIdx.x;
-    int b = 0;
-    for (int high = n_seqs - 1; b < high;) {             // the last sequence whose first chunk is not behind this one
-        const int mid = (b + high + 1) >> 1;
-        if (chunk_base(cu_seqlens, mid) <= f) b = mid;
-        else high = mid - 1;
-    }
-    const int t0 = cu_seqlens[b] + (f - chunk_base(cu_seqlens, b)) * C, n = min(C, cu_seqlens[b + 1] - t0);
-    if (n <= 0) return;
+    const Walked seq = walked_sequence<true>(cu_seqlens, n_seqs, least, f);
+    if (seq.b < 0) return;
+    const int t0 = cu_seqlens[seq.b] + (f - seq.chunk0) * C, n = min(C, cu_seqlens[seq.b + 1] - t0);
     const int kvh = h / (H / G);
     for (int i = tid; i < 2 * C * (DK / 4); i += 256) {
         const int r = i / (DK / 4), w = i % (DK / 4), t = r & (C - 1);
@@ -160,7 +184,7 @@ delta_chunk_prepare_kernel(const float* __restrict__ u, int ldu, int q_off, int 
     }
 }
 
-// One block per (columns of a head, value head, sequence); DS columns.  A thread owns 4 columns of one or two rows of the chunk's
+// One block per (columns of a head, value head, walked sequence); DS columns.  A thread owns 4 columns of one or two rows of the chunk's
 // products (ty and 63 - ty: the triangular products then take every warp equally long), and 4 columns of DK / RG neighbouring
 // rows of the state (in registers; shared memory holds a copy to read from).
 template <int DK, int DS>
@@ -174,7 +198,7 @@ template <int DK, int DS>
 __global__ void __launch_bounds__(256, 1)
 delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, int v_off, const float* __restrict__ scratch, const float* __restrict__ vecs,
                    float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ cu_seqlens,
-                   const int* __restrict__ kv_lens, float* __restrict__ out, int H, int G, int dv) {
+                   const int* __restrict__ kv_lens, float* __restrict__ out, int n_seqs, int least, int H, int G, int dv) {
     typedef Walk<DK, DS> W;
     constexpr int LD = W::LD, RG = W::RG, RK = W::RK, RS = W::RS;
     extern __shared__ __align__(16) float sm[];
@@ -194,9 +218,10 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
     IK_AFTER_WAIT(cu_seqlens);
     IK_AFTER_WAIT(kv_lens);
     ik_pdl_launch_dependents();
-    const int tid = threadIdx.x, b = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * DS;
+    const Walked seq = walked_sequence<false>(cu_seqlens, n_seqs, least, blockIdx.z);
+    if (seq.b < 0) return;
+    const int tid = threadIdx.x, b = seq.b, h = blockIdx.y, col0 = blockIdx.x * DS;
     const int lo = cu_seqlens[b], hi = cu_seqlens[b + 1], end = kv_lens[b], start = end - (hi - lo);
-    if (hi <= lo) return;
     const int tx = tid % W::CG, ty = tid / W::CG, kvh = h / (H / G);
     const int col = col0 + 4 * tx, k0 = RS * ty;
     auto row = [&](int i) { return i == 0 ? ty : C - 1 - ty; };
@@ -205,7 +230,7 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
     const size_t per = (size_t)H * DK * dv;
     const float* st_in = state + ((size_t)slots[b] * 2 + ((start - 1) & 1)) * per + ((size_t)h * dv + (live ? col : 0)) * DK + k0;
     float* st_out = state + ((size_t)slots[b] * 2 + ((end - 1) & 1)) * per + ((size_t)h * dv + (live ? col : 0)) * DK + k0;
-    const int f0 = chunk_base(cu_seqlens, b), n_chunks = (hi - lo + C - 1) / C;
+    const int f0 = seq.chunk0, n_chunks = (hi - lo + C - 1) / C;
 
     auto bring_kq = [&](int j) {
         float* dst = KQ + (j & 1) * 2 * C * LD;
@@ -356,48 +381,51 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
 
 template <int DK, int DS>
 int walk(const float* u, int ldu, int q_off, int k_off, int v_off, const float* scratch, const float* vecs, float* state, const int* slots,
-         const int* cu_seqlens, const int* kv_lens, float* out, int B, int H, int G, int dv, cudaStream_t stream) {
+         const int* cu_seqlens, const int* kv_lens, float* out, int B, int least, int n_walked, int H, int G, int dv, cudaStream_t stream) {
     constexpr size_t smem = Walk<DK, DS>::FLOATS * sizeof(float);
     const cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<DK, DS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    IK_RETURN_IF_ERROR(ik_launch(delta_chunk_kernel<DK, DS>, dim3((dv + DS - 1) / DS, H, B), 256, smem, stream, u, ldu, q_off, k_off, v_off, scratch,
-                                 vecs, state, slots, cu_seqlens, kv_lens, out, H, G, dv));
+    IK_RETURN_IF_ERROR(ik_launch(delta_chunk_kernel<DK, DS>, dim3((dv + DS - 1) / DS, H, n_walked), 256, smem, stream, u, ldu, q_off, k_off, v_off,
+                                 scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, H, G, dv));
     IK_LAUNCH_STATUS();
 }
 
 template <int DK>
 int chunks(const float* u, int ldu, int q_off, int k_off, int v_off, const float* bg, float* scratch, float* state, const int* slots,
-           const int* cu_seqlens, const int* kv_lens, float* out, int T, int B, int H, int G, int dv, cudaStream_t stream) {
-    const int flat = T / C + B;
-    float* vecs = scratch + (size_t)flat * H * 2 * C * C;
+           const int* cu_seqlens, const int* kv_lens, float* out, int B, int least, int n_walked, int n_chunks, int H, int G, int dv,
+           cudaStream_t stream) {
+    float* vecs = scratch + (size_t)n_chunks * H * 2 * C * C;
     constexpr size_t smem = (2 * C * (DK + 4) + 2 * C * TLD + C) * sizeof(float) + C * sizeof(double);
     const cudaError_t e = cudaFuncSetAttribute(delta_chunk_prepare_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    IK_RETURN_IF_ERROR(ik_launch(delta_chunk_prepare_kernel<DK>, dim3(flat, H), 256, smem, stream, u, ldu, q_off, k_off, bg, scratch, vecs, cu_seqlens,
-                                 B, H, G));
+    IK_RETURN_IF_ERROR(ik_launch(delta_chunk_prepare_kernel<DK>, dim3(n_chunks, H), 256, smem, stream, u, ldu, q_off, k_off, bg, scratch, vecs,
+                                 cu_seqlens, B, least, H, G));
     // 32 columns a block do a third fewer loads per multiply-add; 16 where that leaves more than half of the SMs idle
-    if (2LL * B * H * ((dv + 31) / 32) <= ik_sm_count())
-        return walk<DK, 16>(u, ldu, q_off, k_off, v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, H, G, dv, stream);
-    return walk<DK, 32>(u, ldu, q_off, k_off, v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, H, G, dv, stream);
+    if (2LL * n_walked * H * ((dv + 31) / 32) <= ik_sm_count())
+        return walk<DK, 16>(u, ldu, q_off, k_off, v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, H, G, dv, stream);
+    return walk<DK, 32>(u, ldu, q_off, k_off, v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, H, G, dv, stream);
 }
 
 }  // namespace
 
-// Floats of scratch for these sizes; 0 where the chunks do not apply (short prompts, key sizes other than 64 and 128, value sizes
-// that are no multiple of 4): ik_delta_rule runs those.
+// Floats of scratch for B sequences of T tokens together; 0 where the chunks do not apply (short prompts, key sizes other than 64 and
+// 128, value sizes that are no multiple of 4): ik_delta_rule runs those.
 IK_EXPORT long long ik_delta_chunks_scratch(int T, int B, int max_new, int H, int dk, int dv) {
     if (T <= 0 || B <= 0 || B > 65535 || H > 65535 || max_new < C || (dk != 64 && dk != 128) || dv % 4) return 0;
     return (long long)(T / C + B) * H * (2 * C * C + VEC);
 }
 
-// As ik_delta_rule, a chunk of tokens at a time.  IK_UNSUPPORTED where rows of q, k or v are not on 16 bytes.
+// As ik_delta_rule, a chunk of tokens at a time, for the sequences that bring at least `least` tokens (the others are left alone): at
+// most n_walked of them, of at most n_chunks chunks together, for which scratch has room.  IK_UNSUPPORTED where rows of q, k or v are not
+// on 16 bytes.
 IK_EXPORT int ik_delta_chunks(const float* u, int ldu, int q_off, int k_off, int v_off, const float* bg, float* state, const int* slots,
-                              const int* cu_seqlens, const int* kv_lens, float* out, float* scratch, int T, int B, int H, int G, int dk, int dv,
-                              cudaStream_t stream) {
-    if (T < 0 || B < 0 || H <= 0 || G <= 0 || H % G || dv <= 0 || !state || !bg || !scratch) return IK_BAD_ARGUMENT;
-    if (T == 0 || B == 0) return IK_OK;
+                              const int* cu_seqlens, const int* kv_lens, float* out, float* scratch, int T, int B, int least, int n_walked,
+                              int n_chunks, int H, int G, int dk, int dv, cudaStream_t stream) {
+    if (T < 0 || B < 0 || least <= 0 || n_walked < 0 || n_chunks < 0 || n_walked > 65535 || H <= 0 || G <= 0 || H % G || dv <= 0 || !state || !bg ||
+        !scratch) return IK_BAD_ARGUMENT;
+    if (T == 0 || B == 0 || n_walked == 0 || n_chunks == 0) return IK_OK;
     if (ldu % 4 || q_off % 4 || k_off % 4 || v_off % 4 || dv % 4 || ((uintptr_t)u | (uintptr_t)out | (uintptr_t)scratch) % 16) return IK_UNSUPPORTED;
-    if (dk == 128) return chunks<128>(u, ldu, q_off, k_off, v_off, bg, scratch, state, slots, cu_seqlens, kv_lens, out, T, B, H, G, dv, stream);
-    if (dk == 64) return chunks<64>(u, ldu, q_off, k_off, v_off, bg, scratch, state, slots, cu_seqlens, kv_lens, out, T, B, H, G, dv, stream);
+    if (dk == 128) return chunks<128>(u, ldu, q_off, k_off, v_off, bg, scratch, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, n_chunks, H, G, dv, stream);
+    if (dk == 64) return chunks<64>(u, ldu, q_off, k_off, v_off, bg, scratch, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, n_chunks, H, G, dv, stream);
     return IK_UNSUPPORTED;
 }

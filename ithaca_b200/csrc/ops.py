@@ -94,8 +94,8 @@ _SIGNATURES = {
     "ik_scale_add_norm": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _f, _vp],
     "ik_plain_act": [_vp, _vp, _i, _u64, _i, _vp],
     "ik_delta_prepare": [_vp, _i, _i, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _f, _f, _vp],
-    "ik_delta_rule": [_vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
-    "ik_delta_chunks": [_vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
+    "ik_delta_rule": [_vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
+    "ik_delta_chunks": [_vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
     "ik_delta_chunks_scratch": [_i, _i, _i, _i, _i, _i],
     "ik_head_norm_gate": [_vp, _vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _f, _i, _i, _vp],
     "ik_latent_prepare": [_vp, _i, _i, _i, _vp, _f, _vp, _vp, _i, _vp, _i, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i,
@@ -1406,14 +1406,59 @@ def delta_prepare(u: torch.Tensor, q_off: int, k_off: int, p: torch.Tensor, b_of
     return bg
 
 
+def delta_chunks_from(n_new, n_heads: int, dk: int, dv: int, n_sm: int) -> int:
+    """The fewest tokens with which a sequence of a step goes through the chunks (0: none does): the least of what the step takes.
+
+    Token by token a step is a chain of its longest sequence's tokens, 0.37 us each while an SM has one block (32 columns, 64 with keys
+    of 64) and 0.21 us a block beyond, and a block's start for every sequence.  In chunks a block of 32 columns has an SM to itself: 10.5
+    us a chunk however few tokens are in it (5.5 with keys of 64; with 16 columns, where twice the blocks still fit the SMs, 7.9 and
+    5.3), 3 us a block, and what forms T and P, 71 ns per chunk and head and 18 us at least.
+    Measured on B200 (heads of 128 x 128; us, token by token / all in chunks / this rule), 16 heads: one prompt of 2,000 805 / 287 / 288, 8 of
+    2,000 1,824 / 1,654 / 1,654, 8 of 70 71 / 117 / 71, 32 of 70 231 / 411 / 231, 63 decoding sequences beside a prompt of 64 69 / 451 / 69, of
+    512 344 / 491 / 122, of 2,000 1,355 / 630 / 329; 32 heads: 16 of 64 210 / 231 / 210, the three with 63 decoding ones 107 / 883 / 106,
+    436 / 965 / 184, 1,565 / 1,236 / 498."""
+    if not n_new or max(n_new) < 64:
+        return 0
+    columns, token_columns = -(-dv // 32), -(-dv // (64 if dk <= 64 else 32))
+    narrow, wide = (7.9, 10.5) if dk > 64 else (5.3, 5.5)
+
+    def by_token(part):
+        if not part:
+            return 0.0
+        top = max(part)
+        blocks = -(-sum(part) * n_heads * token_columns // (top * n_sm))
+        return 3.5 + top * max(0.37, 0.07 + 0.21 * blocks) + 0.041 * len(part) * n_heads * dk * dv / 16384
+
+    def in_chunks(part):
+        counts = [-(-n // 64) for n in part]
+        n_blocks, total = len(part) * n_heads * columns, sum(counts)
+        step = narrow if 2 * n_blocks <= n_sm else wide
+        walk = max(counts) * step + 3.0
+        if n_blocks > n_sm:
+            walk = max(walk, (total * step / len(part) + 3.0) * -(-n_blocks // n_sm))
+        return max(18.0, 0.071 * total * n_heads) + walk
+
+    best, least = by_token(n_new), 0
+    for tokens in (1, 32, 64, 128, 256, 512, 1024):
+        many = [n for n in n_new if n >= tokens]
+        if not many:
+            break
+        cost = in_chunks(many) + by_token([n for n in n_new if 0 < n < tokens])
+        if cost < best:
+            best, least = cost, tokens
+    return least
+
+
 def delta_rule(u: torch.Tensor, q_off: int, k_off: int, v_off: int, bg: torch.Tensor, state: torch.Tensor, ctx, n_heads: int,
-               n_qk_heads: int, dk: int, dv: int, chunks: bool = False) -> torch.Tensor:
+               n_qk_heads: int, dk: int, dv: int, chunks: bool = False, chunks_from: Optional[int] = None) -> torch.Tensor:
     """The gated delta rule over the step's tokens: per head S <- g S; u = b (v - S^T k); S <- S + k u^T; o = S^T q.  q, k
     (``n_qk_heads`` heads, unit vectors) and v are column ranges of ``u`` (float), ``bg`` [T, 2, heads] the steps and decays,
     ``state`` [max_slots, 2, heads, dv, dk] float (column by column).  Returns float [T, heads * dv].
 
-    ``chunks``: prompts may run 64 tokens at a time (float all the same, but a token's sums then depend on where its chunk
-    begins, so a prompt cut otherwise does not give the same bits: for the 16-bit path)."""
+    ``chunks``: sequences may run 64 tokens at a time (float all the same, but a token's sums then depend on where its chunk
+    begins, so a prompt cut otherwise does not give the same bits: for the 16-bit path).  Those of ``chunks_from`` tokens and more do,
+    the others token by token (None: as ``delta_chunks_from`` says of the lengths the context knows on the host; where it knows none, all
+    do as soon as one brings 64)."""
     _need(u, "u", torch.float32)
     _need(bg, "bg", torch.float32)
     _need(state, "state", torch.float32)
@@ -1424,18 +1469,42 @@ def delta_rule(u: torch.Tensor, q_off: int, k_off: int, v_off: int, bg: torch.Te
     out = torch.empty((T, n_heads * dv), dtype=torch.float32, device=u.device)
     _work(f"delta_rule {T}x{n_heads}x{dk}x{dv}", T * (2 * n_qk_heads * dk + 2 * n_heads * dv) * 4 + 8 * ctx.n_seqs * n_heads * dk * dv,
           6 * T * n_heads * dk * dv)
-    need = lib().ik_delta_chunks_scratch(T, ctx.n_seqs, ctx.max_new, n_heads, dk, dv) if chunks and not ctx.is_decode else 0
-    if need:
-        scratch = torch.empty(need, dtype=torch.float32, device=u.device)
-        st = lib().ik_delta_chunks(_ptr(u), u.stride(0), q_off, k_off, v_off, _ptr(bg), _ptr(state), _ptr(ctx.slots), _ptr(ctx.cu_seqlens),
-                                   _ptr(ctx.kv_lens), _ptr(out), _ptr(scratch), T, ctx.n_seqs, n_heads, n_qk_heads, dk, dv, _stream())
-        if st != -2:
-            _check(st, "delta_chunks", kernels=2)
-            return out
+    below = 0                                             # sequences of that many tokens and more have run in chunks
+    if chunks and not ctx.is_decode and lib().ik_delta_chunks_scratch(T, ctx.n_seqs, ctx.max_new, n_heads, dk, dv):
+        n_new = list(getattr(ctx, "host_n_new", ()))
+        known = len(n_new) == ctx.n_seqs
+        if chunks_from is None:
+            chunks_from = _delta_chunks_from_of(ctx, n_new, n_heads, dk, dv) if known else 1
+        many = [n for n in n_new if n >= chunks_from] if known else []
+        walked, tokens = (len(many), sum(many)) if known else (ctx.n_seqs, T)
+        if chunks_from > 0 and walked > 0:
+            need = lib().ik_delta_chunks_scratch(tokens, walked, ctx.max_new, n_heads, dk, dv)
+            n_chunks = sum(-(-n // 64) for n in many) if known else tokens // 64 + walked
+            scratch = torch.empty(need, dtype=torch.float32, device=u.device)
+            st = lib().ik_delta_chunks(_ptr(u), u.stride(0), q_off, k_off, v_off, _ptr(bg), _ptr(state), _ptr(ctx.slots), _ptr(ctx.cu_seqlens),
+                                       _ptr(ctx.kv_lens), _ptr(out), _ptr(scratch), T, ctx.n_seqs, chunks_from, walked, n_chunks, n_heads,
+                                       n_qk_heads, dk, dv, _stream())
+            if st != -2:
+                _check(st, "delta_chunks", kernels=2)
+                below = chunks_from
+                if (tokens == T if known else chunks_from <= 1):
+                    return out
     _check(lib().ik_delta_rule(_ptr(u), u.stride(0), q_off, k_off, v_off, _ptr(bg), _ptr(state), _ptr(ctx.slots), _ptr(ctx.cu_seqlens),
                                _ptr(ctx.kv_lens), _ptr(out), T, ctx.n_seqs, n_heads, n_qk_heads, dk, dv, 1 if ctx.is_decode else 0,
-                               _stream()), "delta_rule")
+                               below, _stream()), "delta_rule")
     return out
+
+
+def _delta_chunks_from_of(ctx, n_new, n_heads: int, dk: int, dv: int) -> int:
+    """``delta_chunks_from`` of a step, once for all its layers of one size."""
+    shared = getattr(ctx, "shared", None)
+    key = ("delta_chunks_from", n_heads, dk, dv)
+    if shared is None or key not in shared:
+        least = delta_chunks_from(n_new, n_heads, dk, dv, sm_count())
+        if shared is None:
+            return least
+        shared[key] = least
+    return shared[key]
 
 
 HEAD_GATES = {None: 0, "silu": 1, "sigmoid": 2}
