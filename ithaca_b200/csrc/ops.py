@@ -1178,12 +1178,33 @@ def causal_conv(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], 
     return out
 
 
+def scan_pieces_pay(T: int, B: int, max_new: int, inner: int, N: int, n_sm: int) -> bool:
+    """Whether a step's selective scan (bfloat16 inputs) runs in pieces rather than whole sequences.
+
+    A whole sequence is a chain of its tokens, 0.11 to 0.15 us each while its SMs have few blocks, more with every block; pieces run side
+    by side but form every token's exponentials twice, and a sequence costs blocks of its own in both passes however short it is.
+    Measured on B200 (us, whole / pieces), 16 states: 4,096 channels, one prompt of 200 26 / 39, 1,000 116 / 88, 4,000 454 / 318, two of
+    2,000 287 / 318, 3,000 + 1,910 399 / 380, eight of 2,000 790 / 1,083, 63 decoding sequences beside a prompt of 200 46 / 122, of 2,000
+    352 / 250; 2,048 channels, two of 2,000 229 / 168, four 287 / 322; 8,192, one of 4,000 569 / 622.  64 states: 1,024 channels, two of
+    2,000 318 / 278, three 354 / 413."""
+    if max_new <= 0:
+        return False
+    blocks = -(-inner // (32 if N <= 16 else 16 if N <= 32 else 8)) / n_sm                  # of a sequence, per SM
+    at_work = T / max_new * blocks
+    token = 0.085 + 0.034 * at_work if N <= 16 else 0.125 + 0.022 * at_work
+    if B * blocks > 2.3:                                                                     # four states a thread, a longer chain
+        token = max(token, 0.17)
+    return max_new * token > 17.0 + 0.083 * T * blocks + 1.5 * B * blocks
+
+
 def selective_scan(u: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[torch.Tensor], A: torch.Tensor, bc: torch.Tensor,
                    b_off: int, c_off: int, D: Optional[torch.Tensor], z: Optional[torch.Tensor], state: torch.Tensor, ctx,
-                   out_dtype: torch.dtype) -> torch.Tensor:
+                   out_dtype: torch.dtype, pieces: Optional[bool] = None) -> torch.Tensor:
     """The selective scan over the step's tokens, sequence by sequence.  ``u`` [T, inner], ``dt_raw`` [T, inner] float
     (before bias and softplus), ``A`` [inner, N] float (negative), B and C = columns ``b_off``.. and ``c_off``.. of ``bc``,
-    ``z`` [T, inner] float (rows may be a column range) for the gate y * silu(z), ``state`` [max_slots, 2, inner, N] float."""
+    ``z`` [T, inner] float (rows may be a column range) for the gate y * silu(z), ``state`` [max_slots, 2, inner, N] float.
+    ``pieces``: prompts with bfloat16 inputs in pieces that run side by side, where the sizes allow it (None: where
+    ``scan_pieces_pay`` says so)."""
     _need(u, "u")
     _need(dt_raw, "dt_raw", torch.float32)
     _need(A, "A", torch.float32)
@@ -1204,7 +1225,9 @@ def selective_scan(u: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[torc
     _work(f"selective_scan {T}x{inner}x{N}", T * inner * (u.element_size() + 8 + out.element_size()) + 8 * ctx.n_seqs * inner * N,
           9 * T * inner * N)
     max_new = getattr(ctx, "max_new", 0)                  # a caller that does not say gets every sequence token by token
-    need = lib().ik_selective_scan_scratch(_code(u), T, ctx.n_seqs, max_new, inner, N, 1 if ctx.is_decode else 0)
+    need = 0
+    if pieces or (pieces is None and not ctx.is_decode and scan_pieces_pay(T, ctx.n_seqs, max_new, inner, N, sm_count())):
+        need = lib().ik_selective_scan_scratch(_code(u), T, ctx.n_seqs, max_new, inner, N, 1 if ctx.is_decode else 0)
     scratch = torch.empty(need, dtype=torch.float32, device=u.device) if need else None
     st = lib().ik_selective_scan(_ptr(u), _code(u), _ptr(dt_raw), _ptr(dt_bias), _ptr(A), _ptr(bc), bc.stride(0), b_off, c_off,
                                  _ptr(D), _ptr(z), ldz, _ptr(state), _ptr(ctx.slots), _ptr(ctx.cu_seqlens), _ptr(ctx.kv_lens),
