@@ -427,7 +427,8 @@ def attention_run(cfg, reps):
         lens = torch.tensor([kv_len], dtype=torch.int32, device=dev)
         status = torch.zeros(1, dtype=torch.int32, device=dev)
         res = torch.empty_like(q)
-        run = lambda: A.prefill(q, k, v, cu, lens, table, 1, n_new, heads, 1 / math.sqrt(hd), 0, status, out=res)
+        two = hd in (64, 128) and heads // kv_heads % 2 == 0 and A.two_heads_pay([n_new], [kv_len], heads, hd, 0, A.sm_count())
+        run = lambda: A.prefill(q, k, v, cu, lens, table, 1, n_new, heads, 1 / math.sqrt(hd), 0, status, out=res, two_heads=two)
         for _ in range(2):
             run()
         torch.cuda.synchronize()

@@ -697,7 +697,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 //   warp 0 loads, warp 1 issues, warps 2..5 and 6..9 are the softmax of the first and the second head (one thread per query).
 // Keys past the last page of an odd number are the last page again: masked as keys, and finite as values.
 // Measured on B200 (one head a block / this; us): 32 heads of 128 on 8, one prompt of 2,048 56.6 / 51.4, six of 50 to 2,000 132 / 112; heads of 64
-// 51.3 / 43.4 and 117 / 94; 2,048 behind 6,144 240 / 225 and 225 / 191.  See the rule in ik_attn_prefill_tc for where it loses.
+// 51.3 / 43.4 and 117 / 94; 2,048 behind 6,144 240 / 225 and 225 / 191.  Where it loses: two_heads_pay in attention_bf16.py.
 constexpr int TP_KEYS = 2 * PAGE, TP_NS = HD == 64 ? 3 : 2;
 constexpr int TP_STEP_BYTES = TP_KEYS * HD * 2;                // keys (or values) of a step
 constexpr int TP_SMEM = 2 * TC_Q_BYTES + TP_NS * 2 * TP_STEP_BYTES + 256;
@@ -1394,12 +1394,12 @@ IK_EXPORT int ik_attn_prefill(const void* q, const void* k_pages, const void* v_
 }
 
 // The tcgen05 kernel (head sizes 64 and 128; IK_UNSUPPORTED otherwise).  T: rows of q.
-// two_heads: 1 = the kernel with two heads a block or IK_UNSUPPORTED, -1 = where the rule says so.
+// two_heads: the kernel with two heads a block, or IK_UNSUPPORTED where there are options or an odd number of heads per kv head.
 static int prefill_tc(const void* q, const void* k_pages, const void* v_pages, void* out, const int* cu_seqlens,
                       const int* kv_lens, const int* table, int table_stride, int T, int B, int max_new, int nh,
                       int nkv, float scale, float softcap, int window, int keep, int sink, const float* sink_v, const float* key_scales,
                       const float* slopes, float reach_norm, float reach_coef, int reach_every, int page_size, int n_pages, int* status, cudaStream_t stream,
-                      int two_heads) {
+                      bool two_heads) {
     if (!options_fit(key_scales, slopes)) return IK_UNSUPPORTED;
     const Reach far{reach_norm, softcap, reach_coef, reach_every};
 #if IK_HD == 64 || IK_HD == 128
@@ -1417,11 +1417,8 @@ static int prefill_tc(const void* q, const void* k_pages, const void* v_pages, v
     if (st != IK_OK) return st;
     st = ik_make_map(&mv, v_pages, kv_rows, HD, HD, PAGE);
     if (st != IK_OK) return st;
-    // Two heads a block want about one and a half blocks an SM; with fewer the blocks of one head, twice as many, fill the SMs better
-    // (us, one head / two: 1,024 tokens, 32 heads of 128 26.3 / 28.6, 2,048 tokens, 16 heads 39.7 / 42.8, twelve prompts of 100 21.4 / 24.7).
-    const bool can_pair = !SLOPES && !ONE_ROW && softcap == 0.f && !sink && keep == 0 && (nh / nkv) % 2 == 0;
-    if (two_heads == 1 && !can_pair) return IK_UNSUPPORTED;
-    if (can_pair && (two_heads == 1 || 2LL * ((T + TC_BM - 1) / TC_BM) * (nh / 2) >= 3LL * ik_sm_count())) {
+    if (two_heads) {
+        if (SLOPES || ONE_ROW || softcap != 0.f || sink || keep != 0 || (nh / nkv) % 2) return IK_UNSUPPORTED;
         auto pairs = attn_prompt_pairs_kernel;
         cudaError_t e2 = cudaFuncSetAttribute(pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM);
         if (e2 != cudaSuccess) return (int)e2;
@@ -1448,12 +1445,12 @@ static int prefill_tc(const void* q, const void* k_pages, const void* v_pages, v
         int page_size, int n_pages, int *status, cudaStream_t stream
 IK_EXPORT int ik_attn_prefill_tc(IK_PREFILL_ARGS) {
     return prefill_tc(q, k_pages, v_pages, out, cu_seqlens, kv_lens, table, table_stride, T, B, max_new, nh, nkv, scale, softcap, window, keep, sink,
-                      sink_v, key_scales, slopes, reach_norm, reach_coef, reach_every, page_size, n_pages, status, stream, -1);
+                      sink_v, key_scales, slopes, reach_norm, reach_coef, reach_every, page_size, n_pages, status, stream, false);
 }
-// The kernel with two heads a block whatever the sizes; IK_UNSUPPORTED with options or an odd number of heads per kv head.
+// The kernel with two heads a block; IK_UNSUPPORTED with options or an odd number of heads per kv head.
 IK_EXPORT int ik_attn_prefill_two_heads(IK_PREFILL_ARGS) {
     return prefill_tc(q, k_pages, v_pages, out, cu_seqlens, kv_lens, table, table_stride, T, B, max_new, nh, nkv, scale, softcap, window, keep, sink,
-                      sink_v, key_scales, slopes, reach_norm, reach_coef, reach_every, page_size, n_pages, status, stream, 1);
+                      sink_v, key_scales, slopes, reach_norm, reach_coef, reach_every, page_size, n_pages, status, stream, true);
 }
 #undef IK_PREFILL_ARGS
 

@@ -85,9 +85,10 @@ def prefill(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, cu_se
             kv_lens: torch.Tensor, table: torch.Tensor, n_seqs: int, max_new: int, n_heads: int, scale: float,
             window: int, status: Optional[torch.Tensor], out: Optional[torch.Tensor] = None,
             kind: str = "auto", work: Optional[Tuple[int, int]] = None, softcap: float = 0.0, sink=False, keep: int = 0,
-            key_scales: Optional[torch.Tensor] = None, slopes: Optional[torch.Tensor] = None, reach=None) -> torch.Tensor:
-    """``kind``: "tc" = the tcgen05 kernels (head sizes 64 and 128), "two_heads" = the one with two heads a block, "mma" = the
-    warp-level kernel, "auto" = tcgen05 where it applies.  ``softcap``: scores become cap * tanh(score / cap) (0 = no cap).  ``sink``: the
+            key_scales: Optional[torch.Tensor] = None, slopes: Optional[torch.Tensor] = None, reach=None,
+            two_heads: bool = False) -> torch.Tensor:
+    """``kind``: "tc" = the tcgen05 kernel (head sizes 64 and 128), "two_heads" = the one with two heads a block, "mma" = the
+    warp-level kernel, "auto" = tcgen05 where it applies (``two_heads``: with two heads a block where that kernel takes the call).  ``softcap``: scores become cap * tanh(score / cap) (0 = no cap).  ``sink``: the
     softmax's denominator counts one more key of score 0 that carries no value (True), or of a score per head (a float32
     tensor [n_heads], not scaled).  ``key_scales``: the pages' rows are keys and values (``v_pages`` None), and every score is
     multiplied by its key's number.  ``slopes`` [n_heads]: a score loses slope * distance, behind the cap.  ``reach`` = (norm, coef, every): no
@@ -98,22 +99,80 @@ def prefill(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, cu_se
     m = module(hd, slopes is not None, key_scales is not None)
     if out is None:
         out = torch.empty_like(q)
-    if kind in ("tc", "two_heads") or (kind == "auto" and hd in (64, 128)):
+    ways = [kind] if kind in ("tc", "two_heads") else []
+    if kind == "auto" and hd in (64, 128):
+        ways = ["two_heads", "tc"] if two_heads else ["tc"]
+    for way in ways:
         ops._work(f"attention prefill tcgen05 {q.shape[0]}x{n_heads}", *(work or (0, 0)))
-        run = m.ik_attn_prefill_two_heads if kind == "two_heads" else m.ik_attn_prefill_tc
-        st = run(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(cu_seqlens), _ptr(kv_lens),
+        st = (m.ik_attn_prefill_two_heads if way == "two_heads" else m.ik_attn_prefill_tc)(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(cu_seqlens), _ptr(kv_lens),
                                   _ptr(table), table.stride(0), q.shape[0], n_seqs, max_new, n_heads, nkv, scale, softcap, window, keep,
                                   ops.sink_flag(sink), _ptr(ops.sink_values(sink, n_heads)), _ptr(key_scales), _ptr(slopes), *(reach or (0.0, 0.0, 0)), page_size, n_pages, _ptr(status), _stream())
         if st != -2:
             _check(st, "attention prefill (tcgen05)")
             return out
-        if kind != "auto":
-            raise KernelError("attention prefill (tcgen05): head size or alignment not supported")
+    if kind in ("tc", "two_heads"):
+        raise KernelError("attention prefill (tcgen05): head size or alignment not supported")
     ops._work(f"attention prefill mma {q.shape[0]}x{n_heads}", *(work or (0, 0)))
     _check(m.ik_attn_prefill(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(cu_seqlens), _ptr(kv_lens),
                              _ptr(table), table.stride(0), n_seqs, max_new, n_heads, nkv, scale, softcap, window, keep, ops.sink_flag(sink),
                              _ptr(ops.sink_values(sink, n_heads)), _ptr(key_scales), _ptr(slopes), *(reach or (0.0, 0.0, 0)), page_size, n_pages, _ptr(status), _stream()), "attention prefill")
     return out
+
+
+# Per head size and kernel (one head a block, two): us of a block besides its keys (with a window: more), per step of 64 or 128 keys
+# beside other blocks and alone, of a block whose tile a shorter sequence does not have, the share of a whole round that a last round
+# of equal blocks costs, of a launch, and the share of the longest block that unequal sequences add.
+_Ways = Tuple[float, float, float, float, float, float, float, float]
+PREFILL_COSTS: Dict[int, Tuple[_Ways, _Ways]] = {
+    64: ((4.67, 1.27, 0.987, 0.737, 1.56, 0.89, 4.87, 0.38), (7.07, 2.41, 1.688, 1.583, 0.93, 1.08, 3.57, 0.0)),
+    128: ((5.87, 1.94, 1.063, 0.749, 1.46, 0.76, 5.42, 0.54), (8.55, 2.77, 2.034, 1.898, 0.73, 0.97, 2.64, 0.11))}
+
+
+def two_heads_pay(n_new, kv_lens, n_heads: int, hd: int, window: int, n_sm: int) -> bool:
+    """Whether the prompts of a step run two heads a block (prompts without options, an even number of heads per kv head).
+
+    Such a block has an SM to itself; of those with one head an SM holds two, and there are twice as many.  So two heads pay where
+    tiles of 128 queries see many keys, and lose where they see few (short prompts, windows) or where the last round of the SMs is nearly
+    empty.  The times of both are estimated from the tiles that exist; the estimates' figures are fitted to measurements, 5 to 7 % off.
+    Measured on B200 (us, one head / two; 32 heads on 8), heads of 128 and of 64: one prompt of 1,024 23 / 27 and 21 / 23, of 2,048 52 / 49 and
+    49 / 42, of 4,096 148 / 143 and 134 / 121; 24 of 100 28 / 33 and 25 / 29, 64 of 130 124 / 168 and 104 / 139, eight of 1,000 114 / 128 and
+    98 / 105, six of 50 to 2,000 134 / 118 and 112 / 92; 4,096 under a window of 128 52 / 63 and 45 / 56, of 1,024 94 / 97 and 84 / 85;
+    512 behind 3,000 54 / 66 and 51 / 57."""
+    counts = {}                                                     # tiles by the pages they see
+    n_tiles = most = 0
+    for n, e in zip(n_new, kv_lens):
+        most = max(most, -(-n // 128))
+        for lo in range(e - n, e, 128):
+            pages = (min(lo + 128, e) - 1) // 64 - (max(0, lo + 1 - window) // 64 if window else 0) + 1
+            counts[pages] = counts.get(pages, 0) + 1
+            n_tiles += 1
+    if not n_tiles:
+        return False
+    missing = most * len(n_new) - n_tiles
+
+    def time(heads, slots, step_pages, costs):
+        base, windowed, step, alone, none, last, launch, uneven = costs
+        base += windowed if window else 0.0
+        mean = base + step * sum(-(-p // step_pages) * c for p, c in counts.items()) / n_tiles
+        top = -(-max(counts) // step_pages)
+        longest = base + alone * top
+        rounds = n_tiles * heads / slots
+        us = longest
+        if n_tiles * heads > n_sm:
+            us = max(longest, mean * (rounds + last * (mean / (base + step * top)) ** 3 * (-(-n_tiles * heads // slots) - rounds)))
+        return us + none * heads * missing / slots + (uneven * longest if missing > 0.2 * n_tiles else 0.0) + launch
+
+    # near a tie two heads of 128 come out 2 % too dear, and 4 % for a prompt alone
+    one, two = PREFILL_COSTS[hd]
+    return time(n_heads // 2, n_sm, 2, two) < (1.0 if hd == 64 else 1.04 if len(n_new) == 1 else 1.02) * time(n_heads, 2 * n_sm, 1, one)
+
+
+def _two_heads_of(ctx, n_heads: int, hd: int, window: int) -> bool:
+    """``two_heads_pay`` of a step, once for all its layers of one kind."""
+    key = ("two_heads_pay", n_heads, hd, window)
+    if key not in ctx.shared:
+        ctx.shared[key] = two_heads_pay(ctx.host_n_new, ctx.host_kv_lens, n_heads, hd, window, ops.sm_count())
+    return ctx.shared[key]
 
 
 def decode(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, kv_lens: torch.Tensor, table: torch.Tensor,
@@ -168,5 +227,7 @@ def attend(q, k_pages, v_pages, ctx, table, n_heads: int, scale: float, window: 
             chunk = min(chunk, REACH_CHUNK_PAGES)
         return decode(q, k_pages, v_pages, ctx.kv_lens, table, ctx.n_seqs, ctx.kv_len_bound, n_heads, scale, window,
                       status, chunk_pages=chunk, work=work, **options, softcap=softcap, sink=sink, keep=keep, key_scales=key_scales, slopes=slopes, reach=reach)
+    plain = hd in (64, 128) and key_scales is None and slopes is None and not softcap and not ops.sink_flag(sink) and not keep and n_heads // nkv % 2 == 0
     return prefill(q, k_pages, v_pages, ctx.cu_seqlens, ctx.kv_lens, table, ctx.n_seqs, ctx.max_new, n_heads, scale,
-                   window, status, work=work, softcap=softcap, sink=sink, keep=keep, key_scales=key_scales, slopes=slopes, reach=reach)
+                   window, status, work=work, softcap=softcap, sink=sink, keep=keep, key_scales=key_scales, slopes=slopes, reach=reach,
+                   two_heads=plain and _two_heads_of(ctx, n_heads, hd, int(window or 0)))
