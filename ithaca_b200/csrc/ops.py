@@ -493,8 +493,10 @@ def wide_takes(M: int, N: int, K: int) -> bool:
     the pairs busy with its narrowest tiles of 256 tokens x 128 features.  Measured on B200, other kernel / this one
     (us): 36 tiles' worth and more: 4096 x 4096 at 300 tokens 20.0 / 19.1, 28672 x 4096 at 200 80 / 60, 16384 x 2048 at
     130 29 / 23, 4096 x 14336 at 512 67 / 58, 2048 x 8192 at 768 34 / 32; below: 6144 x 4096 at 130 17.5 / 20.1, 4096 x 14336 at 256
-    49 / 57, 2048 x 8192 at 512 27.5 / 30.5.  Up to 128 tokens the other kernel's slices of K win."""
-    return M > 128 and M * N >= 36 * 256 * 128
+    49 / 57, 2048 x 8192 at 512 27.5 / 30.5.  Up to 128 tokens the other kernel's slices of K win.  With few K steps a tile is mostly
+    its start and its epilogue, and a second tile of 256 tokens for a few of them does not pay: 8192 x 256 at 192 tokens 6.6 / 7.8, at 257
+    7.4 / 8.5, at 400 8.7 / 8.0; 8192 x 512 at 257 8.7 / 9.3, at 400 10.0 / 9.4."""
+    return M > 128 and M * N >= 36 * 256 * 128 and (K >= 1024 or M > 300)
 
 
 _pairs_lib = None

@@ -123,3 +123,37 @@ def test_results_without_an_activation_cost_no_more_than_floats(M, N, K):
             times.append(a.elapsed_time(b))
         best[dtype] = min(times)
     assert best[torch.bfloat16] < 1.25 * best[torch.float32], best
+
+
+def test_which_products_run_on_pairs_of_SMs():
+    takes = ops().wide_takes
+    assert takes(2048, 4096, 4096) and takes(300, 4096, 4096) and takes(130, 28672, 4096)
+    assert not takes(128, 28672, 4096) and not takes(130, 6144, 4096) and not takes(256, 4096, 14336)
+    assert takes(400, 8192, 256) and not takes(192, 8192, 256) and not takes(257, 8192, 512) and takes(257, 8192, 1024)
+
+
+@pytest.mark.parametrize("M,hd,nh,nkv", [(513, 128, 16, 4), (700, 64, 24, 4), (900, 80, 16, 4)])
+def test_rotary_products_as_they_are_dispatched(M, hd, nh, nkv):
+    """Heads of a multiple of 64 go to the pairs of SMs, others to the kernel that takes them."""
+    K, N, n_pages = 1032, (nh + 2 * nkv) * hd, 40
+    x, w = rnd((M, K), 4), rnd((N, K), 5)
+    seq, pos = torch.zeros(M, dtype=torch.int32, device=DEV), torch.arange(M, dtype=torch.int32, device=DEV)
+    table = torch.randperm(n_pages, generator=torch.Generator().manual_seed(1)).to(torch.int32).view(1, n_pages).to(DEV)
+    cos_sin = ops().rope_table(pos, torch.rand(hd // 2, device=DEV))
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    made = []
+    for way in ("dispatched", "wide", "other"):
+        q = torch.zeros((M, nh * hd), dtype=torch.bfloat16, device=DEV)
+        k, v = (torch.zeros((n_pages, nkv, 64, hd), dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        if way == "wide":
+            rs = ops().RopeStore(q.data_ptr(), k.data_ptr(), v.data_ptr(), cos_sin.data_ptr(), seq.data_ptr(), pos.data_ptr(), table.data_ptr(),
+                                 status.data_ptr(), 0, table.stride(0), nh, nkv, hd, 64, n_pages, 1)
+            st = ops().lib().ik_gemm_qkv_rope_wide(x.data_ptr(), w.data_ptr(), M, N, K, K, K, 0, status.data_ptr(), ctypes.byref(rs),
+                                                   torch.cuda.current_stream().cuda_stream)
+            assert st == (-2 if hd % 64 else 0)
+        else:
+            assert ops().gemm_qkv_rope(x, w, q, k, v, cos_sin, seq, pos, table, nh, nkv, hd, True, status, splits=None if way == "dispatched" else 1)
+        made.append((q, k, v))
+    assert status.item() == 0 and ops().wide_takes(M, N, K)
+    for a, b in zip(made[0], made[2 if hd % 64 else 1]):
+        assert torch.equal(a, b) and float(a.float().abs().max()) > 0
