@@ -440,6 +440,11 @@ int wide_width(long long tiles_m, int N, int pairs) {
     return best;
 }
 
+// A grouped plan has a tile to spare for every group, since any group may end in one that is partly filled; on average half of them are
+// in use.  Counted in full they chose the width for work that is not there (us on B200, 8 experts, 4,096 x 14,336, 300 tokens of 2
+// experts each 205 -> 157, 2,048 tokens 626 -> 431; 16 of 1,024 x 512, 600 tokens 10.1 -> 8.6).
+int tiles_in_use(int tiles, int n_groups) { return tiles - n_groups / 2 > 1 ? tiles - n_groups / 2 : 1; }
+
 int wide_impl(const void* X, const void* W, void* Y, int y_dtype, int M, int N, int K, int ldx, int ldw, int ldy, int accumulate,
               IkGlu join, const int* groups, int n_groups, int tile_rows, int bn, int* status, const IkRopeStore* rope, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || K <= 0 || ldx < K || ldw < K || (!rope && ldy < (join ? N / 2 : N))) return IK_BAD_ARGUMENT;
@@ -466,7 +471,7 @@ int wide_impl(const void* X, const void* W, void* Y, int y_dtype, int M, int N, 
     g.tiles_m = (M + cg * ROWS - 1) / (cg * ROWS);
     const int pairs = ik_sm_count() / cg;
     if (pairs < 1) return IK_UNSUPPORTED;
-    g.bn = bn ? bn : wide_width(g.tiles_m, N, pairs);
+    g.bn = bn ? bn : wide_width(tiles_in_use(g.tiles_m, groups ? n_groups : 0), N, pairs);
     if (g.bn != 128 && g.bn != 192 && g.bn != 256) return IK_BAD_ARGUMENT;
     g.tiles_n = (N + g.bn - 1) / g.bn;
     if ((long long)g.tiles_m * g.tiles_n > 0x3fffffff) return IK_UNSUPPORTED;
@@ -524,6 +529,12 @@ IK_EXPORT int ik_gemm_qkv_rope_wide(const void* X, const void* W, int M, int N, 
                                     const IkRopeStore* rope, cudaStream_t stream) {
     if (!rope || !rope->q_out || (rope->hd & 1) || N != (rope->nh + 2 * rope->nkv) * rope->hd) return IK_BAD_ARGUMENT;
     return wide_impl(X, W, nullptr, IK_F32, M, N, K, ldx, ldw, N, 0, IkGlu(), nullptr, 1, 0, bn, status, rope, stream);
+}
+
+// The width of tiles that is chosen for `tiles` token tiles (of which a grouped plan of n_groups keeps some to spare) on so many SMs or pairs.
+IK_EXPORT int ik_gemm_wide_tile_width(int tiles, int n_groups, int N, int pairs) {
+    if (tiles <= 0 || n_groups < 0 || N <= 0 || pairs <= 0) return 0;
+    return wide_width(tiles_in_use(tiles, n_groups), N, pairs);
 }
 
 // Sites: 1 = loader for a free stage, 2 = issuer for a drained accumulator, 3 = issuer for a loaded stage, 4 = epilogue.

@@ -82,6 +82,7 @@ _SIGNATURES = {
     "ik_gemm_wide": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _i, _vp, _vp],
     "ik_gemm_wide_grouped": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp],
     "ik_gemm_qkv_rope_wide": [_vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp],
+    "ik_gemm_wide_tile_width": [_i, _i, _i, _i],
     "ik_gemm_wide_take_wait_record": [_vp],
     "ik_gemm_tcgen05_tile": [_i],
     "ik_gemm_tcgen05_tile_width": [_i, _i],
