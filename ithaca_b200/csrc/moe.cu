@@ -344,6 +344,9 @@ moe_gemm_kernel(const TX* __restrict__ X, const TW* __restrict__ W, TY* __restri
 
 // ------------------------------------------------------------------------------------------ padded order
 // One block.  row_of [A], src_token [n_tiles * bn], tile_group [n_tiles].
+// AT assignments a thread at a time, so that their loads are under way together.  us on B200, one / eight at a time: 16,384 assignments 28 / 25,
+// 8,192 9.3 / 8.7; 2,048 4.8 / 5.2, 128 3.2 / 3.6.
+template <int AT>
 __global__ void __launch_bounds__(1024)
 moe_sort_padded_kernel(const int* __restrict__ chosen, int* __restrict__ row_of, int* __restrict__ src_token,
                        int* __restrict__ tile_group, int A, int E, int top, int bn, int n_tiles, int* __restrict__ src_assign) {
@@ -355,16 +358,25 @@ moe_sort_padded_kernel(const int* __restrict__ chosen, int* __restrict__ row_of,
     for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
     for (int r = threadIdx.x; r < n_tiles * bn; r += blockDim.x) src_token[r] = -1;
     __syncthreads();
-    // eight assignments a thread at a time, so that their loads are under way together (one at a time the block waited for
-    // memory twice per 1,024 assignments: 35 us for 16,384 of them on B200)
-    constexpr int AT = 8;
+    auto count = [&](int e) {
+        if (e >= 0 && e < E) atomicAdd(&cnt[e], 1);
+    };
+    auto place = [&](int a, int e) {
+        if (e < 0 || e >= E) { row_of[a] = 0; return; }
+        const int r = atomicAdd(&cur[e], 1);
+        row_of[a] = r;
+        if (r < n_tiles * bn) {
+            src_token[r] = a / top;
+            if (src_assign) src_assign[r] = a;                // (read only where src_token is not -1)
+        }
+    };
     for (int a0 = threadIdx.x; a0 < A; a0 += AT * 1024) {
+        if (AT == 1) { count(chosen[a0]); continue; }
         int e[AT];
         #pragma unroll
         for (int i = 0; i < AT; i++) e[i] = a0 + i * 1024 < A ? chosen[a0 + i * 1024] : -1;
         #pragma unroll
-        for (int i = 0; i < AT; i++)
-            if (e[i] >= 0 && e[i] < E) atomicAdd(&cnt[e[i]], 1);
+        for (int i = 0; i < AT; i++) count(e[i]);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -377,44 +389,39 @@ moe_sort_padded_kernel(const int* __restrict__ chosen, int* __restrict__ row_of,
     }
     __syncthreads();
     for (int a0 = threadIdx.x; a0 < A; a0 += AT * 1024) {
+        if (AT == 1) { place(a0, chosen[a0]); continue; }
         int e[AT];
         #pragma unroll
-        for (int i = 0; i < AT; i++) e[i] = a0 + i * 1024 < A ? chosen[a0 + i * 1024] : -2;
+        for (int i = 0; i < AT; i++) e[i] = a0 + i * 1024 < A ? chosen[a0 + i * 1024] : -1;
         #pragma unroll
-        for (int i = 0; i < AT; i++) {
-            const int a = a0 + i * 1024;
-            if (a >= A) break;
-            if (e[i] < 0 || e[i] >= E) { row_of[a] = 0; continue; }
-            const int r = atomicAdd(&cur[e[i]], 1);
-            row_of[a] = r;
-            if (r < n_tiles * bn) {
-                src_token[r] = a / top;
-                if (src_assign) src_assign[r] = a;            // (read only where src_token is not -1)
-            }
-        }
+        for (int i = 0; i < AT; i++)
+            if (a0 + i * 1024 < A) place(a0 + i * 1024, e[i]);
     }
 }
 
 // xp[r, :] = x[src_token[r], :], zeros where src_token[r] < 0; rows of d bfloat16, d a multiple of 8
-// Four rows a block: their tokens' numbers are read once, and four rows' loads are under way together.
+// A thread copies the same 16 bytes of ROWS rows, whose tokens' numbers it reads together and whose loads are under way together; a block's rows
+// are blockDim.y times that, its columns blockDim.x (narrow rows share a block).  One row a thread where four would leave SMs idle.
+// us on B200, a flat grid of 16 bytes a thread / blocks of four rows whatever their width / this: 4,096 tokens of 64 (2 of 8 experts) 1.7 /
+// 3.4 / 1.8, 16,384 of 64 2.2 / 9.5 / 2.4, 1,024 of 4,096 5.7 / 7.0 / 5.4, 300 of 2,048 (4 of 32) 3.3 / 3.8 / 3.4, 4,096 of 2,048 19.1 / 15.0 / 15.3.
+template <int ROWS>
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ src_token, uint4* __restrict__ xp, int rows, int d8) {
     ik_pdl_wait();
     IK_AFTER_WAIT(x);
     IK_AFTER_WAIT(src_token);
     ik_pdl_launch_dependents();
-    const int r0 = blockIdx.x * 4;
-    int t[4];
+    const int r0 = (blockIdx.x * blockDim.y + threadIdx.y) * ROWS, c = blockIdx.y * blockDim.x + threadIdx.x;
+    if (c >= d8) return;
+    int t[ROWS];
     #pragma unroll
-    for (int i = 0; i < 4; i++) t[i] = r0 + i < rows ? src_token[r0 + i] : -1;
-    for (int c = threadIdx.x; c < d8; c += 256) {
-        uint4 v[4];
-        #pragma unroll
-        for (int i = 0; i < 4; i++) v[i] = t[i] >= 0 ? x[(size_t)t[i] * d8 + c] : make_uint4(0u, 0u, 0u, 0u);
-        #pragma unroll
-        for (int i = 0; i < 4; i++)
-            if (r0 + i < rows) xp[(size_t)(r0 + i) * d8 + c] = v[i];
-    }
+    for (int i = 0; i < ROWS; i++) t[i] = r0 + i < rows ? src_token[r0 + i] : -1;
+    uint4 v[ROWS];
+    #pragma unroll
+    for (int i = 0; i < ROWS; i++) v[i] = t[i] >= 0 ? x[(size_t)t[i] * d8 + c] : make_uint4(0u, 0u, 0u, 0u);
+    #pragma unroll
+    for (int i = 0; i < ROWS; i++)
+        if (r0 + i < rows) xp[(size_t)(r0 + i) * d8 + c] = v[i];
 }
 
 // The same with every row multiplied by the weight of its assignment (in float, rounded once): xp[r, :] = x[src_token[r], :] *
@@ -465,12 +472,14 @@ __global__ void moe_combine_kernel(const float* __restrict__ parts, const float*
     }
 }
 
-// The same for rows of a multiple of four on 16-byte boundaries, one block per token and four columns a thread: a token's rows and
-// weights are found once, and four rows' loads are under way together (with the gathering four rows a block and the sort eight
-// assignments a thread: a layer of 32 experts, 4 chosen, over 4,096 tokens 2,048 wide 365 -> 329 us on B200).
+// The same for rows of a multiple of four on 16-byte boundaries, four columns a thread: a token's rows and weights are found once, and four
+// rows' loads are under way together.  Threads of a block as in moe_gather_kernel.  us on B200, a flat grid of one column a thread /
+// blocks of one token whatever its width / this: 4,096 tokens of 64 (2 each) 3.0 / 5.2 / 2.0, 16,384 of 256
+// 18.7 / 18.0 / 8.4, 4,096 of 2,048 (4 each) 62 / 33 / 33.
+template <bool NARROW>
 __global__ void __launch_bounds__(256)
 moe_combine4_kernel(const float4* __restrict__ parts, const float* __restrict__ weight, const int* __restrict__ row_of, const float4* __restrict__ extra,
-                    const float* __restrict__ extra_weight, float4* __restrict__ y, int top, int d4, int accumulate) {
+                    const float* __restrict__ extra_weight, float4* __restrict__ y, int T, int top, int d4, int accumulate) {
     ik_pdl_wait();
     IK_AFTER_WAIT(parts);
     IK_AFTER_WAIT(weight);
@@ -478,7 +487,8 @@ moe_combine4_kernel(const float4* __restrict__ parts, const float* __restrict__ 
     IK_AFTER_WAIT(extra);
     IK_AFTER_WAIT(extra_weight);
     ik_pdl_launch_dependents();
-    const size_t t = blockIdx.x;
+    const size_t t = NARROW ? (size_t)blockIdx.x * blockDim.y + threadIdx.y : blockIdx.x;
+    if (NARROW && t >= T) return;
     const float ew = extra && extra_weight ? extra_weight[t] : 1.0f;
     for (int c = threadIdx.x; c < d4; c += 256) {
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -607,15 +617,27 @@ IK_EXPORT int ik_moe_sort_padded(const int* chosen, int* row_of, int* src_token,
                                  int n_tiles, int* src_assign, cudaStream_t stream) {
     if (A < 0 || E <= 0 || top <= 0 || bn <= 0 || n_tiles < 0 || n_tiles < (A / bn + E < A ? A / bn + E : A)) return IK_BAD_ARGUMENT;
     if ((size_t)2 * E * sizeof(int) > 48 * 1024) return IK_UNSUPPORTED;
-    IK_RETURN_IF_ERROR(ik_launch(moe_sort_padded_kernel, 1, 1024, (size_t)2 * E * sizeof(int), stream, chosen, row_of, src_token, tile_group, A, E,
+    IK_RETURN_IF_ERROR(ik_launch(A <= 2048 ? moe_sort_padded_kernel<1> : moe_sort_padded_kernel<8>, 1, 1024, (size_t)2 * E * sizeof(int), stream, chosen, row_of, src_token, tile_group, A, E,
                                  top, bn, n_tiles, src_assign));
     IK_LAUNCH_STATUS();
+}
+
+// Threads of a block of 256 that share a row of n pieces: a power of two.
+static int row_threads(int n) {
+    int w = 1;
+    while (w < n && w < 256) w *= 2;
+    return w;
 }
 
 IK_EXPORT int ik_moe_gather(const void* x, const int* src_token, void* xp, int rows, int d, cudaStream_t stream) {
     if (rows < 0 || d <= 0 || d % 8 || ((uintptr_t)x % 16) || ((uintptr_t)xp % 16)) return IK_BAD_ARGUMENT;
     if (rows == 0) return IK_OK;
-    IK_RETURN_IF_ERROR(ik_launch(moe_gather_kernel, (rows + 3) / 4, 256, 0, stream, (const uint4*)x, src_token, (uint4*)xp, rows, d / 8));
+    const int d8 = d / 8, wide = row_threads(d8), deep = 256 / wide, across = (d8 + wide - 1) / wide;
+    if (across > 65535) return IK_BAD_ARGUMENT;
+    const bool four = (long long)((rows + 4 * deep - 1) / (4 * deep)) * across >= 6LL * ik_sm_count();
+    const int each = four ? 4 * deep : deep;
+    IK_RETURN_IF_ERROR(ik_launch(four ? moe_gather_kernel<4> : moe_gather_kernel<1>, dim3((rows + each - 1) / each, across), dim3(wide, deep), 0, stream,
+                                 (const uint4*)x, src_token, (uint4*)xp, rows, d8));
     IK_LAUNCH_STATUS();
 }
 
@@ -637,8 +659,9 @@ IK_EXPORT int ik_moe_combine(const float* parts, const float* weight, const int*
     if (T == 0) return IK_OK;
     // few tokens are cut by columns over the SMs (the kernel above's flat grid) instead of by tokens
     if (d % 4 == 0 && T >= 2 * ik_sm_count() && ((uintptr_t)parts | (uintptr_t)y | (uintptr_t)extra) % 16 == 0) {
-        IK_RETURN_IF_ERROR(ik_launch(moe_combine4_kernel, T, 256, 0, stream, (const float4*)parts, weight, row_of, (const float4*)extra, extra_weight,
-                                     (float4*)y, top, d / 4, accumulate));
+        const int wide = row_threads(d / 4), deep = 256 / wide;
+        IK_RETURN_IF_ERROR(ik_launch(deep > 1 ? moe_combine4_kernel<true> : moe_combine4_kernel<false>, (T + deep - 1) / deep, dim3(wide, deep), 0, stream, (const float4*)parts, weight, row_of,
+                                     (const float4*)extra, extra_weight, (float4*)y, T, top, d / 4, accumulate));
         IK_LAUNCH_STATUS();
     }
     const size_t total = (size_t)T * d, want = (total + 255) / 256, cap = (size_t)ik_sm_count() * 16;

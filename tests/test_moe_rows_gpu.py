@@ -45,3 +45,35 @@ def test_tokens_in_expert_order(T, top, E, bn, d):
     rest = torch.ones(xp.shape[0], dtype=torch.bool, device=DEV)
     rest[row_of] = False
     assert float(xp[rest].abs().sum()) == 0
+
+
+def test_narrow_rows_cost_what_their_bytes_do():
+    """Rows of 64 against as many bytes in rows of 512: blocks of one row, or four, whatever their width took four to five times as long."""
+    from ithaca_b200.csrc import ops
+
+    def us(call):
+        graph = torch.cuda.CUDAGraph()
+        call()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            for _ in range(20):
+                call()
+        times = []
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            graph.replay()
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b) * 50)
+        return min(times)
+
+    gather, combine = [], []
+    for T, d in ((16384, 64), (2048, 512)):
+        chosen = torch.stack([torch.randperm(8, generator=torch.Generator().manual_seed(i))[:2] for i in range(T)]).to(torch.int32).to(DEV)
+        plan = ops.moe_sort_padded(chosen, 8, 128)
+        x, parts = torch.ones(T, d, dtype=torch.bfloat16, device=DEV), torch.ones(plan.rows, d, device=DEV)
+        weight, out = torch.ones(T, 2, device=DEV), torch.empty(T, d, device=DEV)
+        gather.append(us(lambda: ops.moe_gather(x, plan)))
+        combine.append(us(lambda: ops.moe_combine(parts, weight, out=out, row_of=plan.row_of)))
+    assert gather[0] < 2.5 * gather[1] and combine[0] < 2.5 * combine[1], (gather, combine)
