@@ -97,24 +97,33 @@ def attend(q: torch.Tensor, k_pages: torch.Tensor, ctx, table: torch.Tensor, n_h
     return out
 
 
-PROMPT_KEYS_MOST = 1 << 16        # keys of a step whose heads' keys and values are formed: 8 or 16 KB each with 16 or 32 heads, 1 GB at most
+PROMPT_BYTES_MOST = 1 << 30       # of formed keys, values and gathered latents at a time: sequences take turns where a step's are more
 FORM_KEYS_QUERIES = 64
 
 
-def forms_keys(ctx, k_pages: torch.Tensor, dtype: torch.dtype, dk: int, dr: int, dv: int, rank: int, window: int = 0) -> bool:
+def formed_bytes(keys: int, n_heads: int, rank: int) -> int:
+    """What ``prompt`` allocates for a sequence of so many keys: a latent, and every head's key and value of 128, in whole pages."""
+    return -(-keys // 64) * 64 * 2 * (rank + 256 * n_heads)
+
+
+def forms_keys(ctx, k_pages: torch.Tensor, dtype: torch.dtype, dk: int, dr: int, dv: int, rank: int, window: int = 0, n_heads: int = 32,
+               scale: float = 1.0) -> bool:
     """Whether a step's attention goes over keys and values formed per head (``prompt``) rather than over the cached rows.  Forming
     them costs heads x rank x (dk + dv) products a key; a query that sees the key then saves 2 rank - dk - dv of the 2 rank + dr
     products per head (768 of 1,088), and runs on tcgen05.  Measured on B200 (rank 512, one sequence; us for the layer, over the rows /
     formed): 16 heads, 64 new tokens behind 2,000 190 / 155, 512 behind 2,000 371 / 168, 4,096 from the start 2,056 / 348; 32 heads,
-    64 behind 2,000 228 / 183, 512 behind 2,000 674 / 245; below 64 not measured.  Under a window a query sees that many keys at
-    most, while every key is formed."""
+    64 behind 2,000 228 / 183, 512 behind 2,000 674 / 245; below 64 not measured.  With a rank of 64 a query saves no products, only the kernel's
+    rate: 32 heads, 16 sequences of 64 behind 500 203 / 217, one of 512 behind 2,000 245 / 188, so twice as many queries are asked for.  Under a window a query sees that many keys at
+    most, while every key is formed.  A sequence whose formed keys and values alone exceed ``PROMPT_BYTES_MOST`` (1 GB: 61,680 keys with 32
+    heads, 16,131 with 128) goes over the rows, with the others of its step."""
     if dtype != torch.bfloat16 or k_pages.dtype != torch.bfloat16 or ctx.is_decode or k_pages.shape[1:3] != (1, 64):
         return False
-    if dk != 128 or dv != 128 or dr not in (0, 64) or rank % 64 or k_pages.shape[3] != rank + dr:
+    if dk != 128 or dv != 128 or dr not in (0, 64) or rank % 64 or k_pages.shape[3] != rank + dr or not scale > 0:
         return False
     lens, new = ctx.host_kv_lens, ctx.host_n_new
     keys = sum(lens)
-    return len(lens) == ctx.n_seqs and keys <= PROMPT_KEYS_MOST and sum(n * min(e, window or e) for n, e in zip(new, lens)) >= FORM_KEYS_QUERIES * keys
+    return len(lens) == ctx.n_seqs and all(formed_bytes(e, n_heads, rank) <= PROMPT_BYTES_MOST for e in lens) and sum(n * min(e, window or e) for n, e in zip(new, lens)) >= \
+        FORM_KEYS_QUERIES * (2 if rank < 128 else 1) * keys
 
 
 def prompt(q_plain: torch.Tensor, q_full: torch.Tensor, k_pages: torch.Tensor, w_kv: torch.Tensor, ctx, table: torch.Tensor, n_heads: int,
@@ -123,19 +132,29 @@ def prompt(q_plain: torch.Tensor, q_full: torch.Tensor, k_pages: torch.Tensor, w
     key matrices, then their value matrices.  Returns the heads' results [T, heads * 128]."""
     from . import gemm_bf16
     n_pages, _, _, hd = k_pages.shape
-    T, B = q_plain.shape[0], ctx.n_seqs
-    n_keys = sum(-(-e // 64) * 64 for e in ctx.host_kv_lens)
+    T, lens = q_plain.shape[0], ctx.host_kv_lens
     lib = ops.lib()
-    latents = torch.empty((n_keys, rank), dtype=torch.bfloat16, device=q_plain.device)
-    ops._work(f"latent_gather {n_keys}x{rank}", 2 * ops._nbytes(latents))
-    _check(lib.ik_latent_gather(_ptr(k_pages), _ptr(ctx.cu_seqlens), _ptr(ctx.kv_lens), _ptr(table), table.stride(0), _ptr(latents), B, ctx.max_kv_len,
-                                hd, rank, int(window or 0), n_pages, _ptr(status), _stream()), "latent_gather")
-    kv = gemm_bf16.gemm(latents, w_kv, out_dtype=torch.bfloat16)
     out = torch.empty((T, n_heads * 128), dtype=torch.bfloat16, device=q_plain.device)
-    if ops.profiling():
-        pairs = sum(min(p + 1, window) if window else p + 1 for n, e in zip(ctx.host_n_new, ctx.host_kv_lens) for p in range(e - n, e))
-        ops._work(f"attention latent prompt {T}x{n_heads}", ops._nbytes(q_plain, out, kv), 2 * pairs * n_heads * (256 + hd - rank))
-    _check(lib.ik_latent_prompt(_ptr(q_plain), _ptr(q_full), _ptr(kv), _ptr(k_pages), _ptr(out), _ptr(ctx.cu_seqlens), _ptr(ctx.kv_lens), _ptr(table),
-                                table.stride(0), T, B, ctx.max_new, n_keys, n_heads, hd, rank, scale, int(window or 0), n_pages, _ptr(status),
-                                _stream()), "attention latent prompt")
+    first = 0
+    while first < ctx.n_seqs:                             # as many sequences at a time as ``PROMPT_BYTES_MOST`` has room for
+        end, used = first, 0
+        while end < ctx.n_seqs and (end == first or used + formed_bytes(lens[end], n_heads, rank) <= PROMPT_BYTES_MOST):
+            used += formed_bytes(lens[end], n_heads, rank)
+            end += 1
+        B, n_keys, longest = end - first, sum(-(-e // 64) * 64 for e in lens[first:end]), max(lens[first:end])
+        cu_seqlens, kv_lens, rows = ctx.cu_seqlens[first:], ctx.kv_lens[first:], table[first:]
+        latents = torch.empty((n_keys, rank), dtype=torch.bfloat16, device=q_plain.device)
+        ops._work(f"latent_gather {n_keys}x{rank}", 2 * ops._nbytes(latents))
+        _check(lib.ik_latent_gather(_ptr(k_pages), _ptr(cu_seqlens), _ptr(kv_lens), _ptr(rows), rows.stride(0), _ptr(latents), B, longest,
+                                    hd, rank, int(window or 0), n_pages, _ptr(status), _stream()), "latent_gather")
+        kv = gemm_bf16.gemm(latents, w_kv, out_dtype=torch.bfloat16)
+        if ops.profiling():
+            pairs = sum(min(p + 1, window) if window else p + 1
+                        for n, e in zip(ctx.host_n_new[first:end], lens[first:end]) for p in range(e - n, e))
+            ops._work(f"attention latent prompt {T}x{n_heads}", ops._nbytes(q_plain, out, kv), 2 * pairs * n_heads * (256 + hd - rank))
+        _check(lib.ik_latent_prompt(_ptr(q_plain), _ptr(q_full), _ptr(kv), _ptr(k_pages), _ptr(out), _ptr(cu_seqlens), _ptr(kv_lens), _ptr(rows),
+                                    rows.stride(0), T, B, ctx.max_new, n_keys, n_heads, hd, rank, scale, int(window or 0), n_pages, _ptr(status),
+                                    _stream()), "attention latent prompt")
+        del latents, kv                                   # the next sequences' are made where these were
+        first = end
     return out

@@ -37,7 +37,7 @@ from .linear import Linear
 
 
 class LatentAttention:
-    graph_safe = True       # reads slots, positions and lengths from device arrays only
+    graph_safe = True       # decode steps read slots, positions and lengths from device arrays only (prompts size buffers by the host's lengths)
 
     @classmethod
     def manifest(cls, spec: PartSpec) -> Dict[str, TensorReq]:
@@ -101,11 +101,11 @@ class LatentAttention:
         uv = to_device(tensors[w["uv"]], runtime)
         # per head: Wuk^T [rank, dk] multiplies the plain query; Wuv [dv, rank] multiplies the head's sum of latents
         self.uk_t = uk.view(H, dk, rank).transpose(1, 2).contiguous().to(wdt or uk.dtype)
-        self.uv = uv.view(H, dv, rank).contiguous().to(wdt or uv.dtype)
+        # prompts: one product forms every head's plain keys and values from the rows (see ``attention_latent.prompt``); its lower half is Wuv
+        self.w_kv = torch.cat([uk.to(wdt), uv.to(wdt)], dim=0).contiguous() if wdt is not None and dk == dv == 128 else None
+        self.uv = (uv.contiguous().to(wdt or uv.dtype) if self.w_kv is None else self.w_kv[H * dk:]).view(H, dv, rank)
         self.c_norm_w = as_float32(tensors[w["dkv_norm"]], runtime) if self.own_latent else None
         self.runtime = runtime
-        # prompts: one product forms every head's plain keys and values from the rows (see ``attention_latent.prompt``)
-        self.w_kv = torch.cat([uk.to(wdt), uv.to(wdt)], dim=0).contiguous() if wdt is not None and dk == dv == 128 else None
 
     def cache_requests(self) -> List[object]:
         # one key/value head whose rows are [latent | turned key part]; the values are the rows' leading kv_rank columns
@@ -130,7 +130,7 @@ class LatentAttention:
             q_plain = torch.empty((T, H * dk), dtype=rt.act_dtype, device=x.device)
             ops.latent_prepare(p, 0, self.c_off, self.c_norm_w, self.norm_eps, q_plain, q_full, cache.k_pages, ctx.token_seq,
                                ctx.token_pos, table, self.position.inv_freq if dr else None, H, dk, dr, rank, writes_cache, rt.status)
-        if self.w_kv is not None and attention_latent.forms_keys(ctx, cache.k_pages, rt.act_dtype, dk, dr, dv, rank, self.window or 0):
+        if self.w_kv is not None and attention_latent.forms_keys(ctx, cache.k_pages, rt.act_dtype, dk, dr, dv, rank, self.window or 0, H, self.scale):
             heads = attention_latent.prompt(q_plain, q_full, cache.k_pages, self.w_kv, ctx, table, H, rank, self.scale, self.window or 0, rt.status)
             if self.gate:
                 ops.head_gate(heads, p, self.g_off, heads, H, wide=True)
