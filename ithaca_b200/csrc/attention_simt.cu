@@ -186,17 +186,18 @@ IK_EXPORT int ik_attention_simt(const void* q, int q_dtype, const void* k_pages,
     if (T < 0 || nh <= 0 || nkv <= 0 || nh % nkv || hd <= 0 || hdv <= 0 || hdv > TILE * MAX_R || page_size <= 0 || softcap < 0.f || keep < 0) return IK_BAD_ARGUMENT;
     if (q_dtype != out_dtype) return IK_BAD_ARGUMENT;
     if (T == 0) return IK_OK;
-    // Heads per block: as many of a kv head's as there are in fours or twos, as long as their values fit the threads and the
+    // Heads per block: as many of a kv head's as there are in fours or twos, as long as their values fit the threads, their queries the shared memory, and the
     // blocks still go four times around the SMs (300 tokens, float32, one head / these: 32 heads of 64 on 8 kv heads 620 / 144 us,
     // 200 tokens, 16 heads of 128 on 4 336 / 109).
     const int group = nh / nkv;
+    auto bytes = [&](int n) { return TILE * sizeof(size_t) + (size_t)n * (TILE + 4 + hd) * sizeof(float); };    // of shared memory
     int ng = 1;
     for (int n = 4; n > 1; n /= 2)
-        if (ng == 1 && group % n == 0 && n * hdv <= TILE * MAX_R && (long long)T * nh / n >= 4LL * ik_sm_count()) ng = n;
+        if (ng == 1 && group % n == 0 && n * hdv <= TILE * MAX_R && (long long)T * nh / n >= 4LL * ik_sm_count() && bytes(n) <= 48 * 1024) ng = n;
     const int size = cache_dtype == IK_F32 ? 4 : 2;
     const int vec = hd % 4 == 0 && ((uintptr_t)k_pages % (4 * size)) == 0;
     dim3 grid(T, nh / ng);
-    const size_t smem = TILE * sizeof(size_t) + (size_t)ng * (TILE + 4 + hd) * sizeof(float);
+    const size_t smem = bytes(ng);
 #define IK_ATT_N(TQ, TC, NG)                                                                                          \
     IK_RETURN_IF_ERROR(ik_launch(attention_simt_kernel<TQ, TC, TQ, NG>, grid, TILE, smem, stream, (const TQ*)q, (const TC*)k_pages, (const TC*)v_pages, \
         (TQ*)out, token_seq, token_pos, table, table_stride, nh, nkv, hd, hdv, ldv, scale, softcap, window, keep, sink, sink_v, key_scales, slopes, page_size, n_pages, status, vec))
