@@ -356,6 +356,18 @@ __device__ __forceinline__ void tanh_series_f32x2(float& x0, float& x1, float b)
     asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(y));
 }
 
+// After a wait that gave up: leaves no copy in flight.  armed_k, armed_v: copies of keys and values asked for, NS stages each.
+template <int NS>
+__device__ __forceinline__ void wait_for_copies(uint64_t* q_full, uint64_t* k_full, int armed_k, uint64_t* v_full, int armed_v) {
+    auto wait = [](uint64_t* bar, uint32_t parity) {
+        const long long c0 = wait_clock();
+        while (!mbar_test(bar, parity) && !wait_ran_out(c0, 2000000ull)) {}
+    };
+    wait(q_full, 0);
+    for (int i = max(0, armed_k - NS); i < armed_k; i++) wait(k_full + i % NS, (i / NS) & 1);
+    for (int i = max(0, armed_v - NS); i < armed_v; i++) wait(v_full + i % NS, (i / NS) & 1);
+}
+
 __global__ void __launch_bounds__(192, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, bf16* __restrict__ out,
@@ -450,6 +462,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             if (page < 0 || page >= n_pages) { ik_set_status(status, IK_STATUS_READ_NO_PAGE); page = 0; }
             return (page * nkv + kvh) * PAGE;
         };
+        int armed_k = 0, armed_v = 0;
         // rows that are keys and values: one ring, a stage is free once O += P V has read it
         for (int i = 0; ONE_ROW && i < n_iter; i++) {
             const int s = i % TC_NS;
@@ -460,6 +473,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 bulk_load(Cs + s * PAGE, key_scales + row, PAGE * 4, k_full + s);
             }
             __syncwarp();
+            armed_k = i + 1;
         }
         // keys of page i, then values of page i - 1
         for (int i = 0, row = 0, row_before = 0; !ONE_ROW && i <= n_iter; i++, row_before = row) {
@@ -469,14 +483,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 row = page_row(i);
                 if (elect_one()) load_page(Ks + s * TC_KV_BYTES, &map_k, row, k_full + s, TC_KV_BYTES);
                 __syncwarp();
+                armed_k = i + 1;
             }
             if (i > 0) {
                 const int s = (i - 1) % TC_NS;
                 if (!wait_all(v_free + s, (((i - 1) / TC_NS) & 1) ^ 1, 12, i)) break;
                 if (elect_one()) load_page(Vs + s * TC_KV_BYTES, &map_v, row_before, v_full + s, TC_KV_BYTES);
                 __syncwarp();
+                armed_v = i;
             }
         }
+        if (*abort_flag && lane == 0) wait_for_copies<TC_NS>(q_full, k_full, armed_k, v_full, armed_v);
     } else if (warp == 1) {
         const uint32_t idesc_qk = umma_idesc(PAGE), idesc_pv = umma_idesc(HD, 1);
         const uint32_t q_addr = smem_u32(Qs);
@@ -800,18 +817,7 @@ attn_prompt_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 armed_v = i;
             }
         }
-        if (*abort_flag && lane == 0) {                        // leave no copy in flight
-            const long long c0 = wait_clock();
-            while (!mbar_test(q_full, 0) && !wait_ran_out(c0, 2000000ull)) {}
-            for (int i = max(0, armed_k - TP_NS); i < armed_k; i++) {
-                const long long c1 = wait_clock();
-                while (!mbar_test(k_full + i % TP_NS, (i / TP_NS) & 1) && !wait_ran_out(c1, 2000000ull)) {}
-            }
-            for (int i = max(0, armed_v - TP_NS); i < armed_v; i++) {
-                const long long c1 = wait_clock();
-                while (!mbar_test(v_full + i % TP_NS, (i / TP_NS) & 1) && !wait_ran_out(c1, 2000000ull)) {}
-            }
-        }
+        if (*abort_flag && lane == 0) wait_for_copies<TP_NS>(q_full, k_full, armed_k, v_full, armed_v);
     } else if (warp == 1) {
         const uint32_t idesc_qk = umma_idesc(TP_KEYS), idesc_pv = umma_idesc(HD, 1);
         auto scores = [&](int t, int i) {                      // of head t against step i's keys (which have been waited for)

@@ -152,7 +152,8 @@ ssd_tc_kernel(const __grid_constant__ CUtensorMap map_u, const float* __restrict
     if (warp == 0) {
         if (lane == 0) {
             const int x_off = h * P + p0, b_off = H * P + grp * NS, c_off = H * P + G * NS + grp * NS;
-            for (int c = 0; c < n_chunks; c++) {
+            int armed = 0;
+            for (int c = 0; c < n_chunks; c++, armed = c) {
                 const int s = c & 1;
                 if (!mbar_wait(freed + s, ((c >> 1) & 1) ^ 1, abort_flag, status, lim, 31, c)) break;
                 unsigned char* st = smem + s * SB;
@@ -161,6 +162,11 @@ ssd_tc_kernel(const __grid_constant__ CUtensorMap map_u, const float* __restrict
                 for (int k = 0; k < BOXES; k++) tma_load_2d(st + (BOXES + k) * TILE_BYTES, &map_u, b_off + k * 64, lo + c * Q, full + s);
                 tma_load_2d(st + 2 * BOXES * TILE_BYTES, &map_u, x_off, lo + c * Q, full + s);
             }
+            if (*abort_flag)                                   // leave no copy in flight
+                for (int c = max(0, armed - 2); c < armed; c++) {
+                    const long long c0 = wait_clock();
+                    while (!mbar_test(full + (c & 1), (c >> 1) & 1) && !wait_ran_out(c0, 2000000ull)) {}
+                }
         }
     } else if (warp == 1) {
         if (lane == 0) {
