@@ -17,7 +17,8 @@ from ..csrc import ops
 
 def measure_peaks(device: str = "cuda:0", copy_mib: int = 1024, gemm_n: int = 8192, reps: int = 10) -> Dict[str, float]:
     """``hbm_gbs``: read + write bytes of a copy of ``copy_mib`` MiB (larger than the L2 cache) over its time, the
-    best of ``reps``.  ``bf16_tflops``: a bfloat16 product of gemm_n^3 on the tcgen05 kernel, the best of ``reps``.
+    best of ``reps``.  ``bf16_tflops``: a bfloat16 product of gemm_n^3 on the tcgen05 kernel that the dispatcher
+    takes for it, the best of ``reps``.
     Both with this library's kernels, timed with CUDA events."""
     torch.cuda.set_device(device)
     src = torch.empty(copy_mib << 20, dtype=torch.uint8, device=device)
@@ -42,7 +43,7 @@ def measure_peaks(device: str = "cuda:0", copy_mib: int = 1024, gemm_n: int = 81
     for r in range(reps + 2):
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         a.record()
-        if ops.gemm_tcgen05(x, w, out=y, status=status, splits=1) is None:
+        if ops.gemm_tcgen05(x, w, out=y, status=status) is None:
             raise ops.KernelError("the tcgen05 product refused the peak measurement's sizes")
         b.record()
         torch.cuda.synchronize()
