@@ -124,8 +124,8 @@ def prefill(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, cu_se
 # of equal blocks costs, of a launch, and the share of the longest block that unequal sequences add.
 _Ways = Tuple[float, float, float, float, float, float, float, float]
 PREFILL_COSTS: Dict[int, Tuple[_Ways, _Ways]] = {
-    64: ((4.67, 1.27, 0.987, 0.737, 1.56, 0.89, 4.87, 0.38), (7.07, 2.41, 1.688, 1.583, 0.93, 1.08, 3.57, 0.0)),
-    128: ((5.87, 1.94, 1.063, 0.749, 1.46, 0.76, 5.42, 0.54), (8.55, 2.77, 2.034, 1.898, 0.73, 0.97, 2.64, 0.11))}
+    64: ((4.75, 1.37, 1.028, 0.743, 1.64, 0.80, 4.31, 0.27), (7.04, 2.39, 1.722, 1.594, 0.90, 1.06, 3.65, 0.05)),
+    128: ((6.04, 1.96, 1.086, 0.757, 1.56, 0.70, 4.58, 0.30), (8.51, 2.67, 2.051, 1.907, 0.74, 1.03, 2.63, 0.09))}
 
 
 def two_heads_pay(n_new, kv_lens, n_heads: int, hd: int, window: int, n_sm: int) -> bool:
@@ -160,11 +160,11 @@ def two_heads_pay(n_new, kv_lens, n_heads: int, hd: int, window: int, n_sm: int)
         us = longest
         if n_tiles * heads > n_sm:
             us = max(longest, mean * (rounds + last * (mean / (base + step * top)) ** 3 * (-(-n_tiles * heads // slots) - rounds)))
-        return us + none * heads * missing / slots + (uneven * longest if missing > 0.2 * n_tiles else 0.0) + launch
+        return us + none * heads * missing / slots + uneven * longest * min(1.0, 2.5 * missing / n_tiles) + launch
 
-    # near a tie two heads of 128 come out 2 % too dear, and 4 % for a prompt alone
+    # near a tie two heads of 64 come out 2 % too cheap, and two of 128 4 % too dear for a prompt alone
     one, two = PREFILL_COSTS[hd]
-    return time(n_heads // 2, n_sm, 2, two) < (1.0 if hd == 64 else 1.04 if len(n_new) == 1 else 1.02) * time(n_heads, 2 * n_sm, 1, one)
+    return time(n_heads // 2, n_sm, 2, two) < (0.98 if hd == 64 else 1.04 if len(n_new) == 1 else 1.0) * time(n_heads, 2 * n_sm, 1, one)
 
 
 def _two_heads_of(ctx, n_heads: int, hd: int, window: int) -> bool:
