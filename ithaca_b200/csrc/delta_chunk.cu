@@ -19,7 +19,10 @@ constexpr int C = 64;                                    // tokens of a chunk
 constexpr int TLD = C + 4;                               // row stride of T and P in shared memory
 constexpr int VEC = 132;                                 // floats of a chunk's decays: G [64], G_end / G [64], G_end, padding
 
-// Only sequences of at least `least` (> 0) tokens are walked, and their chunks numbered, in the order of the sequences.
+// SOME: only sequences of at least `least` (> 0) tokens are walked, and their chunks numbered, in the order of the sequences.  Otherwise all
+// are, and chunk j of sequence b has the number cu_seqlens[b] / 64 + b + j (instances of their own: the walk takes 2 % longer where its
+// sequence is looked for).
+__device__ __forceinline__ int chunk_base(const int* cu_seqlens, int b) { return cu_seqlens[b] / C + b; }
 struct Walked {
     int b, chunk0;                                       // the sequence (-1: there is none), the number of its first chunk
 };
@@ -39,11 +42,8 @@ __device__ __forceinline__ Walked walked_sequence(const int* cu_seqlens, int n_s
         }
         const unsigned all = __ballot_sync(0xffffffffu, mine);
         const bool it = mine && (BY_CHUNK ? i < chunks + upto && i >= chunks + upto - own : seen + __popc(all & ((1u << lane) - 1)) == i);
-        const unsigned found = __ballot_sync(0xffffffffu, it);
-        if (found) {
-            const int at = __ffs(found) - 1;
-            return {b0 + at, __shfl_sync(0xffffffffu, chunks + upto - own, at)};
-        }
+        const int found = __reduce_max_sync(0xffffffffu, it ? b : -1);
+        if (found >= 0) return {found, __reduce_max_sync(0xffffffffu, it ? chunks + upto - own : -1)};
         seen += __popc(all);
         chunks += __shfl_sync(0xffffffffu, upto, 31);
     }
@@ -59,7 +59,7 @@ __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_grou
 __device__ __forceinline__ float4 at4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
 // One block per (chunk, value head).
-template <int DK>
+template <int DK, bool SOME>
 __global__ void __launch_bounds__(256)
 delta_chunk_prepare_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, const float* __restrict__ bg, float* __restrict__ scratch,
                            float* __restrict__ vecs, const int* __restrict__ cu_seqlens, int n_seqs, int least, int H, int G) {
@@ -77,9 +77,20 @@ delta_chunk_prepare_kernel(const float* __restrict__ u, int ldu, int q_off, int 
     IK_AFTER_WAIT(cu_seqlens);
     ik_pdl_launch_dependents();
     const int tid = threadIdx.x, h = blockIdx.y, f = blockIdx.x;
-    const Walked seq = walked_sequence<true>(cu_seqlens, n_seqs, least, f);
-    if (seq.b < 0) return;
+    Walked seq = {0, 0};
+    if (SOME) {
+        seq = walked_sequence<true>(cu_seqlens, n_seqs, least, f);
+        if (seq.b < 0) return;
+    } else {
+        for (int high = n_seqs - 1; seq.b < high;) {         // the last sequence whose first chunk is not behind this one
+            const int mid = (seq.b + high + 1) >> 1;
+            if (chunk_base(cu_seqlens, mid) <= f) seq.b = mid;
+            else high = mid - 1;
+        }
+        seq.chunk0 = chunk_base(cu_seqlens, seq.b);
+    }
     const int t0 = cu_seqlens[seq.b] + (f - seq.chunk0) * C, n = min(C, cu_seqlens[seq.b + 1] - t0);
+    if (n <= 0) return;
     const int kvh = h / (H / G);
     for (int i = tid; i < 2 * C * (DK / 4); i += 256) {
         const int r = i / (DK / 4), w = i % (DK / 4), t = r & (C - 1);
@@ -194,7 +205,7 @@ struct Walk {
     static constexpr int FLOATS = 4 * C * LD + C * TLD + 2 * C * TLD + 3 * C * DS + DK * DS + 2 * VEC;
 };
 
-template <int DK, int DS>
+template <int DK, int DS, bool SOME>
 __global__ void __launch_bounds__(256, 1)
 delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, int v_off, const float* __restrict__ scratch, const float* __restrict__ vecs,
                    float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ cu_seqlens,
@@ -218,10 +229,14 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
     IK_AFTER_WAIT(cu_seqlens);
     IK_AFTER_WAIT(kv_lens);
     ik_pdl_launch_dependents();
-    const Walked seq = walked_sequence<false>(cu_seqlens, n_seqs, least, blockIdx.z);
-    if (seq.b < 0) return;
+    Walked seq = {(int)blockIdx.z, 0};
+    if (SOME) {
+        seq = walked_sequence<false>(cu_seqlens, n_seqs, least, blockIdx.z);
+        if (seq.b < 0) return;
+    }
     const int tid = threadIdx.x, b = seq.b, h = blockIdx.y, col0 = blockIdx.x * DS;
     const int lo = cu_seqlens[b], hi = cu_seqlens[b + 1], end = kv_lens[b], start = end - (hi - lo);
+    if (!SOME && hi <= lo) return;
     const int tx = tid % W::CG, ty = tid / W::CG, kvh = h / (H / G);
     const int col = col0 + 4 * tx, k0 = RS * ty;
     auto row = [&](int i) { return i == 0 ? ty : C - 1 - ty; };
@@ -230,7 +245,7 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
     const size_t per = (size_t)H * DK * dv;
     const float* st_in = state + ((size_t)slots[b] * 2 + ((start - 1) & 1)) * per + ((size_t)h * dv + (live ? col : 0)) * DK + k0;
     float* st_out = state + ((size_t)slots[b] * 2 + ((end - 1) & 1)) * per + ((size_t)h * dv + (live ? col : 0)) * DK + k0;
-    const int f0 = seq.chunk0, n_chunks = (hi - lo + C - 1) / C;
+    const int f0 = SOME ? seq.chunk0 : chunk_base(cu_seqlens, b), n_chunks = (hi - lo + C - 1) / C;
 
     auto bring_kq = [&](int j) {
         float* dst = KQ + (j & 1) * 2 * C * LD;
@@ -379,31 +394,31 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
     }
 }
 
-template <int DK, int DS>
+template <int DK, int DS, bool SOME>
 int walk(const float* u, int ldu, int q_off, int k_off, int v_off, const float* scratch, const float* vecs, float* state, const int* slots,
          const int* cu_seqlens, const int* kv_lens, float* out, int B, int least, int n_walked, int H, int G, int dv, cudaStream_t stream) {
     constexpr size_t smem = Walk<DK, DS>::FLOATS * sizeof(float);
-    const cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<DK, DS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<DK, DS, SOME>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    IK_RETURN_IF_ERROR(ik_launch(delta_chunk_kernel<DK, DS>, dim3((dv + DS - 1) / DS, H, n_walked), 256, smem, stream, u, ldu, q_off, k_off, v_off,
+    IK_RETURN_IF_ERROR(ik_launch(delta_chunk_kernel<DK, DS, SOME>, dim3((dv + DS - 1) / DS, H, n_walked), 256, smem, stream, u, ldu, q_off, k_off, v_off,
                                  scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, H, G, dv));
     IK_LAUNCH_STATUS();
 }
 
-template <int DK>
+template <int DK, bool SOME>
 int chunks(const float* u, int ldu, int q_off, int k_off, int v_off, const float* bg, float* scratch, float* state, const int* slots,
            const int* cu_seqlens, const int* kv_lens, float* out, int B, int least, int n_walked, int n_chunks, int H, int G, int dv,
            cudaStream_t stream) {
     float* vecs = scratch + (size_t)n_chunks * H * 2 * C * C;
     constexpr size_t smem = (2 * C * (DK + 4) + 2 * C * TLD + C) * sizeof(float) + C * sizeof(double);
-    const cudaError_t e = cudaFuncSetAttribute(delta_chunk_prepare_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(delta_chunk_prepare_kernel<DK, SOME>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    IK_RETURN_IF_ERROR(ik_launch(delta_chunk_prepare_kernel<DK>, dim3(n_chunks, H), 256, smem, stream, u, ldu, q_off, k_off, bg, scratch, vecs,
+    IK_RETURN_IF_ERROR(ik_launch(delta_chunk_prepare_kernel<DK, SOME>, dim3(n_chunks, H), 256, smem, stream, u, ldu, q_off, k_off, bg, scratch, vecs,
                                  cu_seqlens, B, least, H, G));
     // 32 columns a block do a third fewer loads per multiply-add; 16 where that leaves more than half of the SMs idle
     if (2LL * n_walked * H * ((dv + 31) / 32) <= ik_sm_count())
-        return walk<DK, 16>(u, ldu, q_off, k_off, v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, H, G, dv, stream);
-    return walk<DK, 32>(u, ldu, q_off, k_off, v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, H, G, dv, stream);
+        return walk<DK, 16, SOME>(u, ldu, q_off, k_off, v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, H, G, dv, stream);
+    return walk<DK, 32, SOME>(u, ldu, q_off, k_off, v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, H, G, dv, stream);
 }
 
 }  // namespace
@@ -416,16 +431,22 @@ IK_EXPORT long long ik_delta_chunks_scratch(int T, int B, int max_new, int H, in
 }
 
 // As ik_delta_rule, a chunk of tokens at a time, for the sequences that bring at least `least` tokens (the others are left alone): at
-// most n_walked of them, of at most n_chunks chunks together, for which scratch has room.  IK_UNSUPPORTED where rows of q, k or v are not
-// on 16 bytes.
+// most n_walked of them, of at most n_chunks chunks together, for which scratch has room.  least 1: all of them, n_walked = B and n_chunks =
+// T / 64 + B.  IK_UNSUPPORTED where rows of q, k or v are not on 16 bytes.
 IK_EXPORT int ik_delta_chunks(const float* u, int ldu, int q_off, int k_off, int v_off, const float* bg, float* state, const int* slots,
                               const int* cu_seqlens, const int* kv_lens, float* out, float* scratch, int T, int B, int least, int n_walked,
                               int n_chunks, int H, int G, int dk, int dv, cudaStream_t stream) {
     if (T < 0 || B < 0 || least <= 0 || n_walked < 0 || n_chunks < 0 || n_walked > 65535 || H <= 0 || G <= 0 || H % G || dv <= 0 || !state || !bg ||
         !scratch) return IK_BAD_ARGUMENT;
+    if (least == 1 && (n_walked != B || n_chunks != T / C + B)) return IK_BAD_ARGUMENT;
     if (T == 0 || B == 0 || n_walked == 0 || n_chunks == 0) return IK_OK;
     if (ldu % 4 || q_off % 4 || k_off % 4 || v_off % 4 || dv % 4 || ((uintptr_t)u | (uintptr_t)out | (uintptr_t)scratch) % 16) return IK_UNSUPPORTED;
-    if (dk == 128) return chunks<128>(u, ldu, q_off, k_off, v_off, bg, scratch, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, n_chunks, H, G, dv, stream);
-    if (dk == 64) return chunks<64>(u, ldu, q_off, k_off, v_off, bg, scratch, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, n_chunks, H, G, dv, stream);
+#define IK_CHUNKS(DK)                                                                                                                       \
+    if (dk == DK)                                                                                                                           \
+        return (least == 1 ? chunks<DK, false> : chunks<DK, true>)(u, ldu, q_off, k_off, v_off, bg, scratch, state, slots, cu_seqlens, kv_lens, out, B, \
+                                                                   least, n_walked, n_chunks, H, G, dv, stream)
+    IK_CHUNKS(128);
+    IK_CHUNKS(64);
+#undef IK_CHUNKS
     return IK_UNSUPPORTED;
 }

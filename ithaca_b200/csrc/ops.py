@@ -1439,10 +1439,10 @@ def delta_chunks_from(n_new, n_heads: int, dk: int, dv: int, n_sm: int) -> int:
     of 64) and 0.21 us a block beyond, and a block's start for every sequence.  In chunks a block of 32 columns has an SM to itself: 10.5
     us a chunk however few tokens are in it (5.5 with keys of 64; with 16 columns, where twice the blocks still fit the SMs, 7.9 and
     5.3), 3 us a block, and what forms T and P, 71 ns per chunk and head and 18 us at least.
-    Measured on B200 (heads of 128 x 128; us, token by token / all in chunks / this rule), 16 heads: one prompt of 2,000 805 / 287 / 288, 8 of
-    2,000 1,824 / 1,654 / 1,654, 8 of 70 71 / 117 / 71, 32 of 70 231 / 411 / 231, 63 decoding sequences beside a prompt of 64 69 / 451 / 69, of
-    512 344 / 491 / 122, of 2,000 1,355 / 630 / 329; 32 heads: 16 of 64 210 / 231 / 210, the three with 63 decoding ones 107 / 883 / 106,
-    436 / 965 / 184, 1,565 / 1,236 / 498."""
+    Measured on B200 (heads of 128 x 128; us, token by token / all in chunks / this rule), 16 heads: one prompt of 2,000 743 / 285 / 286, 8 of
+    2,000 1,792 / 1,618 / 1,618, 8 of 70 69 / 115 / 69, 32 of 70 227 / 407 / 227, 63 decoding sequences beside a prompt of 64 68 / 440 / 68, of
+    512 334 / 480 / 123, of 2,000 1,228 / 615 / 330; 32 heads: 16 of 64 207 / 228 / 207, the three with 63 decoding ones 106 / 863 / 106,
+    436 / 946 / 184, 1,446 / 1,209 / 498."""
     if not n_new or max(n_new) < 64:
         return 0
     columns, token_columns = -(-dv // 32), -(-dv // (64 if dk <= 64 else 32))
@@ -1501,11 +1501,14 @@ def delta_rule(u: torch.Tensor, q_off: int, k_off: int, v_off: int, bg: torch.Te
         known = len(n_new) == ctx.n_seqs
         if chunks_from is None:
             chunks_from = _delta_chunks_from_of(ctx, n_new, n_heads, dk, dv) if known else 1
-        many = [n for n in n_new if n >= chunks_from] if known else []
-        walked, tokens = (len(many), sum(many)) if known else (ctx.n_seqs, T)
+        many = [n for n in n_new if n >= max(chunks_from, 1)] if known else []
+        if not known or sum(many) == T:                   # all of them
+            chunks_from, walked, tokens = min(chunks_from, 1), ctx.n_seqs, T
+            n_chunks = T // 64 + ctx.n_seqs
+        else:
+            walked, tokens, n_chunks = len(many), sum(many), sum(-(-n // 64) for n in many)
         if chunks_from > 0 and walked > 0:
             need = lib().ik_delta_chunks_scratch(tokens, walked, ctx.max_new, n_heads, dk, dv)
-            n_chunks = sum(-(-n // 64) for n in many) if known else tokens // 64 + walked
             scratch = torch.empty(need, dtype=torch.float32, device=u.device)
             st = lib().ik_delta_chunks(_ptr(u), u.stride(0), q_off, k_off, v_off, _ptr(bg), _ptr(state), _ptr(ctx.slots), _ptr(ctx.cu_seqlens),
                                        _ptr(ctx.kv_lens), _ptr(out), _ptr(scratch), T, ctx.n_seqs, chunks_from, walked, n_chunks, n_heads,
@@ -1513,7 +1516,7 @@ def delta_rule(u: torch.Tensor, q_off: int, k_off: int, v_off: int, bg: torch.Te
             if st != -2:
                 _check(st, "delta_chunks", kernels=2)
                 below = chunks_from
-                if (tokens == T if known else chunks_from <= 1):
+                if tokens == T:
                     return out
     _check(lib().ik_delta_rule(_ptr(u), u.stride(0), q_off, k_off, v_off, _ptr(bg), _ptr(state), _ptr(ctx.slots), _ptr(ctx.cu_seqlens),
                                _ptr(ctx.kv_lens), _ptr(out), T, ctx.n_seqs, n_heads, n_qk_heads, dk, dv, 1 if ctx.is_decode else 0,
