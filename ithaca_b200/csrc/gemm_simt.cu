@@ -1,7 +1,7 @@
 // Plain matrix product on the CUDA cores: Y[M, N] (+)= X[M, K] * W[N, K]^T.
 //
-// This is the 32-bit path's product and the fallback for shapes the tensor-core kernels
-// refuse.  Operands are converted to float when loaded; every output element is one
+// This is the 32-bit path's product for 32-bit weights, for K < 256 and for rows off 16 bytes (gemm_split.cu takes the others), and the fallback for
+// shapes the 16-bit tensor-core kernels refuse.  Operands are converted to float when loaded; every output element is one
 // float accumulator that adds its K products in ascending k, whatever M and N are, so a
 // row of Y does not depend on which other rows are in the call.  No split along K, no
 // atomics, no reduced-precision matrix mode.  A batch of products of equal shape (one per head, say) runs as one

@@ -84,6 +84,9 @@ _SIGNATURES = {
     "ik_gemm_qkv_rope_wide": [_vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp],
     "ik_gemm_wide_tile_width": [_i, _i, _i, _i],
     "ik_gemm_wide_take_wait_record": [_vp],
+    "ik_gemm_split": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp],
+    "ik_gemm_split_scratch": [_i, _i, _i],
+    "ik_gemm_split_take_wait_record": [_vp],
     "ik_gemm_tcgen05_tile": [_i],
     "ik_gemm_tcgen05_tile_width": [_i, _i],
     "ik_gemm_tcgen05_stream_k_bytes": [],
@@ -265,7 +268,7 @@ def lib():
             fn = getattr(l, name)
             fn.argtypes = sig
             fn.restype = _i
-        l.ik_selective_scan_scratch.restype = l.ik_delta_chunks_scratch.restype = ctypes.c_longlong
+        l.ik_selective_scan_scratch.restype = l.ik_delta_chunks_scratch.restype = l.ik_gemm_split_scratch.restype = ctypes.c_longlong
         _lib = l
     return timed(_lib)
 
@@ -379,6 +382,51 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = No
     _work(f"gemm_simt {M}x{N}x{K}", M * K * x.element_size() + N * K * w.element_size() + M * N * out.element_size(), 2 * M * N * K)
     _check(lib().ik_gemm_simt(_ptr(x), _code(x), _ptr(w), _code(w), _ptr(out), _code(out), M, N, K, x.stride(0),
                               w.stride(0), out.stride(0), 1 if accumulate else 0, _stream()), "gemm_simt")
+    return out
+
+
+SPLIT_ROWS = 4096           # rows of x whose planes are formed at a time
+
+
+def split_takes(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch.float32) -> bool:
+    """Whether a product of the 32-bit path runs on the tensor cores (gemm_split.cu) instead of the CUDA cores (gemm_simt.cu).  The number
+    of rows has no say: a row gets the same bits whatever other rows are in the call.  From K = 256 on the tensor cores are
+    ahead at any number of rows and features (us on B200, CUDA cores / these: K = 256, 32 features 1 row 10.3 / 5.4, 2,000 rows 11.2 / 7.6, 8,192
+    features 11 / 6, 166 / 32; K = 128, 2,000 rows x 32 6.3 / 6.4, 1 row 5.9 / 4.7, which the second launch costs the host; K = 64 3.7 / 4.4)."""
+    K = w.shape[1]
+    return (x.dtype == torch.float32 and w.dtype == torch.bfloat16 and out_dtype == torch.float32 and K >= 256
+            and K % 8 == 0 and w.stride(1) == 1 and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_split(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False,
+               status: Optional[torch.Tensor] = None, tile: int = 0, side_by_side: bool = False) -> torch.Tensor:
+    """out[M, N] (+)= x[M, K] @ w[N, K]^T, x and out float32, w bfloat16: x as three bfloat16 numbers on the tensor cores, sums of
+    128 products there, the rest in float registers.  ``tile``: tokens of a tile (32, 64, 128; 0 = chosen, with whether the slices of K run
+    ``side_by_side``): the same bits every way."""
+    _need(x, "x", torch.float32, contiguous=False)
+    _need(w, "w", torch.bfloat16, contiguous=False)
+    M, K = x.shape
+    N, K2 = w.shape
+    if K != K2 or x.stride(1) != 1 or w.stride(1) != 1:
+        raise KernelError(f"gemm: shapes {tuple(x.shape)} x {tuple(w.shape)}^T do not match or rows are not contiguous")
+    if out is None:
+        if accumulate:
+            raise KernelError("gemm: accumulate needs an output to add to")
+        out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    _need(out, "out", torch.float32, contiguous=False)
+    if out.shape != (M, N) or out.stride(1) != 1:
+        raise KernelError("gemm: the output has the wrong shape")
+    if status is None:
+        status = device_status(x.device)
+    planes = torch.empty((3, min(M, SPLIT_ROWS), K), dtype=torch.bfloat16, device=x.device)
+    for lo in range(0, M, SPLIT_ROWS):
+        m = min(SPLIT_ROWS, M - lo)
+        floats = 8 * m * N if side_by_side else 0 if tile else lib().ik_gemm_split_scratch(m, N, K)
+        partial = torch.empty(floats, dtype=torch.float32, device=x.device) if floats else None
+        _work(f"gemm_split {m}x{N}x{K}", m * K * 4 + N * K * 2 + m * N * 4, 2 * m * N * K)
+        _check(lib().ik_gemm_split(_ptr(x[lo:]), _ptr(w), _ptr(out[lo:]), _ptr(planes), _ptr(partial), m, N, K, x.stride(0), w.stride(0), out.stride(0),
+                                   1 if accumulate else 0, 2 * tile + side_by_side if tile else 0, _ptr(status), _stream()), "gemm_split",
+               kernels=3 if floats else 2)
     return out
 
 
@@ -1008,7 +1056,8 @@ def wait_records() -> str:
     error message, empty if none did."""
     found = []
     rec = (ctypes.c_int * 4)()
-    takers = [("matrix product", lib().ik_gemm_tcgen05_take_wait_record), ("matrix product (wide)", lib().ik_gemm_wide_take_wait_record), ("state-space duality", lib().ik_ssd_take_wait_record),
+    takers = [("matrix product", lib().ik_gemm_tcgen05_take_wait_record), ("matrix product (wide)", lib().ik_gemm_wide_take_wait_record),
+              ("matrix product (32-bit)", lib().ik_gemm_split_take_wait_record), ("state-space duality", lib().ik_ssd_take_wait_record),
               ("latent attention of prompts", lib().ik_latent_prompt_take_wait_record)]
     from . import attention_bf16
     for hd, m in attention_bf16._modules.items():

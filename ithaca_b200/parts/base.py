@@ -42,8 +42,8 @@ _DTYPES = {"bfloat16": torch.bfloat16, "float32": torch.float32}
 @dataclass
 class Runtime:
     """``dtype`` is the compute path: ``bfloat16`` (the serving kernels: 16-bit operands,
-    float accumulation, float residual stream) or ``float32`` (everything in true
-    32-bit arithmetic on the CUDA cores, 32-bit cache)."""
+    float accumulation, float residual stream) or ``float32`` (everything to
+    32-bit precision, 32-bit cache)."""
     dtype: str = "bfloat16"
     device: str = "cuda"
     status: Optional[torch.Tensor] = None      # int32[1]: set by a kernel that met an index out of range

@@ -3,8 +3,9 @@ reference binds it (rows = out features, cols = in features, src/model.cpp:33).
 
 Which kernel runs depends on the runtime's dtype and the shape:
 
-* float32 path: the CUDA-core product (true 32-bit arithmetic, ascending-k sums);
-  the weight stays as stored (bfloat16 is widened exactly when it is loaded).
+* float32 path: the weight stays as stored.  16-bit weights meet the 32-bit inputs on the tensor cores, every input as
+  three 16-bit numbers that add up to it exactly (gemm_split.cu; closer to 64 bits than ascending-k sums); 32-bit weights, short rows and
+  rows off 16 bytes go to the CUDA-core product (ascending-k sums).
 * bfloat16 path: 16-bit operands with float accumulation.  A weight stored in
   32-bit is rounded to bfloat16 once, here, because this path's products are 16-bit.
 """
@@ -44,4 +45,6 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, a
     if x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16:
         from ..csrc import gemm_bf16
         return gemm_bf16.gemm(x, w, out=out, accumulate=accumulate, out_dtype=out_dtype)
+    if ops.split_takes(x, w, out.dtype if out is not None else out_dtype):
+        return ops.gemm_split(x, w, out=out, accumulate=accumulate)
     return ops.gemm_simt(x, w, out=out, accumulate=accumulate, out_dtype=out_dtype)
