@@ -1249,6 +1249,15 @@ def scan_pieces_pay(T: int, B: int, max_new: int, inner: int, N: int, n_sm: int)
     return max_new * token > 17.0 + 0.083 * T * blocks + 1.5 * B * blocks
 
 
+def scan_pieces_beat_stream(T: int, B: int, max_new: int, inner: int, N: int, n_sm: int) -> bool:
+    """Whether pieces also beat whole sequences whose blocks share their work between warps (up to 64 states): only few channels leave so many
+    SMs idle that they do.  us on B200, whole / pieces: 16 states, 256 channels, one prompt of 4,000 152 / 55, 512, one of 8,000 297 / 110, 512, eight of
+    2,000 86 / 179, 2,048, one of 2,000 80 / 98, 4,096, one of 4,000 167 / 325; 64 states, 256, one of 4,000 177 / 91, 1,024 179 / 282."""
+    blocks = -(-inner // (32 if N <= 16 else 16 if N <= 32 else 8)) / n_sm
+    whole = max(0.04 * max_new, 1.07 * B * blocks + 0.031 * T * blocks)
+    return 22.0 + 0.083 * T * blocks + 1.5 * B * blocks < whole
+
+
 def selective_scan(u: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[torch.Tensor], A: torch.Tensor, bc: torch.Tensor,
                    b_off: int, c_off: int, D: Optional[torch.Tensor], z: Optional[torch.Tensor], state: torch.Tensor, ctx,
                    out_dtype: torch.dtype, pieces: Optional[bool] = None) -> torch.Tensor:
@@ -1256,7 +1265,7 @@ def selective_scan(u: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[torc
     (before bias and softplus), ``A`` [inner, N] float (negative), B and C = columns ``b_off``.. and ``c_off``.. of ``bc``,
     ``z`` [T, inner] float (rows may be a column range) for the gate y * silu(z), ``state`` [max_slots, 2, inner, N] float.
     ``pieces``: prompts with bfloat16 inputs in pieces that run side by side, where the sizes allow it (None: where
-    ``scan_pieces_pay`` says so)."""
+    ``scan_pieces_pay`` and ``scan_pieces_beat_stream`` say so)."""
     _need(u, "u")
     _need(dt_raw, "dt_raw", torch.float32)
     _need(A, "A", torch.float32)
@@ -1278,7 +1287,8 @@ def selective_scan(u: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[torc
           9 * T * inner * N)
     max_new = getattr(ctx, "max_new", 0)                  # a caller that does not say gets every sequence token by token
     need = 0
-    if pieces or (pieces is None and not ctx.is_decode and scan_pieces_pay(T, ctx.n_seqs, max_new, inner, N, sm_count())):
+    if pieces or (pieces is None and not ctx.is_decode and scan_pieces_pay(T, ctx.n_seqs, max_new, inner, N, sm_count())
+                  and scan_pieces_beat_stream(T, ctx.n_seqs, max_new, inner, N, sm_count())):
         need = lib().ik_selective_scan_scratch(_code(u), T, ctx.n_seqs, max_new, inner, N, 1 if ctx.is_decode else 0)
     scratch = torch.empty(need, dtype=torch.float32, device=u.device) if need else None
     st = lib().ik_selective_scan(_ptr(u), _code(u), _ptr(dt_raw), _ptr(dt_bias), _ptr(A), _ptr(bc), bc.stride(0), b_off, c_off,

@@ -450,6 +450,218 @@ selective_scan_kernel(const TU* __restrict__ u, const float* __restrict__ dt_raw
     }
 }
 
+// Whole sequences of the 16-bit path with up to 64 states, the work shared between the warps of a block.  Two teams of four warps take turns to bring
+// tiles of TT tokens through registers into one of four places in shared memory (step sizes, their products with the inputs, gates, B, C) and to write the
+// results of the tile before; the four last warps do nothing but the recurrence, a thread four states of a channel, L lanes a channel, CH channels a
+// block, two states per instruction where the hardware has one (mul and fma of f32x2).  So neither waits for the other's latency: a token
+// takes 40 ns with a block to an SM, and with more the reads from shared memory (10 to 14 cycles a warp and token), the exponentials (four a
+// cycle and scheduler) and the issue slots bind about evenly.  Tokens that are not there have a step size of 0: a factor of 1 and nothing added.
+// Measured on B200, 4,096 channels of 16 states (us, the kernel above / this): one prompt of 200 25 / 10, of 3,000 341 / 125, 3,000 + 1,910 399 / 193,
+// eight of 2,000 790 / 437.  One team alone took 231 for 3,000 + 1,910 (a tile's softplus, gates and stores are 225 instructions of one
+// warp in sequence); two states a thread and twice the warps 220; with the sums of four tokens stored before the next four's reads 221.
+template <int L, int CH, int TT>
+struct StreamTile {
+    static constexpr int NPAD = 4 * L, QC = CH / 4, WORKERS = CH * L;
+    // A row of pairs (step size, its product with x; x, gate) is a token's channels: channel 4 q + i in place i QC + q (of 32, q ^ 4 for
+    // i >= 2), rows 2 QC floats further apart than they are long, and the rows of sums likewise: four channels a thread on one side, a few
+    // neighbouring ones a warp on the other, neither meets a bank twice.
+    static constexpr int ROW = 2 * CH + 2 * QC, YLD = CH == 32 ? CH + 8 : CH + 4;
+    static constexpr int BC = TT * ROW, XG = BC + 2 * TT * NPAD, Y = XG + TT * ROW, FLOATS = Y + TT * YLD;         // places of B and C, of x and gate, of the sums
+    static __device__ __forceinline__ int place(int tt, int q, int i) { return tt * ROW + 2 * (i * QC + (CH == 32 ? q ^ (4 * (i >> 1)) : q)); }
+};
+__device__ __forceinline__ uint64_t ik_pack2(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ float2 ik_unpack2(uint64_t v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ uint64_t ik_mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t ik_fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ uint64_t ik_exp2_2(uint64_t v) {
+    float2 x = ik_unpack2(v);
+    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(x.x));
+    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(x.y));
+    return ik_pack2(x.x, x.y);
+}
+
+template <typename TO, int L, int CH, int TT, bool VEC>
+__global__ void __launch_bounds__(256 + CH * L, VEC ? 2 : 1)
+selective_scan_stream_kernel(const __nv_bfloat16* __restrict__ u, const float* __restrict__ dt_raw, const float* __restrict__ dt_bias,
+                             const float* __restrict__ A, const float* __restrict__ bc, int ldbc, int b_off, int c_off,
+                             const float* __restrict__ Dv, const float* __restrict__ z, int ldz, float* __restrict__ state,
+                             const int* __restrict__ slots, const int* __restrict__ cu_seqlens, const int* __restrict__ kv_lens,
+                             TO* __restrict__ out, int inner, int N) {
+    typedef StreamTile<L, CH, TT> Tile;
+    constexpr int NPAD = Tile::NPAD, YLD = Tile::YLD, ALL = 128 + Tile::WORKERS;
+    extern __shared__ __align__(16) float sm[];              // [4][FLOATS]
+    ik_pdl_wait();
+    IK_AFTER_WAIT(u);
+    IK_AFTER_WAIT(dt_raw);
+    IK_AFTER_WAIT(bc);
+    IK_AFTER_WAIT(z);
+    IK_AFTER_WAIT(slots);
+    IK_AFTER_WAIT(cu_seqlens);
+    IK_AFTER_WAIT(kv_lens);
+    ik_pdl_launch_dependents();
+    const int b = blockIdx.y, c0 = blockIdx.x * CH;
+    const int lo = cu_seqlens[b], hi = cu_seqlens[b + 1], end = kv_lens[b], start = end - (hi - lo);
+    if (hi <= lo) return;
+    const int n_tiles = (hi - lo + TT - 1) / TT;
+    // barriers 1 to 4: a place is filled; 5 to 8: its sums are there (one side arrives, the other waits)
+    if (threadIdx.x < 256) {
+        const int tid = threadIdx.x & 127, team = threadIdx.x >> 7;
+        constexpr int QC = Tile::QC, Q = TT * QC;            // four neighbouring channels of a token: places in a tile
+        constexpr int QB = TT * 2 * NPAD / 4, KB = QB / 128; // four neighbouring values of B or C
+        static_assert(Q <= 128 && QB % 128 == 0 && TT % L == 0, "a tile's values and the threads that bring them");
+        const int tt = tid / QC, w = 4 * (tid % QC), col = c0 + w;
+        const bool mine = tid < Q;
+        float bias[4], skip[4];
+        #pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int cc = min(col + i, inner - 1);
+            bias[i] = dt_bias ? dt_bias[cc] : 0.f;
+            skip[i] = Dv ? Dv[cc] : 0.f;
+        }
+        struct Values { uint2 u; float4 d, z, b[KB]; };      // of a tile, on their way
+        // VEC: four values are four neighbours in memory.  No branch stands between these loads and their use two tiles later (a value that
+        // two branches may have set is moved where they meet, and the move waits for the load); what is not there is replaced where it is stored.
+        auto fetch = [&](Values& r, int t0) {
+            const int t = min(t0 + tt, hi - 1);
+            if (VEC) {
+                const int at = min(col, inner - 4);
+                asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(r.u.x), "=r"(r.u.y) : "l"(u + (size_t)t * inner + at));
+                asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.d.x), "=f"(r.d.y), "=f"(r.d.z), "=f"(r.d.w) : "l"(dt_raw + (size_t)t * inner + at));
+                asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.z.x), "=f"(r.z.y), "=f"(r.z.z), "=f"(r.z.w) : "l"(z + (size_t)t * ldz + at));
+            } else {
+                unsigned v[4];
+                #pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int at = min(col + i, inner - 1);
+                    v[i] = ik_ld_now(u + (size_t)t * inner + at);
+                    (&r.d.x)[i] = ik_ld_now(dt_raw + (size_t)t * inner + at);
+                    (&r.z.x)[i] = z ? ik_ld_now(z + (size_t)t * ldz + at) : 0.f;
+                }
+                r.u = make_uint2(v[0] | v[1] << 16, v[2] | v[3] << 16);
+            }
+            #pragma unroll
+            for (int k = 0; k < KB; k++) {
+                const int e = tid + k * 128, n2 = 4 * (e % (NPAD / 2)), n = n2 % NPAD;
+                const float* p = bc + (size_t)min(t0 + e / (NPAD / 2), hi - 1) * ldbc + (n2 < NPAD ? b_off : c_off);
+                if (VEC) asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.b[k].x), "=f"(r.b[k].y), "=f"(r.b[k].z), "=f"(r.b[k].w) : "l"(p + n));
+                else {
+                    #pragma unroll
+                    for (int i = 0; i < 4; i++) (&r.b[k].x)[i] = ik_ld_now(p + min(n + i, N - 1));
+                }
+            }
+        };
+        auto finish = [&](int j) {                           // tile j's results
+            const float* tile = sm + (j & 3) * Tile::FLOATS;
+            asm volatile("bar.sync %0, %1;" :: "r"(5 + (j & 3)), "n"(ALL) : "memory");
+            const int t = lo + j * TT + tt;
+            if (!mine || t >= hi) return;
+            float y[4];
+            const float4 sum = *reinterpret_cast<const float4*>(tile + Tile::Y + tt * YLD + w);
+            #pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 xg = *reinterpret_cast<const float2*>(tile + Tile::XG + Tile::place(tt, tid % QC, i));
+                y[i] = fmaf(skip[i], xg.x, (&sum.x)[i]);
+                if (z) y[i] *= xg.y;
+            }
+            TO* o = out + (size_t)t * inner + col;
+            if (VEC) {
+                if (col < inner) ik_st4(o, 0, make_float4(y[0], y[1], y[2], y[3]));
+            } else {
+                #pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (col + i < inner) ik_st(o, i, y[i]);
+            }
+        };
+        Values r;
+        fetch(r, lo + team * TT);
+        for (int j = team; j < n_tiles; j += 2) {
+            float* tile = sm + (j & 3) * Tile::FLOATS;       // (free: the results of tile j - 4 have been read, by this team)
+            if (mine) {
+                const bool there = lo + j * TT + tt < hi;
+                #pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float x = __uint_as_float(((i & 1) ? (i < 2 ? r.u.x : r.u.y) & 0xffff0000u : (i < 2 ? r.u.x : r.u.y) << 16));
+                    const float dt = there ? ik_softplus_as<true>((&r.d.x)[i] + bias[i]) : 0.f;
+                    *reinterpret_cast<float2*>(tile + Tile::place(tt, tid % QC, i)) = make_float2(dt, dt * x);
+                    *reinterpret_cast<float2*>(tile + Tile::XG + Tile::place(tt, tid % QC, i)) = make_float2(x, ik_silu_as<true>((&r.z.x)[i]));
+                }
+            }
+            #pragma unroll
+            for (int k = 0; k < KB; k++) {
+                const int e = tid + k * 128, n = 4 * (e % (NPAD / 2)) % NPAD;
+                const bool there = lo + j * TT + e / (NPAD / 2) < hi;
+                #pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (!there || (!VEC && n + i >= N)) (&r.b[k].x)[i] = 0.f;
+                *reinterpret_cast<float4*>(tile + Tile::BC + 4 * e) = r.b[k];
+            }
+            asm volatile("bar.arrive %0, %1;" :: "r"(1 + (j & 3)), "n"(ALL) : "memory");
+            fetch(r, lo + (j + 2) * TT);
+            if (j >= 2) finish(j - 2);
+        }
+        if (n_tiles > team) finish(n_tiles - 1 - ((n_tiles - 1 - team) & 1));
+    } else {
+        const int tid = threadIdx.x - 256, l = tid & (L - 1), ch = tid / L, c = c0 + ch, cc = min(c, inner - 1);   // (idle lanes follow along: the shuffles need them)
+        const float* st_in = state + ((size_t)slots[b] * 2 + ((start - 1) & 1)) * inner * N + (size_t)cc * N;
+        float* st_out = state + ((size_t)slots[b] * 2 + ((end - 1) & 1)) * inner * N + (size_t)cc * N;
+        uint64_t S[2], a[2];                                 // states 4 l .. 4 l + 3; a in powers of two
+        #pragma unroll
+        for (int r = 0; r < 2; r++) {
+            float s[2], e[2];
+            #pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int n = 4 * l + 2 * r + i;
+                // (an A of minus infinity: a step size of 0 still leaves the state alone)
+                e[i] = n < N ? fmaxf(A[(size_t)cc * N + n] * 1.44269504f, -3.4e38f) : 0.f;
+                s[i] = n < N && start > 0 ? st_in[n] : 0.f;
+            }
+            S[r] = ik_pack2(s[0], s[1]);
+            a[r] = ik_pack2(e[0], e[1]);
+        }
+        for (int j = 0; j < n_tiles; j++) {
+            float* tile = sm + (j & 3) * Tile::FLOATS;
+            asm volatile("bar.sync %0, %1;" :: "r"(1 + (j & 3)), "n"(ALL) : "memory");
+            // all of the tile's sums before the first is stored: a store in between would hold up the reads behind it
+            float v[TT];
+            #pragma unroll
+            for (int tt = 0; tt < TT; tt++) {
+                const float2 d = *reinterpret_cast<const float2*>(tile + Tile::place(tt, ch >> 2, ch & 3));           // step size, its product with x
+                const float* row = tile + Tile::BC + tt * 2 * NPAD + 4 * l;
+                const ulonglong2 B = *reinterpret_cast<const ulonglong2*>(row), Cv = *reinterpret_cast<const ulonglong2*>(row + NPAD);
+                const uint64_t dd = ik_pack2(d.x, d.x), dx = ik_pack2(d.y, d.y);
+                S[0] = ik_fma2(ik_exp2_2(ik_mul2(dd, a[0])), S[0], ik_mul2(dx, B.x));
+                S[1] = ik_fma2(ik_exp2_2(ik_mul2(dd, a[1])), S[1], ik_mul2(dx, B.y));
+                const float2 sum = ik_unpack2(ik_fma2(S[1], Cv.y, ik_mul2(S[0], Cv.x)));
+                v[tt] = sum.x + sum.y;
+            }
+            // the lanes' sums, L tokens at a time: lane i ends with token i's (as above)
+            #pragma unroll
+            for (int o = L >> 1; o > 0; o >>= 1) {
+                const bool upper = l & o;
+                #pragma unroll
+                for (int t4 = 0; t4 < TT; t4 += L)
+                    #pragma unroll
+                    for (int i = 0; i < o; i++) {
+                        const float theirs = __shfl_xor_sync(0xffffffffu, upper ? v[t4 + i] : v[t4 + i + o], o);
+                        v[t4 + i] = (upper ? v[t4 + i + o] : v[t4 + i]) + theirs;
+                    }
+            }
+            #pragma unroll
+            for (int t4 = 0; t4 < TT; t4 += L) tile[Tile::Y + (t4 + l) * YLD + ch] = v[t4];
+            asm volatile("bar.arrive %0, %1;" :: "r"(5 + (j & 3)), "n"(ALL) : "memory");
+        }
+        if (c < inner) {
+            #pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const float2 s = ik_unpack2(S[r]);
+                const int n = 4 * l + 2 * r;
+                if (n < N) st_out[n] = s.x;
+                if (n + 1 < N) st_out[n + 1] = s.y;
+            }
+        }
+    }
+}
+
 // The states with which a sequence's pieces begin, one thread per channel and state.
 __global__ void __launch_bounds__(256)
 scan_carry_kernel(const float* __restrict__ A, const float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ cu_seqlens,
@@ -542,6 +754,21 @@ static int scan_piece_tokens(int T, int B, int max_new, int inner, int N) {
     return max_new >= 3 * piece && T / piece + B <= 65535 ? piece : 0;
 }
 
+// Whether whole sequences of the 16-bit path run with the work shared between a block's warps.  Its blocks are large: where most sequences bring a few
+// tokens, starting them costs more than the longer sequences gain.  Microseconds, fitted on B200 for 1 to 64 sequences of 1 to 3,000 tokens,
+// 1,024 to 8,192 channels, 16 to 64 states; blocks are those of a sequence per SM (the other kernel / this): 4,096 channels of 16 states, 64 sequences
+// of 2 tokens 33 / 59, of 20 75 / 90, of 100 275 / 217, one of 200 beside 63 of 1 44 / 64, one of 1,000 179 / 83.
+static bool scan_streams(int T, int B, int max_new, int inner, int N) {
+    if (N > 64) return false;
+    const double longest = max_new > 0 ? max_new : T / (double)B;
+    const int ch = N <= 16 ? 32 : N <= 32 ? 16 : 8;
+    const double blocks = (inner + ch - 1) / ch / (double)ik_sm_count();
+    const double chain = 0.113 * longest, all = 0.48 * B * blocks + (N <= 32 ? 0.042 : 0.038) * T * blocks;
+    const double other = fmax(chain, all) + 0.5 * fmin(chain, all);
+    const double here = fmax(0.043 * longest, 1.07 * B * blocks + (N <= 32 ? 0.031 : 0.034) * T * blocks);
+    return B * blocks < 2.0 || here <= other;                    // (two blocks an SM start together)
+}
+
 template <typename TU, typename TO, bool FAST>
 static int launch_scan(const void* u, const float* dt_raw, const float* dt_bias, const float* A, const float* bc, int ldbc, int b_off,
                        int c_off, const float* Dv, const float* z, int ldz, float* state, const int* slots, const int* cu_seqlens,
@@ -554,12 +781,12 @@ static int launch_scan(const void* u, const float* dt_raw, const float* dt_bias,
                                  (size_t)2 * (TT) * (3 * (128 / (L)) + 2 * (L) * (NPT)) * sizeof(float), stream,                \
                                  (const TU*)u, dt_raw, dt_bias, A, bc, ldbc, b_off, c_off, Dv, z, ldz, state, slots, cu_seqlens,  \
                                  kv_lens, (TO*)out, inner, N, pieces))
+#define IK_SCAN_DECODE(NPT, L)                                                                                                  \
+    IK_RETURN_IF_ERROR(ik_launch(selective_scan_decode_kernel<TU, TO, FAST, NPT, L>, dim3((inner + 128 / (L) - 1) / (128 / (L)), B), 128, 0, stream, (const TU*)u, dt_raw,   \
+                                 dt_bias, A, bc, ldbc, b_off, c_off, Dv, z, ldz, state, slots, cu_seqlens, kv_lens, (TO*)out, inner, N))
 #define IK_SCAN(NPT, L, TT)                                                                                                     \
     do {                                                                                                                        \
-        if (one_token_each)                                                                                                     \
-            IK_RETURN_IF_ERROR(ik_launch(selective_scan_decode_kernel<TU, TO, FAST, NPT, L>, dim3((inner + 128 / (L) - 1) / (128 / (L)), B), 128, 0, stream, (const TU*)u, dt_raw,   \
-                                         dt_bias, A, bc, ldbc, b_off, c_off, Dv, z, ldz, state, slots, cu_seqlens, kv_lens, (TO*)out,    \
-                                         inner, N));                                                                            \
+        if (one_token_each) IK_SCAN_DECODE(NPT, L);                                                                             \
         else IK_SCAN_AT(NPT, L, TT, 0, B);                                                                                      \
     } while (0)
 #define IK_SCAN_PIECES(NPT, L, TT)                                                                                              \
@@ -583,18 +810,43 @@ static int launch_scan(const void* u, const float* dt_raw, const float* dt_bias,
             IK_LAUNCH_STATUS();
         }
     }
-    // up to 16 states, 16-bit path: two states a thread while four would leave the SMs with fewer than two warps a scheduler
-    // (one 4,096-token prompt, 4,096 channels: 1.01 -> 0.88 ms).  The float32 path keeps one shape whatever the batch, so
-    // that its sums never depend on what else a step brings.
-    const bool two = FAST && (long long)((inner + 31) / 32) * B * 4 < 8LL * ik_sm_count();
-    if (N <= 16 && two) IK_SCAN(2, 8, 16);
-    else if (N <= 16) IK_SCAN(4, 4, 16);
+    if constexpr (FAST) {
+        if (!one_token_each && scan_streams(T, B, max_new, inner, N)) {
+            const bool vec = inner % 4 == 0 && z && ldz % 4 == 0 && ldbc % 4 == 0 && b_off % 4 == 0 && c_off % 4 == 0 && (N == 16 || N == 32 || N == 64) &&
+                             (((uintptr_t)dt_raw | (uintptr_t)z | (uintptr_t)bc | (2 * (uintptr_t)u)) % 16) == 0 && ((uintptr_t)out % (4 * sizeof(TO))) == 0;
+#define IK_SCAN_STREAM_AT(L, CH, VEC)                                                                                           \
+    IK_RETURN_IF_ERROR(cudaFuncSetAttribute(selective_scan_stream_kernel<TO, L, CH, 16, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
+                                            4 * (int)sizeof(float) * StreamTile<L, CH, 16>::FLOATS));                           \
+    IK_RETURN_IF_ERROR(ik_launch(selective_scan_stream_kernel<TO, L, CH, 16, VEC>, dim3((inner + (CH) - 1) / (CH), B), 256 + (CH) * (L), \
+                                 4 * sizeof(float) * StreamTile<L, CH, 16>::FLOATS, stream, (const __nv_bfloat16*)u, dt_raw, dt_bias, A, bc, ldbc, b_off, \
+                                 c_off, Dv, z, ldz, state, slots, cu_seqlens, kv_lens, (TO*)out, inner, N))
+#define IK_SCAN_STREAM(L, CH)                                                                                                   \
+    do {                                                                                                                        \
+        if (vec) { IK_SCAN_STREAM_AT(L, CH, true); }                                                                            \
+        else { IK_SCAN_STREAM_AT(L, CH, false); }                                                                               \
+    } while (0)
+            if (N <= 16) IK_SCAN_STREAM(4, 32);
+            else if (N <= 32) IK_SCAN_STREAM(8, 16);
+            else IK_SCAN_STREAM(16, 8);
+#undef IK_SCAN_STREAM
+#undef IK_SCAN_STREAM_AT
+            IK_LAUNCH_STATUS();
+        }
+    }
+    // up to 16 states, a decode step of the 16-bit path: two states a thread while four would leave the SMs with fewer than two warps a
+    // scheduler.  The float32 path keeps one shape whatever the batch, so that its sums never depend on what else a step brings.
+    if (FAST && one_token_each && N <= 16 && (long long)((inner + 31) / 32) * B * 4 < 8LL * ik_sm_count()) {
+        IK_SCAN_DECODE(2, 8);
+        IK_LAUNCH_STATUS();
+    }
+    if (N <= 16) IK_SCAN(4, 4, 16);
     else if (N <= 32) IK_SCAN(4, 8, 16);
     else if (N <= 64) IK_SCAN(4, 16, 16);
     else if (N <= 128) IK_SCAN(8, 16, 8);
     else if (N <= 256) IK_SCAN(8, 32, 4);
     else return IK_UNSUPPORTED;
 #undef IK_SCAN
+#undef IK_SCAN_DECODE
     IK_LAUNCH_STATUS();
 }
 
