@@ -266,7 +266,9 @@ IK_EXPORT int ik_delta_rule(const float* u, int ldu, int q_off, int k_off, int v
 // out[t, h*dv + i] = x[t, h, i] * (1 / sqrt(mean_i(x[t, h, :]^2) + eps)) * w[i] * act(p[t, g_off + h*dv + i]), the weight of
 // size dv shared by the heads (w_head = 0) or one of size dv per head (w_head = dv: w[h * dv + i]); act 1: silu, 2: sigmoid,
 // 0: no gate.  One warp per (token, head).
-template <typename TO>
+// NV > 0: dv = 32 NV, and a warp's values and gates, of ROWS heads at a time, are asked for together before the sum of squares (NV = 0: any dv; the
+// same sums in the same order).  What bounds it is the bytes.  Measured on B200, 4,910 tokens, 16 heads of 128, silu (us): 38 -> 26 (100 MB: 15).
+template <typename TO, int NV, int ROWS>
 __global__ void __launch_bounds__(256)
 head_norm_gate_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ p, int ldp, int g_off,
                       TO* __restrict__ out, int rows, int H, int dv, float eps, int act, int w_head) {
@@ -274,33 +276,68 @@ head_norm_gate_kernel(const float* __restrict__ x, const float* __restrict__ w, 
     IK_AFTER_WAIT(x);
     IK_AFTER_WAIT(p);
     ik_pdl_launch_dependents();
-    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    const int t = row / H, h = row - t * H;
+    const int row0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * ROWS, lane = threadIdx.x & 31;
+    if (row0 >= rows) return;
+    auto gated = [&](float v, float g) { return act == 1 ? v * (g / (1.0f + expf(-g))) : act == 2 ? v * (1.0f / (1.0f + expf(-g))) : v; };
+    auto norm = [&](float ss) {
+        #pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        return 1.0f / sqrtf(ss / (float)dv + eps);
+    };
+    if (NV > 0) {
+        float a[ROWS][NV > 0 ? NV : 1], g[ROWS][NV > 0 ? NV : 1];
+        #pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            const int row = min(row0 + r, rows - 1), t = row / H, h = row - t * H;
+            #pragma unroll
+            for (int k = 0; k < NV; k++) {
+                a[r][k] = x[(size_t)row * dv + lane + 32 * k];
+                g[r][k] = act ? p[(size_t)t * ldp + g_off + h * dv + lane + 32 * k] : 0.f;
+            }
+        }
+        #pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            const int row = row0 + r, h = row % H;
+            float ss = 0.f;
+            #pragma unroll
+            for (int k = 0; k < NV; k++) ss = fmaf(a[r][k], a[r][k], ss);
+            const float s = norm(ss);
+            if (row >= rows) break;
+            #pragma unroll
+            for (int k = 0; k < NV; k++)
+                ik_st(out, (size_t)row * dv + lane + 32 * k, gated(a[r][k] * s * w[h * w_head + lane + 32 * k], g[r][k]));
+        }
+        return;
+    }
+    const int row = row0, t = row / H, h = row - t * H;
     const float* a = x + (size_t)row * dv;
     float ss = 0.f;
     for (int i = lane; i < dv; i += 32) ss = fmaf(a[i], a[i], ss);
-    #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float s = 1.0f / sqrtf(ss / (float)dv + eps);
+    const float s = norm(ss);
     const float* g = act ? p + (size_t)t * ldp + g_off + h * dv : nullptr;
-    for (int i = lane; i < dv; i += 32) {
-        float v = a[i] * s * w[h * w_head + i];
-        if (act == 1) v *= g[i] / (1.0f + expf(-g[i]));
-        else if (act == 2) v *= 1.0f / (1.0f + expf(-g[i]));
-        ik_st(out, (size_t)row * dv + i, v);
-    }
+    for (int i = lane; i < dv; i += 32) ik_st(out, (size_t)row * dv + i, gated(a[i] * s * w[h * w_head + i], act ? g[i] : 0.f));
 }
 
 IK_EXPORT int ik_head_norm_gate(const float* x, const float* w, const float* p, int ldp, int g_off, void* out, int out_dtype, int T,
                                 int H, int dv, float eps, int act, int w_head, cudaStream_t stream) {
     if (T < 0 || H <= 0 || dv <= 0 || act < 0 || act > 2 || (act && !p) || (w_head != 0 && w_head != dv)) return IK_BAD_ARGUMENT;
     if (T == 0) return IK_OK;
-    const int rows = T * H, blocks = (rows + 7) / 8;
-    if (out_dtype == IK_F32)
-        IK_RETURN_IF_ERROR(ik_launch(head_norm_gate_kernel<float>, blocks, 256, 0, stream, x, w, p, ldp, g_off, (float*)out, rows, H, dv, eps, act, w_head));
-    else if (out_dtype == IK_BF16)
-        IK_RETURN_IF_ERROR(ik_launch(head_norm_gate_kernel<__nv_bfloat16>, blocks, 256, 0, stream, x, w, p, ldp, g_off, (__nv_bfloat16*)out, rows, H, dv, eps, act, w_head));
+    const int rows = T * H;
+    // two heads a warp where there are enough of them for all SMs
+    const int each = (dv == 64 || dv == 128) && rows >= 64 * ik_sm_count() ? 2 : 1, blocks = (rows + 8 * each - 1) / (8 * each);
+#define IK_HNG_AT(TO, NV, ROWS) IK_RETURN_IF_ERROR(ik_launch(head_norm_gate_kernel<TO, NV, ROWS>, blocks, 256, 0, stream, x, w, p, ldp, g_off, (TO*)out, rows, H, dv, eps, act, w_head))
+#define IK_HNG(TO)                                                                        \
+    do {                                                                                  \
+        if (dv == 128 && each == 2) IK_HNG_AT(TO, 4, 2);                                  \
+        else if (dv == 128) IK_HNG_AT(TO, 4, 1);                                          \
+        else if (dv == 64 && each == 2) IK_HNG_AT(TO, 2, 2);                              \
+        else if (dv == 64) IK_HNG_AT(TO, 2, 1);                                           \
+        else IK_HNG_AT(TO, 0, 1);                                                         \
+    } while (0)
+    if (out_dtype == IK_F32) IK_HNG(float);
+    else if (out_dtype == IK_BF16) IK_HNG(__nv_bfloat16);
     else return IK_BAD_ARGUMENT;
+#undef IK_HNG
+#undef IK_HNG_AT
     IK_LAUNCH_STATUS();
 }
