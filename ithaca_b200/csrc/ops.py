@@ -93,6 +93,7 @@ _SIGNATURES = {
     "ik_rope_table": [_vp, _vp, _vp, _i, _i, _vp],
     "ik_gemm_qkv_rope_mma": [_vp, _vp, _i, _i, _i, _i, _i, _vp, _vp],
     "ik_gemm_qkv_rope_tcgen05": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp],
+    "ik_attention_rows": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _i, _vp, _vp],
     "ik_attention_simt": [_vp, _i, _vp, _vp, _i, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _f, _i, _i, _i, _vp, _vp, _vp, _i, _i, _vp, _vp],
     "ik_gemm_simt_batched": [_vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _u64, _u64, _u64, _vp],
     "ik_scale_add_norm": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _f, _vp],
@@ -764,6 +765,43 @@ def attention_simt(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor
                                    n_heads, nkv, hd, hdv, ldv, scale, softcap, window, keep, sink_flag(sink), _ptr(sink_values(sink, n_heads)),
                                    _ptr(key_scales), _ptr(slopes), page_size, n_pages, _ptr(status), _stream()),
            "attention_simt")
+    return out
+
+
+def attention_rows_pay(n_new, kv_lens, n_heads: int, n_kv_heads: int, window: int) -> bool:
+    """Whether a prompt step's 32-bit attention goes by blocks of 64 rows (``attention_rows``) rather than a token a block (``attention_simt``): the
+    sequences fill a block's tokens on average, and tokens and their tiles of 128 keys are enough to be worth a block's start.  us on B200, a token a
+    block / these (32 heads of 64 on 8 kv heads): one prompt of 20 7.1 / 11.5, 64 13.9 / 15.3, 8 of 16 10.2 / 11.5, 8 of 4 behind 50 12.8 / 44, 6 of
+    100 behind 30 95 / 48, 40 behind 2,000 302 / 215; 16 heads on 16: 8 of 16 8.2 / 35, 6 of 100 91 / 54."""
+    group, heads = n_heads // n_kv_heads, 1
+    while heads < 8 and group % (2 * heads) == 0:
+        heads *= 2
+    if not n_new or len(n_new) != len(kv_lens) or sum(n_new) * heads < 64 * len(n_new):
+        return False
+    return sum(n * -(-min(e, window + 128 if window else e) // 128) for n, e in zip(n_new, kv_lens)) > 128
+
+
+def attention_rows(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, token_seq: torch.Tensor, token_pos: torch.Tensor,
+                   table: torch.Tensor, n_heads: int, scale: float, window: int, status: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """What ``attention_simt`` gives for float32 queries and pages without options but a window, bit for bit, with 64 rows (neighbouring tokens x
+    heads of a kv head) to a block: for prompts.  None where the kernel does not take the sizes (head sizes other than 64 and 128)."""
+    _need(q, "q", torch.float32)
+    _need(k_pages, "k_pages", torch.float32)
+    _need(v_pages, "v_pages", torch.float32)
+    _need(table, "table", torch.int32)
+    n_pages, nkv, page_size, hd = k_pages.shape
+    T = q.shape[0]
+    if q.shape[1] != n_heads * hd or v_pages.shape[:3] != k_pages.shape[:3]:
+        raise KernelError("attention: q or the value pages have the wrong shape")
+    if v_pages.shape[3] != hd:
+        return None
+    out = torch.empty((T, n_heads * hd), dtype=q.dtype, device=q.device)
+    _work(f"attention_rows {T}x{n_heads}", _nbytes(q, out))
+    st = lib().ik_attention_rows(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(token_seq), _ptr(token_pos), _ptr(table), table.stride(0), T,
+                                 n_heads, nkv, hd, scale, window, page_size, n_pages, _ptr(status), _stream())
+    if st == -2:
+        return None
+    _check(st, "attention_rows")
     return out
 
 

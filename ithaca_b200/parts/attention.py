@@ -302,12 +302,18 @@ class Attention:
 def attend(q: torch.Tensor, cache: LayerCache, ctx, table: torch.Tensor, n_heads: int, scale: float, window: int,
            rt: Runtime, softcap: float = 0.0, sink=False, keep: int = 0, slopes: Optional[torch.Tensor] = None, reach=None) -> torch.Tensor:
     """Chooses the attention kernel: tensor-core kernels for bfloat16 when they take the
-    head sizes, else the CUDA-core kernel (always for float32).  A cache entry without value pages (but with key scales) holds
+    head sizes, else a CUDA-core kernel (always for float32: by blocks of rows for prompts, the same bits).  A cache entry without value pages (but with key scales) holds
     rows that are keys and values."""
     if q.dtype == torch.bfloat16 and (cache.v_pages is None or cache.v_pages.shape[3] == cache.k_pages.shape[3]):
         from ..csrc import attention_bf16
         out = attention_bf16.attend(q, cache.k_pages, cache.v_pages, ctx, table, n_heads, scale, window, rt.status,
                                     softcap=softcap, sink=sink, keep=keep, key_scales=cache.key_scales, slopes=slopes, reach=reach)
+        if out is not None:
+            return out
+    plain = not torch.is_tensor(sink) and not (sink or softcap or keep) and cache.key_scales is None and slopes is None
+    if (plain and q.dtype == torch.float32 and cache.v_pages is not None and cache.k_pages.dtype == torch.float32 and not ctx.is_decode
+            and ops.attention_rows_pay(ctx.host_n_new, ctx.host_kv_lens, n_heads, cache.k_pages.shape[1], window)):
+        out = ops.attention_rows(q, cache.k_pages, cache.v_pages, ctx.token_seq, ctx.token_pos, table, n_heads, scale, window, rt.status)
         if out is not None:
             return out
     return ops.attention_simt(q, cache.k_pages, cache.v_pages, ctx.token_seq, ctx.token_pos, table, n_heads, scale,
