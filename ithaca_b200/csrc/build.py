@@ -30,7 +30,7 @@ _COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcom
                  "--expt-relaxed-constexpr"]
 
 # The always-needed kernels.  Specialised modules are listed in SPECIALISED.
-CORE_SOURCES = ["elementwise.cu", "layernorm.cu", "dynamic_tanh.cu", "short_conv.cu", "recurrent.cu", "delta.cu", "delta_chunk.cu", "row_decay.cu", "gla_chunk.cu", "gla_decode.cu", "ssd.cu", "ssd_tcgen05.cu", "hyper.cu", "latent.cu", "latent_prompt.cu", "attention_extras.cu", "moe.cu", "gemm_simt.cu", "gemm_mma.cu", "gemm_tcgen05.cu", "gemm_wide.cu", "gemm_split.cu",
+CORE_SOURCES = ["elementwise.cu", "layernorm.cu", "dynamic_tanh.cu", "short_conv.cu", "recurrent.cu", "delta.cu", "delta_chunk.cu", "row_decay.cu", "gla_chunk.cu", "gla_decode.cu", "ssd.cu", "ssd_tcgen05.cu", "hyper.cu", "latent.cu", "latent_prompt.cu", "attention_extras.cu", "moe.cu", "gemm_simt.cu", "gemm_mma.cu", "gemm_tcgen05.cu", "gemm_wide.cu", "gemm_split.cu", "gemm_batch.cu",
                 "attention_simt.cu", "attention_rows.cu", "sampling.cu"]
 
 _lock = threading.Lock()

@@ -84,6 +84,9 @@ _SIGNATURES = {
     "ik_gemm_qkv_rope_wide": [_vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp],
     "ik_gemm_wide_tile_width": [_i, _i, _i, _i],
     "ik_gemm_wide_take_wait_record": [_vp],
+    "ik_gemm_batch": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _f, _f, _i, _vp, _vp],
+    "ik_gemm_qkv_rope_batch": [_vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp],
+    "ik_gemm_batch_take_wait_record": [_vp],
     "ik_gemm_split": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp],
     "ik_gemm_split_scratch": [_i, _i, _i],
     "ik_gemm_split_take_wait_record": [_vp],
@@ -570,14 +573,29 @@ def pairs_lib():
     return timed(_pairs_lib) if _pairs_lib else None
 
 
+def batch_takes(M: int, N: int, K: int) -> bool:
+    """Whether a product of up to 128 tokens runs on gemm_batch.cu (no scratch, one kernel) rather than in one of the ways of gemm_tcgen05.cu (``tcgen05_splits``).
+    Two kinds of matrix stay behind (us on B200, those ways / this): few features with a long K, which nine slices and a second kernel keep
+    more SMs busy on (2048 x 8192 for 17 tokens 11.4 / 13.6, 48 12.8 / 13.7, 64 13.9 / 13.7, 65 14.5 / 15.9, 100 17.1 / 15.9), and a few tokens by very many features, where equal
+    shares of K steps spare the last of several rounds (128256 x 2048 for 24 tokens 82.7 / 84.4, 64 86.7 / 87.6, 100 94 / 90)."""
+    if M > 128:
+        return False
+    n_sm = sm_count()
+    if K >= 4096 and K >= 3 * N and 8 * -(-N // 128) <= n_sm and (M <= 48 or 64 < M <= 80):
+        return False
+    return not (M <= 64 and -(-N // 256) >= 4 * (n_sm // 2))
+
+
 def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, out_dtype=torch.float32,
                  accumulate: bool = False, splits: Optional[int] = None,
                  status: Optional[torch.Tensor] = None, swiglu: bool = False, pairs: Optional[bool] = None,
-                 glu=None, act: Optional[str] = None, wide: Optional[bool] = None, wide_tile: int = 0) -> Optional[torch.Tensor]:
+                 glu=None, act: Optional[str] = None, wide: Optional[bool] = None, wide_tile: int = 0,
+                 batch: Optional[int] = None) -> Optional[torch.Tensor]:
     """bfloat16 operands on the tcgen05 tensor cores (TMA-fed, accumulators in TMEM).  Returns None
     when the kernel does not take these sizes (K not a multiple of 8, unaligned rows).
 
-    Which kernel: ``wide`` = the one of gemm_wide.cu (two SMs to a tile of 256 tokens; where it does not take the call, the others
+    Which kernel: ``batch`` = the one of gemm_batch.cu, 16 * blocks to a tile + slices of K (0 = chosen), None = where ``batch_takes`` says so and nothing else
+    is asked for; ``wide`` = the one of gemm_wide.cu (two SMs to a tile of 256 tokens; where it does not take the call, the others
     do), None = where ``wide_takes`` says so and neither ``splits`` nor ``pairs`` asks for another; ``pairs`` = the pair mode of
     gemm_tcgen05.cu, None = for more than 256 tokens.  ``wide_tile``: features of a tile (128, 192, 256; 0 = chosen).
 
@@ -603,6 +621,13 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] =
     join = (2 if glu is not None else 1) if swiglu else _act_code(act, swiglu)
     tag = (' +swiglu' if swiglu else '') + (' +' + act if act else '')
     ga, gl, gs = glu if glu is not None else (1.0, 0.0, 0.0)
+    if batch is not None or (wide is None and splits is None and pairs is None and batch_takes(M, N, K)):
+        _work(f"gemm_batch{tag} {M}x{N}x{K}", 2 * (M * K + N * K) + M * n_out * out.element_size(), 2 * M * N * K)
+        st = lib().ik_gemm_batch(_ptr(x), _ptr(w), _ptr(out), _code(out), M, N, K, x.stride(0), w.stride(0), out.stride(0), 1 if accumulate else 0, join,
+                                 ga, gl, gs, batch or 0, _ptr(status), _stream())
+        if st != -2:
+            _check(st, "gemm_batch")
+            return out
     if wide or (wide is None and splits is None and pairs is None and wide_takes(M, N, K)):
         _work(f"gemm_wide{tag} {M}x{N}x{K}", 2 * (M * K + N * K) + M * n_out * out.element_size(), 2 * M * N * K)
         st = lib().ik_gemm_wide(_ptr(x), _ptr(w), _ptr(out), _code(out), M, N, K, x.stride(0), w.stride(0), out.stride(0),
@@ -656,7 +681,7 @@ def rope_table(token_pos: torch.Tensor, inv_freq: torch.Tensor) -> torch.Tensor:
 def gemm_qkv_rope(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
                   cos_sin: torch.Tensor, token_seq: torch.Tensor, token_pos: torch.Tensor, table: torch.Tensor,
                   n_heads: int, n_kv_heads: int, head_dim: int, write_cache: bool, status: Optional[torch.Tensor],
-                  skinny_max: int = 16, splits: Optional[int] = None, bias: Optional[torch.Tensor] = None) -> bool:
+                  skinny_max: int = 16, splits: Optional[int] = None, bias: Optional[torch.Tensor] = None, batch: Optional[int] = None) -> bool:
     """q, k, v = x W^T (+ ``bias``, a float vector over W's rows) with rotary pairs in adjacent rows of W; rotated q to ``q_out``, rotated k and v into
     the pages.  Returns False when the kernels do not take these sizes (the caller then runs the steps apart)."""
     _need(x, "x", torch.bfloat16, contiguous=False)
@@ -684,6 +709,11 @@ def gemm_qkv_rope(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, k_pages
         st = lib().ik_gemm_qkv_rope_mma(_ptr(x), _ptr(w), M, N, K, x.stride(0), w.stride(0), ctypes.byref(rs), _stream())
         kernels = 1
     else:
+        if batch is not None or (splits is None and batch_takes(M, N, K)):
+            st = lib().ik_gemm_qkv_rope_batch(_ptr(x), _ptr(w), M, N, K, x.stride(0), w.stride(0), batch or 0, _ptr(status), ctypes.byref(rs), _stream())
+            if st != -2:
+                _check(st, "gemm_qkv_rope (batch)")
+                return True
         if splits is None and wide_takes(M, N, K):
             st = lib().ik_gemm_qkv_rope_wide(_ptr(x), _ptr(w), M, N, K, x.stride(0), w.stride(0), 0, _ptr(status), ctypes.byref(rs), _stream())
             if st != -2:
@@ -1095,7 +1125,7 @@ def wait_records() -> str:
     found = []
     rec = (ctypes.c_int * 4)()
     takers = [("matrix product", lib().ik_gemm_tcgen05_take_wait_record), ("matrix product (wide)", lib().ik_gemm_wide_take_wait_record),
-              ("matrix product (32-bit)", lib().ik_gemm_split_take_wait_record), ("state-space duality", lib().ik_ssd_take_wait_record),
+              ("matrix product (batch)", lib().ik_gemm_batch_take_wait_record), ("matrix product (32-bit)", lib().ik_gemm_split_take_wait_record), ("state-space duality", lib().ik_ssd_take_wait_record),
               ("latent attention of prompts", lib().ik_latent_prompt_take_wait_record)]
     from . import attention_bf16
     for hd, m in attention_bf16._modules.items():
