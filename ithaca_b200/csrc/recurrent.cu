@@ -95,9 +95,11 @@ causal_conv4_kernel(const float* __restrict__ x, int ldx, const float* __restric
 
 // The same for prompts: a thread takes RUN neighbouring tokens of its four channels and keeps the inputs behind the current
 // one in registers, so an input is read once (and TAPS - 1 more at the run's start and where a sequence begins) instead of TAPS
-// times.  The sum of a token runs in the same order as above.
+// times.  The sum of a token runs in the same order as above.  What bounds it is the bytes, as long as enough blocks have their loads under way: runs of
+// eight in 118 registers (two blocks an SM) took 41 us for 4,910 tokens of 3,072 channels in float and 36 of 4,096 in 16 bits, of four in 80 37 and 36,
+// of four in 64 (four blocks) 31 and 30, of two 40 and 41 (18 for the bytes).
 template <typename TO, int TAPS, int RUN>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 causal_conv4_run_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, const float* __restrict__ bias,
                         const float* __restrict__ ring, const int* __restrict__ slots, const int* __restrict__ cu_seqlens,
                         const int* __restrict__ token_seq, const int* __restrict__ token_pos, TO* __restrict__ out, int T, int C, int act) {
@@ -181,8 +183,8 @@ IK_EXPORT int ik_causal_conv(const float* x, int ldx, const float* w, const floa
     if (by4 && (out_dtype == IK_F32 || out_dtype == IK_BF16)) {
         const int threads = C / 4 >= 256 ? 256 : ((C / 4 + 31) / 32) * 32;
         const dim3 grid(T, (C / 4 + threads - 1) / threads);
-        constexpr int RUN = 8;
-        const bool runs = !inl && taps >= 2 && taps <= 4 && (long long)T * grid.y >= 8LL * RUN * ik_sm_count();   // enough blocks either way
+        constexpr int RUN = 4;
+        const bool runs = !inl && taps >= 2 && taps <= 4 && (long long)T * grid.y >= 64LL * ik_sm_count();   // enough blocks either way
 #define IK_CONV_RUN(TO, TAPS)                                                                                                       \
     IK_RETURN_IF_ERROR(ik_launch(causal_conv4_run_kernel<TO, TAPS, RUN>, dim3((T + RUN - 1) / RUN, grid.y), threads, 0, stream, x, ldx, w, bias, \
                                  (const float*)ring, slots, cu_seqlens, token_seq, token_pos, (TO*)out, T, C, act))
