@@ -6,11 +6,12 @@
 //   S <- G_end S + K^T ((G_end / G) U).
 // delta_chunk_prepare_kernel forms T and P of every chunk and head side by side; delta_chunk_kernel walks a sequence's chunks with
 // a slice of a head's columns per block: five small products a chunk in place of 64 dependent steps.  The tokens' chain is what
-// bounds the token-by-token kernel (0.37 to 0.4 us a token; which sequences of a step go which way: ops.delta_chunks_from); the chunks' chain is bound by the walk's
-// reads from shared memory (half a 16-byte read per four multiply-adds and thread, and an SM returns 128 bytes of reads a cycle)
-// beside its multiply-adds, about 8,200 cycles a chunk and block at full rate.
-// Measured on B200: a layer 2,048 wide with 16 heads of 128 over two prompts of 3,000 and fewer tokens 2,776 -> 790 us (the rule itself
-// 2,240 -> 600: 89 us of T and P, 509 us of the walk, 10.8 us a chunk; with 512 threads, each half the results, the walk took 606).
+// bounds the token-by-token kernel (0.37 to 0.4 us a token; which sequences of a step go which way: ops.delta_chunks_from); the chunks' chain is
+// bound by the walk's products and the latencies between them.
+// Measured on B200: a layer 2,048 wide with 16 heads of 128 over two prompts of 3,000 and 1,910 tokens 2,776 us token by token; T and P 78 us, and the walk
+// 505 us (10.7 us a chunk) with float products on the CUDA cores, which read half of 16 bytes from shared memory per four multiply-adds, against 329 us
+// (7 us a chunk) on the tensor cores.
+#include <math_constants.h>
 #include "common.cuh"
 
 namespace {
@@ -199,32 +200,140 @@ delta_chunk_prepare_kernel(const float* __restrict__ u, int ldu, int q_off, int 
     }
 }
 
-// One block per (columns of a head, value head, walked sequence); DS columns.  A thread owns 4 columns of one or two rows of the chunk's
-// products (ty and 63 - ty: the triangular products then take every warp equally long), and 4 columns of DK / RG neighbouring
-// rows of the state (in registers; shared memory holds a copy to read from).
-template <int DK, int DS>
+// The five products of a chunk run on the tensor cores (mma.sync, bfloat16) with every float as the sum of three bfloat16 numbers, h + m + l, which
+// hold its 24 bits: h h' + (h m' + m h' + m m' + h l' + l h'), the small terms in sums of their own; what is left out is under 2^-23 of a
+// product.  Sums of the large terms leave the tensor core every 16 products and are added as floats (it drops bits towards zero).  Numbers of 3.3e38 and
+// more count as infinite, bits below 2^-133 go.
+//
+// Everything is transposed, columns of the state first: a warp's sums [columns][tokens or keys' components] are then, lane by lane, what it has to
+// leave as the first operand of the next product, and K, Q, T and P are second operands as they lie (K once more, transposed by the load, for the state).
+// Eight warps share the tokens of each product (8 each; warps w and w + 4 meet the long and the short rows of the triangles on one scheduler) and the
+// state (DK / 8 components each, floats in registers); its planes and those of V - G (K S) and of U pass through shared memory.  Four more
+// warps bring the next chunk's K, Q, T and P as planes: they hold them in registers until the place is free.
+//
+// One block per (16 MT columns of a head, value head, walked sequence).  Bound by the tensor pipe (mma.sync takes 940 multiply-adds a cycle and SM: 6,700
+// cycles a chunk with MT = 2) and by what its latencies leave between three barriers a chunk: 13,000 cycles a chunk with MT = 2, 9,700 with MT = 1 (eight warps to bring in place of four, or a matrix asked for
+// ahead, change nothing).  Distance to 64 bits over prompts of 1,000 to 3,000 tokens: results 1.84e-7 (float products 1.95e-7), states 1.00e-7
+// (1.01e-7); with decays near one 2.0e-7 (4.6e-7) and 1.7e-7 (4.3e-7); with decays around 0.1, where a state is a few tokens' products, 2.2e-7 (2.2e-7)
+// and 8.5e-8 (3.7e-8).
+template <int DK, int MT>
 struct Walk {
-    static constexpr int CG = DS / 4, RG = 256 / CG, LD = DK + 4;
-    static constexpr int RK = C / RG, RS = DK / RG;      // rows of K (and of Q), and of the state, a thread owns
-    static constexpr int FLOATS = 4 * C * LD + C * TLD + 2 * C * TLD + 3 * C * DS + DK * DS + 2 * VEC;
+    static constexpr int LDK = DK + 8, LDT = C + 8;      // row strides of the planes (rows on 16 bytes, 8 of them over all banks)
+    static constexpr int NT = DK / 64, KS = DK / 16;     // 8-wide pieces of the state a warp owns; steps of 16 components
+    static constexpr int K = 0, Q = K + 3 * C * LDK * 2, T = Q + 3 * C * LDK * 2, P = T + 3 * C * LDT * 2;
+    static constexpr int S = P + 3 * C * LDT * 2;        // first operands: [step][plane][MT][lane] 16 bytes
+    static constexpr int R = S + KS * 3 * MT * 512, U = R + 4 * 3 * MT * 512, E = U + 4 * 3 * MT * 512;
+    static constexpr int FIRST = E + 4 * 3 * MT * 512;   // [16 MT] the first token of a chunk that is not finite in a column
+    static constexpr int BYTES = FIRST + 16 * MT * 4;
+};
+constexpr int MULTIPLIERS = 256, BRINGERS = 128, ALL = MULTIPLIERS + BRINGERS;
+// barriers 1 to 4: K, Q, T, P are there; 5 to 8: they have been read; 9: the multipliers among themselves
+__device__ __forceinline__ void bar_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(ALL) : "memory"); }
+__device__ __forceinline__ void bar_wait(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(ALL) : "memory"); }
+__device__ __forceinline__ void bar_multipliers() { asm volatile("bar.sync 9, %0;" ::"n"(MULTIPLIERS) : "memory"); }
+__device__ __forceinline__ bool bar_any(bool mine) {     // a barrier of the multipliers that also says whether any of them said so
+    int any;
+    asm volatile("{ .reg .pred p, q; setp.ne.s32 p, %1, 0; barrier.red.or.pred q, 9, %2, p; selp.s32 %0, 1, 0, q; }"
+                 : "=r"(any) : "r"((int)mine), "n"(MULTIPLIERS) : "memory");
+    return any;
+}
+__device__ __forceinline__ unsigned two_bf16(float x, float y) {          // x in the lower half
+    unsigned r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+    return r;
+}
+__device__ __forceinline__ void planes(float x, float y, unsigned& h, unsigned& m, unsigned& l) {
+    h = two_bf16(x, y);
+    x -= __uint_as_float(h << 16);
+    y -= __uint_as_float(h & 0xffff0000u);
+    m = two_bf16(x, y);
+    l = two_bf16(x - __uint_as_float(m << 16), y - __uint_as_float(m & 0xffff0000u));
+}
+__device__ __forceinline__ void mma(float (&d)[4], const uint4& a, unsigned b0, unsigned b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+}
+// One step of 16: the terms but the largest into lo; that is added to hi.
+template <int MT>
+__device__ __forceinline__ void mma_planes(float (&hi)[MT][4], float (&lo)[MT][4], const uint4 (&a)[MT][3], const unsigned (&b)[3][2]) {
+    constexpr int AP[5] = {2, 0, 1, 1, 0}, BP[5] = {0, 2, 1, 0, 1};
+    #pragma unroll
+    for (int i = 0; i < 5; i++)
+        #pragma unroll
+        for (int mt = 0; mt < MT; mt++) mma(lo[mt], a[mt][AP[i]], b[BP[i]][0], b[BP[i]][1]);
+    float h[MT][4] = {};
+    #pragma unroll
+    for (int mt = 0; mt < MT; mt++) mma(h[mt], a[mt][0], b[0][0], b[0][1]);
+    #pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+        #pragma unroll
+        for (int c = 0; c < 4; c++) hi[mt][c] += h[mt][c];
+}
+template <int MT>
+__device__ __forceinline__ void first_operand(uint4 (&a)[MT][3], const char* from, int step, int lane) {
+    #pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+        #pragma unroll
+        for (int p = 0; p < 3; p++) a[mt][p] = *reinterpret_cast<const uint4*>(from + (((step * 3 + p) * MT + mt) * 32 + lane) * 16);
+}
+// A warp's sums c of an 8-wide piece, as half of a step's first operand.
+template <int MT>
+__device__ __forceinline__ void leave(char* to, int piece, int mt, int lane, const float (&c)[4]) {
+    uint2 h, m, l;
+    planes(c[0], c[1], h.x, m.x, l.x);
+    planes(c[2], c[3], h.y, m.y, l.y);
+    char* at = to + ((piece >> 1) * 3 * MT + mt) * 512 + lane * 16 + (piece & 1) * 8;
+    *reinterpret_cast<uint2*>(at) = h;
+    *reinterpret_cast<uint2*>(at + MT * 512) = m;
+    *reinterpret_cast<uint2*>(at + 2 * MT * 512) = l;
+}
+// Two 8 x 8 pieces of a second operand whose rows are the results' (n), or (TRANS) the sum's (k).
+template <bool TRANS>
+__device__ __forceinline__ void second_operand(unsigned (&b)[2], unsigned at) {
+    if (TRANS) asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(b[0]), "=r"(b[1]) : "r"(at) : "memory");
+    else asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(b[0]), "=r"(b[1]) : "r"(at) : "memory");
+}
+
+// A matrix of 64 rows of `width` floats, n of them there (zeros else), as planes with rows of `ld`: read into registers, then left.
+template <int WIDTH, int LD>
+struct Bring {
+    static constexpr int N = C * WIDTH / 8 / BRINGERS;
+    uint4 h[N], m[N], l[N];
+    __device__ __forceinline__ void read(const float* from, size_t stride, int n, int tid) {
+        #pragma unroll
+        for (int i = 0; i < N; i++) {
+            const int r = (tid + i * BRINGERS) / (WIDTH / 8), w = (tid + i * BRINGERS) % (WIDTH / 8);
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+            if (r < n) {
+                x = at4(from + (size_t)r * stride + 8 * w);
+                y = at4(from + (size_t)r * stride + 8 * w + 4);
+            }
+            planes(x.x, x.y, h[i].x, m[i].x, l[i].x);
+            planes(x.z, x.w, h[i].y, m[i].y, l[i].y);
+            planes(y.x, y.y, h[i].z, m[i].z, l[i].z);
+            planes(y.z, y.w, h[i].w, m[i].w, l[i].w);
+        }
+    }
+    __device__ __forceinline__ void leave(char* to, int tid) const {
+        #pragma unroll
+        for (int i = 0; i < N; i++) {
+            const int r = (tid + i * BRINGERS) / (WIDTH / 8), w = (tid + i * BRINGERS) % (WIDTH / 8);
+            char* at = to + (r * LD + 8 * w) * 2;
+            *reinterpret_cast<uint4*>(at) = h[i];
+            *reinterpret_cast<uint4*>(at + C * LD * 2) = m[i];
+            *reinterpret_cast<uint4*>(at + 2 * C * LD * 2) = l[i];
+        }
+    }
 };
 
-template <int DK, int DS, bool SOME>
-__global__ void __launch_bounds__(256, 1)
+template <int DK, int MT, bool SOME>
+__global__ void __launch_bounds__(ALL, 1)
 delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, int v_off, const float* __restrict__ scratch, const float* __restrict__ vecs,
                    float* __restrict__ state, const int* __restrict__ slots, const int* __restrict__ cu_seqlens,
                    const int* __restrict__ kv_lens, float* __restrict__ out, int n_seqs, int least, int H, int G, int dv) {
-    typedef Walk<DK, DS> W;
-    constexpr int LD = W::LD, RG = W::RG, RK = W::RK, RS = W::RS;
-    extern __shared__ __align__(16) float sm[];
-    float* const KQ = sm;                                // [2][K, Q][64][LD]
-    float* const Ts = KQ + 4 * C * LD;                   // [64][TLD]
-    float* const Ps = Ts + C * TLD;                      // [2][64][TLD]
-    float* const Vs = Ps + 2 * C * TLD;                  // [64][DS]
-    float* const Us = Vs + C * DS;                       // [64][DS]: V - G (K S), then U
-    float* const Es = Us + C * DS;                       // [64][DS]: (G_end / G) U
-    float* const Ss = Es + C * DS;                       // [DK][DS]
-    float* const vec = Ss + DK * DS;                     // [2][VEC]
+    typedef Walk<DK, MT> W;
+    constexpr int NT = W::NT, KS = W::KS;
+    extern __shared__ __align__(16) char sb[];
     ik_pdl_wait();
     IK_AFTER_WAIT(u);
     IK_AFTER_WAIT(scratch);
@@ -238,174 +347,259 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
         seq = walked_sequence<false>(cu_seqlens, n_seqs, least, blockIdx.z);
         if (seq.b < 0) return;
     }
-    const int tid = threadIdx.x, b = seq.b, h = blockIdx.y, col0 = blockIdx.x * DS;
+    const int b = seq.b, h = blockIdx.y, col0 = blockIdx.x * 16 * MT;
     const int lo = cu_seqlens[b], hi = cu_seqlens[b + 1], end = kv_lens[b], start = end - (hi - lo);
     if (!SOME && hi <= lo) return;
-    const int tx = tid % W::CG, ty = tid / W::CG, kvh = h / (H / G);
-    const int col = col0 + 4 * tx, k0 = RS * ty;
-    auto row = [&](int i) { return i == 0 ? ty : C - 1 - ty; };
-    static_assert(RK * RG == C && RK <= 2, "a thread's rows");
-    const bool live = col < dv;                          // dv is a multiple of 4
-    const size_t per = (size_t)H * DK * dv;
-    const float* st_in = state + ((size_t)slots[b] * 2 + ((start - 1) & 1)) * per + ((size_t)h * dv + (live ? col : 0)) * DK + k0;
-    float* st_out = state + ((size_t)slots[b] * 2 + ((end - 1) & 1)) * per + ((size_t)h * dv + (live ? col : 0)) * DK + k0;
+    const int kvh = h / (H / G);
     const int f0 = SOME ? seq.chunk0 : chunk_base(cu_seqlens, b), n_chunks = (hi - lo + C - 1) / C;
+    const float* const tp = scratch + ((size_t)f0 * H + h) * 2 * C * C;
+    const size_t tp_step = (size_t)H * 2 * C * C;
 
-    auto bring_kq = [&](int j) {
-        float* dst = KQ + (j & 1) * 2 * C * LD;
-        const int t0 = lo + j * C, n = min(C, hi - t0);
-        for (int i = tid; i < 2 * C * (DK / 4); i += 256) {
-            const int r = i / (DK / 4), w = i % (DK / 4), t = r & (C - 1);
-            copy16(dst + r * LD + 4 * w, u + (size_t)(t0 + min(t, n - 1)) * ldu + (r < C ? k_off : q_off) + kvh * DK + 4 * w, t < n);
+    if (threadIdx.x >= MULTIPLIERS) {                    // bring
+        const int tid = threadIdx.x - MULTIPLIERS;
+        for (int j = 0; j < n_chunks; j++) {
+            const int t0 = lo + j * C, n = min(C, hi - t0);
+            {
+                Bring<DK, W::LDK> x;
+                x.read(u + (size_t)t0 * ldu + q_off + kvh * DK, ldu, n, tid);
+                if (j) bar_wait(6);
+                x.leave(sb + W::Q, tid);
+                bar_arrive(2);
+            }
+            {
+                Bring<C, W::LDT> x;
+                x.read(tp + j * tp_step, C, C, tid);
+                if (j) bar_wait(7);
+                x.leave(sb + W::T, tid);
+                bar_arrive(3);
+            }
+            {
+                Bring<DK, W::LDK> x;
+                x.read(u + (size_t)t0 * ldu + k_off + kvh * DK, ldu, n, tid);
+                if (j) bar_wait(5);
+                x.leave(sb + W::K, tid);
+                bar_arrive(1);
+            }
+            {
+                Bring<C, W::LDT> x;
+                x.read(tp + j * tp_step + C * C, C, C, tid);
+                if (j) bar_wait(8);
+                x.leave(sb + W::P, tid);
+                bar_arrive(4);
+            }
         }
-        const float* p = scratch + ((size_t)(f0 + j) * H + h) * 2 * C * C + C * C;
-        for (int i = tid; i < C * (C / 4); i += 256) copy16(Ps + (j & 1) * C * TLD + (i / (C / 4)) * TLD + 4 * (i % (C / 4)), p + 4 * i, true);
-        const float* ve = vecs + ((size_t)(f0 + j) * H + h) * VEC;
-        if (tid < VEC / 4) copy16(vec + (j & 1) * VEC + 4 * tid, ve + 4 * tid, true);
-    };
-    auto bring_tv = [&](int j) {
-        const int t0 = lo + j * C, n = min(C, hi - t0);
-        const float* p = scratch + ((size_t)(f0 + j) * H + h) * 2 * C * C;
-        for (int i = tid; i < C * (C / 4); i += 256) copy16(Ts + (i / (C / 4)) * TLD + 4 * (i % (C / 4)), p + 4 * i, true);
-        for (int i = tid; i < C * W::CG; i += 256) {
-            const int t = i / W::CG, w = col0 + 4 * (i % W::CG);
-            copy16(Vs + 4 * i, u + (size_t)(t0 + min(t, n - 1)) * ldu + v_off + h * dv + min(w, dv - 4), t < n && w < dv);
-        }
-    };
-    bring_kq(0);
-    bring_tv(0);
-    copies_commit();
-    float S[RS][4];                                      // [row k0 + r][column c]
+        return;
+    }
+
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, pair = 2 * (lane & 3);
+    int* const first = (int*)(sb + W::FIRST);
+    if (threadIdx.x < 16 * MT) first[threadIdx.x] = C;
+    const size_t per = (size_t)H * DK * dv;
+    const float* const st_in = state + ((size_t)slots[b] * 2 + ((start - 1) & 1)) * per + (size_t)h * dv * DK;
+    float* const st_out = state + ((size_t)slots[b] * 2 + ((end - 1) & 1)) * per + (size_t)h * dv * DK;
+    // element c of a lane's sums: column 16 mt + row + 8 (c / 2), token or component pair + c % 2 of the warp's piece
+    auto column = [&](int mt, int c) { return col0 + 16 * mt + row + 8 * (c >> 1); };
+    float S[NT][MT][4];
     #pragma unroll
-    for (int c = 0; c < 4; c++)
+    for (int i = 0; i < NT; i++)
         #pragma unroll
-        for (int r = 0; r < RS; r++) S[r][c] = live && start > 0 ? st_in[(size_t)c * DK + r] : 0.f;
+        for (int mt = 0; mt < MT; mt++)
+            #pragma unroll
+            for (int c = 0; c < 4; c++)
+                S[i][mt][c] = start > 0 && column(mt, c) < dv ? st_in[(size_t)column(mt, c) * DK + 8 * (w * NT + i) + pair + (c & 1)] : 0.f;
+    const unsigned base = (unsigned)__cvta_generic_to_shared(sb);
+    // where this lane's rows of second operands begin: tokens 8 w + .., pieces of 8 along the row; (K for the state) tokens .., the warp's components
+    const unsigned by_token = ((8 * w + (lane & 7)) * W::LDK + 8 * ((lane >> 3) & 1)) * 2, by_row = ((8 * w + (lane & 7)) * W::LDT + 8 * ((lane >> 3) & 1)) * 2;
+    const unsigned by_component = ((lane & 15) * W::LDK + 8 * w * NT) * 2;
 
+    float v[MT][4], g[2], e[2], g_end;                   // this chunk's, asked for a chunk ahead
+    auto ask = [&](int j) {
+        const int t0 = lo + j * C + 8 * w + pair;
+        #pragma unroll
+        for (int mt = 0; mt < MT; mt++)
+            #pragma unroll
+            for (int c = 0; c < 4; c++)
+                v[mt][c] = t0 + (c & 1) < hi && column(mt, c) < dv ? u[(size_t)(t0 + (c & 1)) * ldu + v_off + (size_t)h * dv + column(mt, c)] : 0.f;
+        const float* ve = vecs + ((size_t)(f0 + j) * H + h) * VEC;
+        #pragma unroll
+        for (int c = 0; c < 2; c++) {
+            g[c] = ve[8 * w + pair + c];
+            e[c] = ve[C + 8 * w + pair + c];
+        }
+        g_end = ve[2 * C];
+    };
+    ask(0);
+    auto leave_state = [&]() {
+        #pragma unroll
+        for (int i = 0; i < NT; i++)
+            #pragma unroll
+            for (int mt = 0; mt < MT; mt++) leave<MT>(sb + W::S, w * NT + i, mt, lane, S[i][mt]);
+    };
+    leave_state();
+    bar_multipliers();
     for (int j = 0; j < n_chunks; j++) {
-        #pragma unroll
-        for (int r = 0; r < RS; r++) *reinterpret_cast<float4*>(Ss + (k0 + r) * DS + 4 * tx) = make_float4(S[r][0], S[r][1], S[r][2], S[r][3]);
-        copies_wait();
-        __syncthreads();                                 // this chunk's K, Q, P, T, V and the state are there
-        if (j + 1 < n_chunks) { bring_kq(j + 1); copies_commit(); }
-        const float* K = KQ + (j & 1) * 2 * C * LD;
-        const float* P = Ps + (j & 1) * C * TLD;
-        const float* gam = vec + (j & 1) * VEC;
-        // K S and Q S
-        float ks[RK][4] = {}, qs[RK][4] = {};
-        #pragma unroll 2
-        for (int d = 0; d < DK; d += 4) {
-            float4 s[4], a;
+        // K S and Q S (products and sums rounded one by one: as many columns a block as there are, the bits are the same)
+        float ks[MT][4] = {}, qs[MT][4] = {};
+        {
+            float klo[MT][4] = {}, qlo[MT][4] = {};
+            bar_wait(2);
+            bar_wait(1);
             #pragma unroll
-            for (int e = 0; e < 4; e++) s[e] = at4(Ss + (d + e) * DS + 4 * tx);
-            #pragma unroll
-            for (int i = 0; i < 2 * RK; i++) {
-                a = at4(K + ((i < RK ? 0 : C) + row(i % RK)) * LD + d);
-                float (&acc)[4] = i < RK ? ks[i % RK] : qs[i % RK];
-                const float av[4] = {a.x, a.y, a.z, a.w};
+            for (int s = 0; s < KS; s++) {
+                uint4 a[MT][3];
+                unsigned kb[3][2], qb[3][2];
+                first_operand<MT>(a, sb + W::S, s, lane);
                 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    acc[0] = fmaf(av[e], s[e].x, acc[0]); acc[1] = fmaf(av[e], s[e].y, acc[1]);
-                    acc[2] = fmaf(av[e], s[e].z, acc[2]); acc[3] = fmaf(av[e], s[e].w, acc[3]);
+                for (int p = 0; p < 3; p++) {
+                    second_operand<false>(kb[p], base + W::K + by_token + (p * C * W::LDK + 16 * s) * 2);
+                    second_operand<false>(qb[p], base + W::Q + by_token + (p * C * W::LDK + 16 * s) * 2);
                 }
+                mma_planes<MT>(ks, klo, a, kb);
+                mma_planes<MT>(qs, qlo, a, qb);
             }
-        }
-        #pragma unroll
-        for (int i = 0; i < RK; i++) {
-            const int t = row(i);
-            const float4 v = at4(Vs + t * DS + 4 * tx);
-            const float g = gam[t];
-            *reinterpret_cast<float4*>(Us + t * DS + 4 * tx) = make_float4(fmaf(-g, ks[i][0], v.x), fmaf(-g, ks[i][1], v.y),
-                                                                           fmaf(-g, ks[i][2], v.z), fmaf(-g, ks[i][3], v.w));
-        }
-        __syncthreads();
-        // U = T (...), then O = G (Q S) + P U: lower triangles.  A row meets its own and earlier tokens only (not zeros times
-        // later ones: their infinities would show).
-        auto lower = [&](const float* A, float (&acc)[RK][4]) {
             #pragma unroll
-            for (int i = 0; i < RK; i++) {
-                const int t = row(i);
-                const float* a = A + t * TLD;
-                #pragma unroll 4
-                for (int s = 0; s < (t & ~3); s += 4) {
-                    const float4 a4 = at4(a + s);
-                    const float av[4] = {a4.x, a4.y, a4.z, a4.w};
-                    #pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const float4 x = at4(Us + (s + e) * DS + 4 * tx);
-                        acc[i][0] = fmaf(av[e], x.x, acc[i][0]); acc[i][1] = fmaf(av[e], x.y, acc[i][1]);
-                        acc[i][2] = fmaf(av[e], x.z, acc[i][2]); acc[i][3] = fmaf(av[e], x.w, acc[i][3]);
-                    }
-                }
-                for (int s = t & ~3; s <= t; s++) {
-                    const float w = a[s];
-                    const float4 x = at4(Us + s * DS + 4 * tx);
-                    acc[i][0] = fmaf(w, x.x, acc[i][0]); acc[i][1] = fmaf(w, x.y, acc[i][1]);
-                    acc[i][2] = fmaf(w, x.z, acc[i][2]); acc[i][3] = fmaf(w, x.w, acc[i][3]);
-                }
-            }
+            for (int mt = 0; mt < MT; mt++)
+                #pragma unroll
+                for (int c = 0; c < 4; c++) { ks[mt][c] += klo[mt][c]; qs[mt][c] = __fmul_rn(g[c & 1], qs[mt][c] + qlo[mt][c]); }
+            if (j + 1 < n_chunks) bar_arrive(6);
+        }
+        // V - G (K S).  What is not finite must not meet the zeros of earlier tokens' rows in a product: it goes in as 0, and from its token on the
+        // column's results, and its state, are NaN.
+        bool bad = false;
+        float x[MT][4];
+        auto finite = [&](float& r) {
+            if (!(fabsf(r) < 3.3e38f)) { bad = true; return 0.f; }
+            return r;
         };
-        float un[RK][4] = {};
-        lower(Ts, un);
-        __syncthreads();                                 // everybody has read the right-hand sides, T and V
-        #pragma unroll
-        for (int i = 0; i < RK; i++) {
-            const int t = row(i);
-            const float e = gam[C + t];
-            *reinterpret_cast<float4*>(Us + t * DS + 4 * tx) = make_float4(un[i][0], un[i][1], un[i][2], un[i][3]);
-            *reinterpret_cast<float4*>(Es + t * DS + 4 * tx) = make_float4(e * un[i][0], e * un[i][1], e * un[i][2], e * un[i][3]);
-        }
-        if (j + 1 < n_chunks) { bring_tv(j + 1); copies_commit(); }
-        __syncthreads();
-        const int t0 = lo + j * C;
-        #pragma unroll
-        for (int i = 0; i < RK; i++) {
-            const float g = gam[row(i)];
+        auto remember = [&](const float (&r)[MT][4]) {
             #pragma unroll
-            for (int c = 0; c < 4; c++) qs[i][c] *= g;
-        }
-        lower(P, qs);
+            for (int mt = 0; mt < MT; mt++)
+                #pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (!(fabsf(r[mt][c]) < 3.3e38f)) atomicMin(first + column(mt, c) - col0, 8 * w + pair + (c & 1));
+            bar_multipliers();
+        };
         #pragma unroll
-        for (int i = 0; i < RK; i++) {
-            const int t = t0 + row(i);
-            if (live && t < hi) *reinterpret_cast<float4*>(out + (size_t)t * H * dv + (size_t)h * dv + col) = make_float4(qs[i][0], qs[i][1], qs[i][2], qs[i][3]);
+        for (int mt = 0; mt < MT; mt++) {
+            float r[4];
+            #pragma unroll
+            for (int c = 0; c < 4; c++) {
+                x[mt][c] = fmaf(-g[c & 1], ks[mt][c], v[mt][c]);
+                r[c] = finite(x[mt][c]);
+            }
+            leave<MT>(sb + W::R, w, mt, lane, r);
         }
-        // the state: S <- G_end S + K^T E
-        const float g_end = gam[2 * C];
-        #pragma unroll
-        for (int r = 0; r < RS; r++)
+        const float e0 = e[0], e1 = e[1], ge = g_end;
+        if (j + 1 < n_chunks) ask(j + 1);
+        bool any = bar_any(bad);
+        if (any) remember(x);
+        // U = T (..): a row meets its own and earlier steps of 16 tokens
+        {
+            float hi4[MT][4] = {}, lo4[MT][4] = {};
+            bar_wait(3);
             #pragma unroll
-            for (int c = 0; c < 4; c++) S[r][c] *= g_end;
-        #pragma unroll 4
-        for (int t = 0; t < C; t++) {
-            const float4 x = at4(Es + t * DS + 4 * tx);
-            float a[RS];
-            if (RS == 4) { const float4 a4 = at4(K + t * LD + k0); a[0] = a4.x; a[1 % RS] = a4.y; a[2 % RS] = a4.z; a[3 % RS] = a4.w; }
-            else if (RS == 2) { const float2 a2 = *reinterpret_cast<const float2*>(K + t * LD + k0); a[0] = a2.x; a[1 % RS] = a2.y; }
-            else a[0] = K[t * LD + k0];
+            for (int s = 0; s < 4; s++)
+                if (s <= w >> 1) {
+                    uint4 a[MT][3];
+                    unsigned tb[3][2];
+                    first_operand<MT>(a, sb + W::R, s, lane);
+                    #pragma unroll
+                    for (int p = 0; p < 3; p++) second_operand<false>(tb[p], base + W::T + by_row + (p * C * W::LDT + 16 * s) * 2);
+                    mma_planes<MT>(hi4, lo4, a, tb);
+                }
+            if (j + 1 < n_chunks) bar_arrive(7);
+            bad = false;
             #pragma unroll
-            for (int r = 0; r < RS; r++) {
-                S[r][0] = fmaf(a[r], x.x, S[r][0]); S[r][1] = fmaf(a[r], x.y, S[r][1]);
-                S[r][2] = fmaf(a[r], x.z, S[r][2]); S[r][3] = fmaf(a[r], x.w, S[r][3]);
+            for (int mt = 0; mt < MT; mt++) {
+                float r[4], re[4];
+                #pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    x[mt][c] = hi4[mt][c] + lo4[mt][c];
+                    r[c] = finite(x[mt][c]);
+                    re[c] = __fmul_rn((c & 1) ? e1 : e0, r[c]);
+                }
+                leave<MT>(sb + W::U, w, mt, lane, r);
+                leave<MT>(sb + W::E, w, mt, lane, re);
             }
         }
-        // (the copy of the state is written anew before the next barrier; it was last read before the one after K S)
-    }
-    if (live) {
-        #pragma unroll
-        for (int c = 0; c < 4; c++)
+        if (bar_any(bad)) {
+            any = true;
+            remember(x);
+        }
+        // O = G (Q S) + P U
+        {
+            float hi4[MT][4] = {}, lo4[MT][4] = {};
+            bar_wait(4);
             #pragma unroll
-            for (int r = 0; r < RS; r++) st_out[(size_t)c * DK + r] = S[r][c];
+            for (int s = 0; s < 4; s++)
+                if (s <= w >> 1) {
+                    uint4 a[MT][3];
+                    unsigned pb[3][2];
+                    first_operand<MT>(a, sb + W::U, s, lane);
+                    #pragma unroll
+                    for (int p = 0; p < 3; p++) second_operand<false>(pb[p], base + W::P + by_row + (p * C * W::LDT + 16 * s) * 2);
+                    mma_planes<MT>(hi4, lo4, a, pb);
+                }
+            if (j + 1 < n_chunks) bar_arrive(8);
+            const int t0 = lo + j * C + 8 * w + pair;
+            #pragma unroll
+            for (int mt = 0; mt < MT; mt++)
+                #pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    float o = qs[mt][c] + (hi4[mt][c] + lo4[mt][c]);
+                    if (any && 8 * w + pair + (c & 1) >= first[column(mt, c) - col0]) o = CUDART_NAN_F;
+                    if (t0 + (c & 1) < hi && column(mt, c) < dv) out[(size_t)(t0 + (c & 1)) * H * dv + (size_t)h * dv + column(mt, c)] = o;
+                }
+        }
+        // the state: S <- G_end S + K^T ((G_end / G) U)
+        {
+            float hi4[NT][MT][4] = {}, lo4[NT][MT][4] = {};
+            #pragma unroll
+            for (int s = 0; s < 4; s++) {
+                uint4 a[MT][3];
+                first_operand<MT>(a, sb + W::E, s, lane);
+                #pragma unroll
+                for (int i = 0; i < NT; i++) {
+                    unsigned kb[3][2];
+                    #pragma unroll
+                    for (int p = 0; p < 3; p++) second_operand<true>(kb[p], base + W::K + by_component + ((p * C + 16 * s) * W::LDK + 8 * i) * 2);
+                    mma_planes<MT>(hi4[i], lo4[i], a, kb);
+                }
+            }
+            if (j + 1 < n_chunks) bar_arrive(5);
+            #pragma unroll
+            for (int i = 0; i < NT; i++)
+                #pragma unroll
+                for (int mt = 0; mt < MT; mt++)
+                    #pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        S[i][mt][c] = fmaf(ge, S[i][mt][c], hi4[i][mt][c] + lo4[i][mt][c]);
+                        if (any && first[column(mt, c) - col0] < C) S[i][mt][c] = CUDART_NAN_F;
+                    }
+        }
+        if (j + 1 < n_chunks) {
+            leave_state();                               // (last read before the barrier behind V - G (K S))
+            bar_multipliers();
+            if (any && threadIdx.x < 16 * MT) first[threadIdx.x] = C;      // (next touched behind the next barrier)
+        }
     }
+    #pragma unroll
+    for (int i = 0; i < NT; i++)
+        #pragma unroll
+        for (int mt = 0; mt < MT; mt++)
+            #pragma unroll
+            for (int c = 0; c < 4; c++)
+                if (column(mt, c) < dv) st_out[(size_t)column(mt, c) * DK + 8 * (w * NT + i) + pair + (c & 1)] = S[i][mt][c];
 }
 
-template <int DK, int DS, bool SOME>
+template <int DK, int MT, bool SOME>
 int walk(const float* u, int ldu, int q_off, int k_off, int v_off, const float* scratch, const float* vecs, float* state, const int* slots,
          const int* cu_seqlens, const int* kv_lens, float* out, int B, int least, int n_walked, int H, int G, int dv, cudaStream_t stream) {
-    constexpr size_t smem = Walk<DK, DS>::FLOATS * sizeof(float);
-    const cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<DK, DS, SOME>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr size_t smem = Walk<DK, MT>::BYTES;
+    const cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<DK, MT, SOME>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    IK_RETURN_IF_ERROR(ik_launch(delta_chunk_kernel<DK, DS, SOME>, dim3((dv + DS - 1) / DS, H, n_walked), 256, smem, stream, u, ldu, q_off, k_off, v_off,
-                                 scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, H, G, dv));
+    IK_RETURN_IF_ERROR(ik_launch(delta_chunk_kernel<DK, MT, SOME>, dim3((dv + 16 * MT - 1) / (16 * MT), H, n_walked), ALL, smem, stream, u, ldu, q_off, k_off,
+                                 v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, H, G, dv));
     IK_LAUNCH_STATUS();
 }
 
@@ -421,8 +615,8 @@ int chunks(const float* u, int ldu, int q_off, int k_off, int v_off, const float
                                  cu_seqlens, B, least, H, G));
     // 32 columns a block do a third fewer loads per multiply-add; 16 where that leaves more than half of the SMs idle
     if (2LL * n_walked * H * ((dv + 31) / 32) <= ik_sm_count())
-        return walk<DK, 16, SOME>(u, ldu, q_off, k_off, v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, H, G, dv, stream);
-    return walk<DK, 32, SOME>(u, ldu, q_off, k_off, v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, H, G, dv, stream);
+        return walk<DK, 1, SOME>(u, ldu, q_off, k_off, v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, H, G, dv, stream);
+    return walk<DK, 2, SOME>(u, ldu, q_off, k_off, v_off, scratch, vecs, state, slots, cu_seqlens, kv_lens, out, B, least, n_walked, H, G, dv, stream);
 }
 
 }  // namespace

@@ -83,3 +83,22 @@ def test_what_is_not_finite_stays_behind_its_token(where):
     got = ops.delta_rule(bad_u, *args, bad_bg, before.clone(), ctx, H, G, dk, dv, chunks=True)
     assert torch.equal(got[:101], whole[:101])
     assert not torch.isfinite(got[101]).all() and not torch.isfinite(got[149]).all()
+
+
+@pytest.mark.parametrize("H,G,dk,dv", [(3, 1, 128, 36), (2, 2, 64, 64), (40, 8, 128, 64)])            # 16 and 32 columns a block
+def test_columns_beside_one_that_is_not_finite(H, G, dk, dv):
+    from ithaca_b200.csrc import ops
+    u, bg, before, ctx, cu, slots = make(H, G, dk, dv, [200, 64], [0, 9], 4, "usual")
+    args = (4, 4 + G * dk, 4 + 2 * G * dk, bg)
+    state, state1, bad = before.clone(), before.clone(), u.clone()
+    whole = ops.delta_rule(u, *args, state, ctx, H, G, dk, dv, chunks=True)
+    col = (H - 1) * dv + 19
+    bad[77, 4 + 2 * G * dk + col] = float("-inf")
+    got = ops.delta_rule(bad, *args, state1, ctx, H, G, dk, dv, chunks=True)
+    others = torch.arange(H * dv, device=DEV) != col
+    assert torch.equal(got[:, others], whole[:, others]) and torch.equal(got[:77], whole[:77]) and torch.equal(got[200:], whole[200:])
+    assert not torch.isfinite(got[77:200, col]).any()
+    p = 199 & 1
+    assert not torch.isfinite(state1[slots[0], p, H - 1, 19]).any()
+    state1[slots[0], p, H - 1, 19] = state[slots[0], p, H - 1, 19]
+    assert torch.equal(state1, state)
