@@ -376,7 +376,7 @@ def products_sweep(cfg, token_counts, reps):
                     continue
                 variants[label] = (lambda s_: lambda w: ops.gemm_tcgen05(x, w, out=y, status=status, splits=s_))(s)
             variants["cublas"] = lambda w: torch.matmul(x, w.T, out=yb)
-            row = {"product": name, "rows": n, "k": k, "tokens": tokens, "picked_splits": None if ops.wide_takes(tokens, n, k) else ops.tcgen05_splits(tokens, n, k), "picked_wide": ops.wide_takes(tokens, n, k),
+            row = {"product": name, "rows": n, "k": k, "tokens": tokens, "picked_splits": None if ops.wide_takes(tokens, n, k) or ops.batch_takes(tokens, n, k) else ops.tcgen05_splits(tokens, n, k), "picked_wide": ops.wide_takes(tokens, n, k),
                    "picked_skinny": gemm_bf16.takes_skinny(tokens, n, k), "ideal_us": round(n * k * 2 / pk_hbm() / 1e3, 1)}
             for label, fn in variants.items():
                 for w in ws[:2]:

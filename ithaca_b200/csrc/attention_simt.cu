@@ -6,8 +6,8 @@
 // absolute multiples of 128 (the tiles of the first `keep` keys, which stay visible behind the window, come first), so the order in which a query's keys are reduced depends
 // only on its position, not on how the tokens were cut into steps or batched.
 // Scores, the running maximum, the sum and the output are float; exp is the accurate
-// function.  This is the 32-bit path's attention and the fallback for head sizes the
-// tensor-core kernels do not take.  Options: a cap on the scores, s <- cap * tanh(s / cap) after the scale
+// function.  This is the 32-bit path's attention (prompts without options of head sizes 64 and 128 run in attention_rows.cu, with the
+// same bits) and the fallback for head sizes the tensor-core kernels do not take.  Options: a cap on the scores, s <- cap * tanh(s / cap) after the scale
 // (cap 0 = none), value heads of another size than the key heads (hdv), values that are the leading hdv columns of the
 // key rows themselves (v_pages = k_pages with ldv = hd: a latent that serves as key and value), and a sink: one more
 // key of score 0 that carries no value, so that the weights are exp(s_j) / (1 + sum exp(s_j)).  Under a window the first

@@ -515,8 +515,8 @@ def tcgen05_cluster_fits(M: int, N: int, K: int, n_cl: int) -> bool:
 
 
 def tcgen05_splits(M: int, N: int, K: int) -> int:
-    """How the tcgen05 product shares out its work: 1 = whole tiles dealt round robin; n > 1 = n slices
-    of K and a second kernel that adds them; 0 = stream-K (equal shares of all K steps of all tiles);
+    """How gemm_tcgen05.cu shares out the work of the products that are left to it (``batch_takes``, ``wide_takes``): 1 = whole tiles
+    dealt round robin; n > 1 = n slices of K and a second kernel that adds them; 0 = stream-K (equal shares of all K steps of all tiles);
     -n = clusters of n blocks per tile, each a slice of K, summed in shared memory (no scratch, one kernel).
     Measured on B200 with 2048 x 2048 .. 28672 x 4096 weights (``bench.py --only products --tokens ...``): with
     fewer tiles than half the SMs, K is sliced: by clusters of 2 or 4 where that busies at least half the SMs (clusters

@@ -262,9 +262,9 @@ template <bool FAST> __device__ __forceinline__ float ik_scan_step(float S, floa
 // states into the pieces' states at entry, S <- exp(a * sum dt) S + S_piece; MODE 2 runs the pieces from there and writes the
 // results.  MODE 0: whole sequences.  Pieces have flat numbers: piece j of sequence b is cu_seqlens[b] / piece + b + j, of
 // which there are at most T / piece + B.
-// Which steps go this way: ops.scan_pieces_pay.  Measured on B200, 4,096 channels of 16 states: prompts of 3,000 and 1,910 tokens 685 us
-// with a shuffle tree per token, 399 with the sums of a channel's lanes exchanged L tokens at a time (below), 380 in pieces as well;
-// one prompt of 4,000 832 / 454 / 318.
+// Which steps go this way: ops.scan_pieces_pay, and ops.scan_pieces_beat_stream where whole sequences run in selective_scan_stream_kernel.  Measured on
+// B200, 4,096 channels of 16 states: prompts of 3,000 and 1,910 tokens 685 us with a shuffle tree per token, 399 with the sums of a channel's lanes
+// exchanged L tokens at a time (below), 380 in pieces as well, 193 in the stream kernel.
 struct ScanPieces {
     int piece;                                        // tokens; 0 = whole sequences
     int n_seqs;
