@@ -67,14 +67,15 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k_p
             b++;
         }
         const int row_lo = a * heads, row_hi = b * heads;
-        const int first = window > 0 && least + 1 > window ? (least + 1 - window) / TILE : 0;
+        // (the pages before the first key that any of the run's rows sees may have been given back)
+        const int seen = window > 0 && least + 1 > window ? least + 1 - window : 0, first = seen / TILE;
         for (int tile = first; tile * TILE <= most; tile++) {
             const int base = tile * TILE, n_keys = min(TILE, most - base + 1);
             if (tid < n_keys) {
-                const int page = table[(size_t)seq * table_stride + (base + tid) / page_size];
+                const int page = base + tid < seen ? 0 : table[(size_t)seq * table_stride + (base + tid) / page_size];
                 size_t off = 0;
                 if (page < 0 || page >= n_pages) ik_set_status(status, IK_STATUS_READ_NO_PAGE);
-                else off = ((size_t)page * nkv + kvh) * page_size + (base + tid) % page_size;
+                else if (base + tid >= seen) off = ((size_t)page * nkv + kvh) * page_size + (base + tid) % page_size;
                 place[tid] = off;
             }
             __syncthreads();

@@ -53,6 +53,27 @@ def test_a_missing_page_is_reported():
     assert status.item() != 0 and torch.equal(got, ops.attention_simt(q, k, v, seq, pos, table, nh, scale, 0, status))
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("new,old,window", [([200], [300], 100), ([65, 70], [500, 129], 64), ([3, 90], [640, 200], 129), ([130, 1, 40], [0, 300, 0], 70)])
+def test_pages_behind_the_window_may_be_gone(hd, new, old, window):
+    """A cache gives back the pages that lie wholly before the first key a window still reaches (their column of the table is -1): nothing is
+    missed, and nothing of what the pool's first row holds instead gets into the result."""
+    from ithaca_b200.csrc import ops
+    q, k, v, seq, pos, table, nh, scale = made(8, 2, hd, new, old, 5)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    gone = 0
+    for i, o in enumerate(old):
+        n = max(0, o + 1 - window) // 64
+        table[i, :n] = -1
+        gone += n
+    k[0, :, 0], v[0, :, 0] = float("nan"), float("nan")
+    table[table == 0] = k.shape[0] - 1
+    k[-1], v[-1] = 0.5, 0.25
+    rows, simt = (f(q, k, v, seq, pos, table, nh, scale, window, status) for f in (ops.attention_rows, ops.attention_simt))
+    assert gone > 0 and status.item() == 0 and torch.equal(rows, simt) and bool(torch.isfinite(rows).all())
+
+
 # measured on B200: heads, kv heads, new tokens, tokens before them, window, us a token a block, us these
 @pytest.mark.parametrize("nh,nkv,new,old,window,simt,rows", [
     (32, 8, [1], [0], 0, 4.5, 8.5), (32, 8, [20], [0], 0, 7.1, 11.5), (32, 8, [64], [0], 0, 13.9, 15.3), (32, 8, [300, 35, 130], [0] * 3, 0, 119, 60),
