@@ -194,9 +194,9 @@ delta_chunk_prepare_kernel(const float* __restrict__ u, int ldu, int q_off, int 
             }
         __syncthreads();
     }
-    for (int i = tid; i < C * C; i += 256) {
+    for (int i = tid; i < C * C; i += 256) {                 // (0, not 0 * beta, above the diagonal: the walk reads whole blocks of 16)
         const int t = i / C, s = i % C;
-        outT[i] = (s >> 4) <= (t >> 4) ? Ts[t * TLD + s] * beta[s] : 0.f;
+        outT[i] = s <= t ? Ts[t * TLD + s] * beta[s] : 0.f;
     }
 }
 

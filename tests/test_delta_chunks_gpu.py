@@ -68,7 +68,7 @@ def test_delta_rule_in_chunks(H, G, dk, dv, new, start, decay):
     assert torch.equal(state[0], before[0])
 
 
-@pytest.mark.parametrize("where", ["k", "v", "decay"])
+@pytest.mark.parametrize("where", ["k", "v", "decay", "factor"])
 def test_what_is_not_finite_stays_behind_its_token(where):
     from ithaca_b200.csrc import ops
     H, G, dk, dv = 2, 1, 128, 64
@@ -76,8 +76,8 @@ def test_what_is_not_finite_stays_behind_its_token(where):
     args = (4, 4 + G * dk, 4 + 2 * G * dk)
     whole = ops.delta_rule(u, *args, bg, before.clone(), ctx, H, G, dk, dv, chunks=True)
     bad_u, bad_bg = u.clone(), bg.clone()
-    if where == "decay":
-        bad_bg[101, 1] = float("nan")
+    if where in ("decay", "factor"):
+        bad_bg[101, int(where == "decay")] = float("nan")
     else:
         bad_u[101, 4 + G * dk if where == "k" else 4 + 2 * G * dk + 5] = float("inf") if where == "v" else float("nan")
     got = ops.delta_rule(bad_u, *args, bad_bg, before.clone(), ctx, H, G, dk, dv, chunks=True)
