@@ -457,7 +457,8 @@ selective_scan_kernel(const TU* __restrict__ u, const float* __restrict__ dt_raw
 // results of the tile before; the four last warps do nothing but the recurrence, a thread four states of a channel, L lanes a channel, CH channels a
 // block, two states per instruction where the hardware has one (mul and fma of f32x2).  So neither waits for the other's latency: a token
 // takes 40 ns with a block to an SM, and with more the reads from shared memory (10 to 14 cycles a warp and token), the exponentials (four a
-// cycle and scheduler) and the issue slots bind about evenly.  Tokens that are not there have a step size of 0: a factor of 1 and nothing added.
+// cycle and scheduler) and the issue slots bind about evenly.  Tokens that are not there have a step size and an
+// input of 0: a factor of 1 and nothing added.
 // Measured on B200, 4,096 channels of 16 states (us, the kernel above / this): one prompt of 200 25 / 10, of 3,000 341 / 125, 3,000 + 1,910 399 / 193,
 // eight of 2,000 790 / 437.  One team alone took 231 for 3,000 + 1,910 (a tile's softplus, gates and stores are 225 instructions of one
 // warp in sequence); two states a thread and twice the warps 220; with the sums of four tokens stored before the next four's reads 221.
@@ -582,7 +583,7 @@ selective_scan_stream_kernel(const __nv_bfloat16* __restrict__ u, const float* _
                 const bool there = lo + j * TT + tt < hi;
                 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    const float x = __uint_as_float(((i & 1) ? (i < 2 ? r.u.x : r.u.y) & 0xffff0000u : (i < 2 ? r.u.x : r.u.y) << 16));
+                    const float x = there ? __uint_as_float(((i & 1) ? (i < 2 ? r.u.x : r.u.y) & 0xffff0000u : (i < 2 ? r.u.x : r.u.y) << 16)) : 0.f;
                     const float dt = there ? ik_softplus_as<true>((&r.d.x)[i] + bias[i]) : 0.f;
                     *reinterpret_cast<float2*>(tile + Tile::place(tt, tid % QC, i)) = make_float2(dt, dt * x);
                     *reinterpret_cast<float2*>(tile + Tile::XG + Tile::place(tt, tid % QC, i)) = make_float2(x, ik_silu_as<true>((&r.z.x)[i]));
@@ -613,8 +614,8 @@ selective_scan_stream_kernel(const __nv_bfloat16* __restrict__ u, const float* _
             #pragma unroll
             for (int i = 0; i < 2; i++) {
                 const int n = 4 * l + 2 * r + i;
-                // (an A of minus infinity: a step size of 0 still leaves the state alone)
-                e[i] = n < N ? fmaxf(A[(size_t)cc * N + n] * 1.44269504f, -3.4e38f) : 0.f;
+                e[i] = n < N ? A[(size_t)cc * N + n] * 1.44269504f : 0.f;
+                if (fabsf(e[i]) > 3.4e38f) e[i] = copysignf(3.4e38f, e[i]);          // (an infinite A: a step size of 0 still leaves the state alone; NaN stays)
                 s[i] = n < N && start > 0 ? st_in[n] : 0.f;
             }
             S[r] = ik_pack2(s[0], s[1]);

@@ -56,6 +56,34 @@ def test_stream(inner, N, new, start, less, odt):
     assert torch.equal(state[0], before[0])
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("inner,N", [(40, 17), (64, 16)])                      # values one by one, and by fours
+@pytest.mark.parametrize("T", [16, 21])
+def test_numbers_that_are_not_finite(inner, N, T):
+    """A NaN in A makes its channel's results and that state NaN; an infinite last input makes its channel's states infinite, also where the last tile
+    is not full.  Other channels keep their bits."""
+    from ithaca_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(T)
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)
+    u, dt, bc, z = rnd(T, inner).to(torch.bfloat16), rnd(T, inner), rnd(T, 4 + 2 * N), rnd(T, 2 * inner)[:, inner:]
+    A, D, before = -torch.exp(rnd(inner, N) * 0.5), rnd(inner), rnd(1, 2, inner, N)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    ctx = SimpleNamespace(n_seqs=1, max_new=T, slots=i32([0]), cu_seqlens=i32([0, T]), kv_lens=i32([T + 2]), is_decode=False)
+
+    def run(u, A):
+        state = before.clone()
+        return ops.selective_scan(u, dt, None, A, bc, 4, 4 + N, D, z, state, ctx, torch.float32, pieces=False), state[0, (T + 1) & 1]
+    y0, S0 = run(u, A)
+    bad_A, bad_u = A.clone(), u.clone()
+    bad_A[3, 2], bad_u[T - 1, 7] = float("nan"), float("inf")
+    y, S = run(bad_u, bad_A)
+    assert bool(y[:, 3].isnan().all()) and bool(S[3, 2].isnan()) and int(S.isnan().sum()) == 1
+    assert torch.equal(S[7], torch.copysign(torch.full_like(S[7], float("inf")), bc[T - 1, 4:4 + N])) and not bool(torch.isfinite(y[T - 1, 7]))
+    same = torch.ones(inner, dtype=torch.bool, device=DEV)
+    same[3] = same[7] = False
+    assert torch.equal(y[:, same], y0[:, same]) and torch.equal(S[same], S0[same]) and torch.equal(y[:T - 1, 7], y0[:T - 1, 7])
+
+
 # measured on B200: channels, states, step's longest and number of sequences, us whole, us in pieces
 MEASURED = [(256, 16, 4000, 1, 152, 55), (512, 16, 8000, 1, 297, 110), (512, 16, 2000, 8, 86, 179), (2048, 16, 2000, 1, 80, 98), (2048, 16, 2000, 2, 86, 174),
             (4096, 16, 4000, 1, 167, 325), (64, 16, 2000, 1, 79, 41), (256, 64, 4000, 1, 177, 91), (1024, 64, 4000, 1, 179, 282), (1024, 64, 2000, 8, 504, 1001)]
