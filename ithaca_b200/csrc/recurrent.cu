@@ -615,7 +615,9 @@ selective_scan_stream_kernel(const __nv_bfloat16* __restrict__ u, const float* _
             for (int i = 0; i < 2; i++) {
                 const int n = 4 * l + 2 * r + i;
                 e[i] = n < N ? A[(size_t)cc * N + n] * 1.44269504f : 0.f;
-                if (fabsf(e[i]) > 3.4e38f) e[i] = copysignf(3.4e38f, e[i]);          // (an infinite A: a step size of 0 still leaves the state alone; NaN stays)
+                // (an infinite A: a step size of 0 still leaves the state alone; NaN stays)
+                asm("max.NaN.f32 %0, %0, %1;" : "+f"(e[i]) : "f"(-3.4e38f));
+                asm("min.NaN.f32 %0, %0, %1;" : "+f"(e[i]) : "f"(3.4e38f));
                 s[i] = n < N && start > 0 ? st_in[n] : 0.f;
             }
             S[r] = ik_pack2(s[0], s[1]);
