@@ -239,9 +239,9 @@ def attend(q, k_pages, v_pages, ctx, table, n_heads: int, scale: float, window: 
         rows = hd * 2 + 4 if key_scales is not None else 2 * hd * 2             # bytes of a key (and value) per kv head
         work = (2 * q.numel() * 2 + keys * nkv * rows, 4 * hd * n_heads * pairs)
     if ctx.is_decode:
-        # from the bound, not from this step's longest sequence: a captured graph is replayed for other lengths
+        # from the bound; the single lengths have a say only where the step is not captured: a graph is replayed for other lengths
         chunk = decode_chunk_pages(ctx.n_seqs, n_heads, nkv, seen_pages(ctx.kv_len_bound, window, keep, page_size) * page_size, page_size)
-        if len(ctx.host_kv_lens) == ctx.n_seqs > 1:
+        if len(ctx.host_kv_lens) == ctx.n_seqs > 1 and not getattr(ctx, "replayed", False):
             key = ("decode_chunk", n_heads, nkv, window, keep, page_size)              # once for all layers of a kind
             if key not in ctx.shared:
                 ctx.shared[key] = decode_chunk_pages_uneven([seen_pages(e, window, keep, page_size) for e in ctx.host_kv_lens], n_heads, nkv, chunk, sm_count())

@@ -31,6 +31,7 @@ class StepContext:
     max_new: int
     max_kv_len: int
     kv_len_bound: int = 0              # no sequence is longer than this (sizes grids; >= max_kv_len)
+    replayed: bool = False             # captured, and replayed for other lengths than this step's: only the bound counts
     host_slots: List[int] = field(default_factory=list)
     host_n_new: List[int] = field(default_factory=list)
     host_kv_lens: List[int] = field(default_factory=list)

@@ -67,8 +67,8 @@ class _Launched:
 def _bucket(cols: int) -> int:
     """Block-table widths are rounded up so that a growing sequence re-captures rarely: to multiples of 4 up to 32,
     then in four steps per doubling (40, 48, 56, 64, 80, ...).  What a captured step derives from the length of its
-    longest sequence (grid sizes, the chunk length of decode attention) it derives from the width's upper end, so
-    beyond 1,024 positions no graph is replayed for a longest sequence shorter than four fifths of what it was shaped for."""
+    longest sequence (grid sizes, the chunk length of decode attention) it derives from the width's upper end, and nothing
+    from the single lengths, so beyond 1,024 positions no graph is replayed for a longest sequence shorter than four fifths of what it was shaped for."""
     p = 4
     while 2 * p < cols:
         p *= 2
@@ -254,7 +254,8 @@ class GraphDecoder:
         offsets, sizes, total = field_offsets([B, B, B, B + 1, B, B, B] + [B * cols] * n_groups)
         buffer = torch.empty(total, dtype=torch.int32, device=st.runtime.device)
         ctx = st.prepare(slots, tokens, "last", into=buffer, table_cols=cols)
-        ctx.kv_len_bound = cols * page
+        # the graph is replayed for other lengths: what the kernels choose for it follows from its shape alone, not from which lengths came first
+        ctx.kv_len_bound, ctx.replayed = cols * page, True
         torch.cuda.current_stream().synchronize()
         st.model.forward(ctx, st.cache)                      # eager warm-up: writes this step's keys and values
         torch.cuda.current_stream().synchronize()
