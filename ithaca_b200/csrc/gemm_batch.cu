@@ -27,7 +27,7 @@
 namespace {
 
 typedef __nv_bfloat16 bf16;
-constexpr int BK = 64, EPI_WARPS = 8, THREADS = 128 + 32 * EPI_WARPS, MOST_STAGES = 12, BUDGET = 215 * 1024;
+constexpr int BK = 64, EPI_WARPS = 8, THREADS = 128 + 32 * EPI_WARPS, MOST_STAGES = 12, BUDGET = 215 * 1024, MOST_SMEM = BUDGET + 1536;
 constexpr int A_BYTES = 128 * BK * 2;
 template <int BN, int CG> constexpr int stage_bytes() { return A_BYTES + BN / CG * BK * 2; }
 enum { OUT_F32 = 0, OUT_BF16 = 1, OUT_JOIN = 2, OUT_ROPE = 3, OUT_ACT = 4 };
@@ -366,7 +366,8 @@ int launch_batch(const CUtensorMap& mx, const CUtensorMap& mw, BatchArgs& g, cud
     g.stages = (BUDGET - room) / STAGE;
     if (g.stages > MOST_STAGES) g.stages = MOST_STAGES;
     const int smem = g.stages * STAGE + room + 1024 + 512;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // the most of any call, not this one's: another thread may launch the same instance for another share in between
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST_SMEM);
     if (e != cudaSuccess) return (int)e;
     const int most = ik_sm_count() / CG;
     cudaLaunchConfig_t cfg = {};
@@ -399,10 +400,10 @@ int clusters_of_four() {
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 4; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3(4 * 64); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = BUDGET + 1536;
+        cfg.gridDim = dim3(4 * 64); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = MOST_SMEM;
         cfg.attrs = attr; cfg.numAttrs = 1;
         int n = 0;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BUDGET + 1536) != cudaSuccess ||
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST_SMEM) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
             (void)cudaGetLastError();
             n = ik_sm_count() / 5;

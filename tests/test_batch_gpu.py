@@ -103,3 +103,32 @@ def test_products_take_the_faster_way(M, N, K, other, here, monkeypatch):
     from ithaca_b200.csrc import ops
     monkeypatch.setattr(ops, "sm_count", lambda: 148)
     assert ops.batch_takes(M, N, K) == (here < other)
+
+
+@pytest.mark.gpu
+def test_two_threads_with_other_shares():
+    """Two shares of one instance want other amounts of shared memory: neither thread's launch is refused for what the other asked for."""
+    import threading
+
+    from ithaca_b200.csrc import ops
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    x, w = rnd((40, 1024), 1), rnd((256, 1024), 2)
+    want = {way: ops.gemm_tcgen05(x, w, batch=way, status=status) for way in (17, 18, 20)}
+    failed = []
+
+    def work(way):
+        y = torch.empty_like(want[way])
+        try:
+            for _ in range(3000):
+                ops.gemm_tcgen05(x, w, out=y, batch=way, status=status)
+            torch.cuda.synchronize()
+            if not torch.equal(y, want[way]):
+                failed.append(f"{way}: other bits")
+        except Exception as e:
+            failed.append(f"{way}: {e}")
+    threads = [threading.Thread(target=work, args=(way,)) for way in (17, 18, 20)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed and status.item() == 0
