@@ -117,7 +117,7 @@ def test_two_threads_with_other_shares():
     failed = []
 
     def work(way):
-        y = torch.empty_like(want[way])
+        y = torch.zeros_like(want[way])                         # (a kernel: the thread has the device's context from here on)
         try:
             for _ in range(3000):
                 ops.gemm_tcgen05(x, w, out=y, batch=way, status=status)
