@@ -3,8 +3,9 @@
 //
 // A float is the sum of three bfloat16 numbers without a remainder (its 24 significant bits in three eights), and a product of two
 // bfloat16 numbers is a float without rounding.  So X goes to the tensor core as three planes, each multiplied by W, and nothing is lost
-// before the sums (but what a number below 2^-110 has under 2^-133).  Those are what the error comes from: tcgen05.mma drops the bits that do
-// not fit when it adds to its accumulator, always towards zero, so a long chain of them leans.  Here a chain is 64 k: eight instructions for
+// before the sums.  (The small planes are stored 2^7 and 2^15 times too large, and what has been summed is scaled down where the next plane's
+// products begin, so that a small number's last bits do not fall below 2^-133, the least bfloat16; only the last bit of a number below 2^-125
+// does.)  The sums are what the error comes from: tcgen05.mma drops the bits that do not fit when it adds to its accumulator, always towards zero, so a long chain of them leans.  Here a chain is 64 k: eight instructions for
 // the two small planes, then four for the large one.  The chain's sum is taken out of TMEM and added to a float in registers,
 // rounded to nearest, while the next chains run in other columns of TMEM.  Slices of K, cut by K alone, join in their order what Y
 // holds: a row of Y has the same bits whatever other rows are in the call, whatever tile takes it, and whether the slices run one after another in one
@@ -20,6 +21,7 @@
 // What bounds it: with many tokens the tensor pipe (three times the operations of a 16-bit product), with few the bytes of W and the start.
 // Measured on B200 (us in replayed graphs, with the kernels that form the planes and add the slices; gemm_simt.cu / this): 2,048 tokens x 16384 x
 // 2048 2,446 / 276 (498 TFLOP/s), 2048 x 8192 1,443 / 179; 465 tokens 737 / 76, 475 / 47; 1 token 177 / 15, 302 / 17; 128256 x 2048 for 3 tokens 861 / 84.
+#include <type_traits>
 #define IK_FAMILY 8
 #include "tc_common.cuh"
 
@@ -29,6 +31,7 @@ typedef __nv_bfloat16 bf16;
 constexpr int BK = 64;
 constexpr int A_BYTES = 128 * BK * 2;
 constexpr int MAX_SLICES = 8;
+constexpr int MID_SCALE = 7, LOW_SCALE = 15;          // powers of two by which the small planes are stored too large
 template <int BN> struct Cfg {
     static constexpr int PLANE = BN / 2 * BK * 2;                  // a block's half of the tokens, one plane
     static constexpr int STAGE = A_BYTES + 3 * PLANE;
@@ -54,10 +57,17 @@ __device__ __forceinline__ void load_pair_3d(uint32_t dst, const CUtensorMap* ma
     asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
                  :: "r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
 }
+// D = A B + D 2^-SCALE (acc = 0: D = A B).
+template <int SCALE>
 __device__ __forceinline__ void product_pair(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t acc) {
-    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
-                 "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t}"
-                 :: "r"(d), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(acc) : "memory");
+    if (SCALE)
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+                     "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p, %6;\n\t}"
+                     :: "r"(d), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(acc), "n"(SCALE) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+                     "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t}"
+                     :: "r"(d), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(acc) : "memory");
 }
 // Arrives on the barrier (at the same place in both blocks) once the products issued so far are done.
 __device__ __forceinline__ void commit_pair(uint64_t* bar) {
@@ -183,11 +193,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                     const uint32_t acc = tmem + buf * BN, a_lo = lo0 + (uint32_t)s * (C::STAGE >> 4), b_lo = a_lo + (A_BYTES >> 4);
                     if (elect_one()) {
                         // the small planes first: their sums are far below the last bit of the large one's
+                        auto product = [&](auto scale, int p, int j) {
+                            product_pair<decltype(scale)::value>(acc, a_lo + 2 * j, b_lo + p * (PLANE >> 4) + 2 * j, hi, idesc, (uint32_t)(p != 2 || j != 0));
+                        };
+                        product(std::integral_constant<int, 0>(), 2, 0);
                         #pragma unroll
-                        for (int p = 2; p >= 0; p--)
-                            #pragma unroll
-                            for (int j = 0; j < BK / 16; j++)
-                                product_pair(acc, a_lo + 2 * j, b_lo + p * (PLANE >> 4) + 2 * j, hi, idesc, (uint32_t)(p != 2 || j != 0));
+                        for (int j = 1; j < BK / 16; j++) product(std::integral_constant<int, 0>(), 2, j);
+                        product(std::integral_constant<int, LOW_SCALE - MID_SCALE>(), 1, 0);
+                        #pragma unroll
+                        for (int j = 1; j < BK / 16; j++) product(std::integral_constant<int, 0>(), 1, j);
+                        product(std::integral_constant<int, MID_SCALE>(), 0, 0);
+                        #pragma unroll
+                        for (int j = 1; j < BK / 16; j++) product(std::integral_constant<int, 0>(), 0, j);
                         commit_pair(empty + s);
                         commit_pair(acc_full + buf);
                     }
@@ -258,16 +275,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
 }
 
-// The leading eight significant bits of a float; what is below 2^-133 goes.  Cut off, not rounded: a large float does not become infinite, and
-// the three planes of a float have one sign.
-__device__ __forceinline__ uint32_t leading(float v) { return __float_as_uint(v) & 0xffff0000u; }
-// In place of a plane that would be zero: 2^-40 of the number (or the least there is), which no sum of floats notices.  An infinite weight then gives
-// the infinity it gives beside the number itself, and not 0 * inf.
-__device__ __forceinline__ uint32_t in_place_of_zero(uint32_t h) {
-    const uint32_t e = (h >> 23) & 255u;
-    return (h & 0x7fff0000u) == 0u || e == 255u ? h : e > 40u ? h - (40u << 23) : (h & 0x80000000u) | 0x10000u;
+// The leading eight significant bits of a float, cut off and not rounded: a large float does not become infinite, and the planes have one sign.  Where
+// nothing would be left for the next plane, one step less: no plane of a float from 2^-117 on is zero, so that an infinite weight gives the
+// infinity it gives beside the number itself, and not 0 * inf.
+__device__ __forceinline__ float leading(float v) {
+    const uint32_t bits = __float_as_uint(v), h = bits & 0xffff0000u;
+    return __uint_as_float(h == bits && (h & 0x7fff0000u) > 0x10000u ? h - 0x10000u : h);
 }
-
 // The three planes of eight neighbouring floats of a row; infinities and NaN are the same in all three.
 __global__ void __launch_bounds__(256) split_planes_kernel(const float* __restrict__ X, bf16* __restrict__ planes, int M, int K, size_t ldx, int vec) {
     ik_pdl_wait();
@@ -294,15 +308,14 @@ __global__ void __launch_bounds__(256) split_planes_kernel(const float* __restri
         #pragma unroll
         for (int e = 0; e < 2; e++) {
             const uint32_t bits = __float_as_uint(v[i + e]);
-            uint32_t h = bits & 0xffff0000u, mid = 0u, low = 0u;
             if ((bits & 0x7f800000u) != 0x7f800000u) {
-                const float r = v[i + e] - __uint_as_float(h);
-                mid = leading(r);
-                low = leading(r - __uint_as_float(mid));
-            } else if (bits & 0x7fffffu) h |= 0x400000u;               // (a NaN whose mark lies in the bits that are cut off)
-            part[e][0] = h;
-            part[e][1] = mid ? mid : in_place_of_zero(h);
-            part[e][2] = low ? low : in_place_of_zero(h);
+                const float h = leading(v[i + e]), rest = (v[i + e] - h) * (float)(1 << MID_SCALE), mid = leading(rest);
+                part[e][0] = __float_as_uint(h);
+                part[e][1] = __float_as_uint(mid);
+                part[e][2] = __float_as_uint((rest - mid) * (float)(1 << (LOW_SCALE - MID_SCALE))) & 0xffff0000u;
+            } else {                                                   // (a NaN whose mark lies in the bits that are cut off)
+                part[e][0] = part[e][1] = part[e][2] = (bits & 0xffff0000u) | ((bits & 0x7fffffu) ? 0x400000u : 0u);
+            }
         }
         #pragma unroll
         for (int p = 0; p < 3; p++) out[p][i / 2] = (part[0][p] >> 16) | part[1][p];

@@ -64,6 +64,20 @@ def test_numbers_that_are_not_finite():
     assert int(a[[3, 5]].isinf().sum()) >= 2 * 296 and bool(a[[4, 8]].isnan().all())
 
 
+def test_small_numbers():
+    """Every plane of a small number is there: the same bits as of a larger one, down to where a float itself has fewer."""
+    from ithaca_b200.csrc import ops
+    x, w = rnd((40, 512), 10), rnd((300, 512), 11, torch.bfloat16)
+    x = torch.where(x.abs() < 2.0 ** -8, torch.ones_like(x), x)
+    got = ops.gemm_split(x, w)
+    assert torch.equal(ops.gemm_split(x * 2.0 ** -110, w * 2.0 ** 60) * 2.0 ** 50, got)
+    tiny = (torch.randint(-2 ** 22, 2 ** 22, (40, 512), generator=torch.Generator().manual_seed(1)) * 2).double().to(DEV) * 2.0 ** -149
+    small = tiny.float()
+    assert torch.equal(small.double(), tiny)
+    want = tiny @ (w.double() * 2.0 ** 100).T
+    assert float((ops.gemm_split(small, w * 2.0 ** 100).double() - want).norm() / want.norm()) < 2.5e-7
+
+
 def test_dispatch():
     """The rule asks for nothing but the weight's form, so that rows do not change with the rows beside them."""
     from ithaca_b200.csrc import ops
