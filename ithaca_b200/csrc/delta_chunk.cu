@@ -18,7 +18,8 @@ namespace {
 
 constexpr int C = 64;                                    // tokens of a chunk
 constexpr int TLD = C + 4;                               // row stride of T and P in shared memory
-constexpr int VEC = 132;                                 // floats of a chunk's decays: G [64], G_end / G [64], G_end, padding
+// A chunk's floats beside T and P: G [64], G_end / G [64], G_end, padding, the diagonals of T [64] and P [64].
+constexpr int VEC_T = 132, VEC_P = VEC_T + C, VEC = VEC_P + C;
 
 // SOME: only sequences of at least `least` (> 0) tokens are walked, and their chunks numbered, in the order of the sequences.  Otherwise all
 // are, and chunk j of sequence b has the number cu_seqlens[b] / 64 + b + j (instances of their own: the walk takes 2 % longer where its
@@ -123,6 +124,7 @@ delta_chunk_prepare_kernel(const float* __restrict__ u, int ldu, int q_off, int 
     __syncthreads();
     float* const vec = vecs + ((size_t)f * H + h) * VEC;
     if (tid < C) {
+        vec[VEC_T + tid] = beta[tid];
         vec[tid] = expf((float)logs[tid]);
         vec[C + tid] = expf((float)(logs[C - 1] - logs[tid]));     // (tokens that are not there have a decay of 1)
         if (tid == 0) vec[2 * C] = expf((float)logs[C - 1]);
@@ -154,7 +156,8 @@ delta_chunk_prepare_kernel(const float* __restrict__ u, int ldu, int q_off, int 
         for (int j = 0; j < 4; j++) {
             const int t = ti + 16 * i, s = tj + 16 * j;
             const float ratio = s <= t ? expf((float)(logs[t] - logs[s])) : 0.f;
-            outP[t * C + s] = s <= t ? ratio * qk[i][j] : 0.f;
+            outP[t * C + s] = s < t ? ratio * qk[i][j] : 0.f;
+            if (s == t) vec[VEC_P + t] = qk[i][j];
             Ms[t * TLD + s] = s < t ? beta[t] * ratio * kk[i][j] : 0.f;
         }
     __syncthreads();
@@ -196,14 +199,15 @@ delta_chunk_prepare_kernel(const float* __restrict__ u, int ldu, int q_off, int 
     }
     for (int i = tid; i < C * C; i += 256) {                 // (0, not 0 * beta, above the diagonal: the walk reads whole blocks of 16)
         const int t = i / C, s = i % C;
-        outT[i] = s <= t ? Ts[t * TLD + s] * beta[s] : 0.f;
+        outT[i] = s < t ? Ts[t * TLD + s] * beta[s] : 0.f;
     }
 }
 
 // The five products of a chunk run on the tensor cores (mma.sync, bfloat16) with every float as the sum of three bfloat16 numbers, h + m + l, which
 // hold its 24 bits: h h' + (h m' + m h' + m m' + h l' + l h'), the small terms in sums of their own; what is left out is under 2^-23 of a
-// product.  Sums of the large terms leave the tensor core every 16 products and are added as floats (it drops bits towards zero).  Numbers of 3.3e38 and
-// more count as infinite, bits below 2^-133 go.
+// product.  Sums of the large terms leave the tensor core every 16 products and are added as floats (it drops bits towards zero).  What a strong decay leaves
+// of a sum, a token's own term of T (..) and P U and the last token's of K^T E, is no part of those sums: it is multiplied and added as floats, one
+// rounding to nearest.  Numbers of 3.3e38 and more count as infinite, bits below 2^-133 go.
 //
 // Everything is transposed, columns of the state first: a warp's sums [columns][tokens or keys' components] are then, lane by lane, what it has to
 // leave as the first operand of the next product, and K, Q, T and P are second operands as they lie (K once more, transposed by the load, for the state).
@@ -213,9 +217,10 @@ delta_chunk_prepare_kernel(const float* __restrict__ u, int ldu, int q_off, int 
 //
 // One block per (16 MT columns of a head, value head, walked sequence).  Bound by the tensor pipe (mma.sync takes 940 multiply-adds a cycle and SM: 6,700
 // cycles a chunk with MT = 2) and by what its latencies leave between three barriers a chunk: 13,000 cycles a chunk with MT = 2, 9,700 with MT = 1 (eight warps to bring in place of four, or a matrix asked for
-// ahead, change nothing).  Distance to 64 bits over prompts of 1,000 to 3,000 tokens: results 1.84e-7 (float products 1.95e-7), states 1.00e-7
-// (1.01e-7); with decays near one 2.0e-7 (4.6e-7) and 1.7e-7 (4.3e-7); with decays around 0.1, where a state is a few tokens' products, 2.2e-7 (2.2e-7)
-// and 8.5e-8 (3.7e-8).
+// ahead, change nothing).  Distance to 64 bits over prompts of 1,000 and 1,500 tokens, 8 heads of 128 (2-norm, results and states, float products
+// on the CUDA cores / these): decays around 0.1 2.07e-7 3.7e-8 / 2.07e-7 3.7e-8, 0.5 2.09e-7 4.7e-8 / 2.09e-7 5.1e-8, 0.8 to 1 2.32e-7 1.01e-7 / 2.15e-7
+// 0.85e-7, 0.97 2.48e-7 1.28e-7 / 2.12e-7 0.92e-7, near one 4.39e-7 4.09e-7 / 1.93e-7 1.56e-7.  (With those terms in the sums too: 2.23e-7 9.3e-8 around 0.1,
+// and 1.5 % less time.)
 template <int DK, int MT>
 struct Walk {
     static constexpr int LDK = DK + 8, LDT = C + 8;      // row strides of the planes (rows on 16 bytes, 8 of them over all banks)
@@ -224,7 +229,8 @@ struct Walk {
     static constexpr int S = P + 3 * C * LDT * 2;        // first operands: [step][plane][MT][lane] 16 bytes
     static constexpr int R = S + KS * 3 * MT * 512, U = R + 4 * 3 * MT * 512, E = U + 4 * 3 * MT * 512;
     static constexpr int FIRST = E + 4 * 3 * MT * 512;   // [16 MT] the first token of a chunk that is not finite in a column
-    static constexpr int BYTES = FIRST + 16 * MT * 4;
+    static constexpr int LAST = FIRST + 16 * MT * 4;     // [16 MT] (G_end / G) U of the chunk's last token
+    static constexpr int BYTES = LAST + 16 * MT * 4;
 };
 constexpr int MULTIPLIERS = 256, BRINGERS = 128, ALL = MULTIPLIERS + BRINGERS;
 // barriers 1 to 4: K, Q, T, P are there; 5 to 8: they have been read; 9: the multipliers among themselves
@@ -393,6 +399,7 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
 
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, pair = 2 * (lane & 3);
     int* const first = (int*)(sb + W::FIRST);
+    float* const last = (float*)(sb + W::LAST);
     if (threadIdx.x < 16 * MT) first[threadIdx.x] = C;
     const size_t per = (size_t)H * DK * dv;
     const float* const st_in = state + ((size_t)slots[b] * 2 + ((start - 1) & 1)) * per + (size_t)h * dv * DK;
@@ -412,7 +419,7 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
     const unsigned by_token = ((8 * w + (lane & 7)) * W::LDK + 8 * ((lane >> 3) & 1)) * 2, by_row = ((8 * w + (lane & 7)) * W::LDT + 8 * ((lane >> 3) & 1)) * 2;
     const unsigned by_component = ((lane & 15) * W::LDK + 8 * w * NT) * 2;
 
-    float v[MT][4], g[2], e[2], g_end;                   // this chunk's, asked for a chunk ahead
+    float v[MT][4], g[2], e[2], t_own[2], p_own[2], g_end;   // this chunk's, asked for a chunk ahead
     auto ask = [&](int j) {
         const int t0 = lo + j * C + 8 * w + pair;
         #pragma unroll
@@ -425,6 +432,8 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
         for (int c = 0; c < 2; c++) {
             g[c] = ve[8 * w + pair + c];
             e[c] = ve[C + 8 * w + pair + c];
+            t_own[c] = ve[VEC_T + 8 * w + pair + c];
+            p_own[c] = ve[VEC_P + 8 * w + pair + c];
         }
         g_end = ve[2 * C];
     };
@@ -489,7 +498,8 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
             }
             leave<MT>(sb + W::R, w, mt, lane, r);
         }
-        const float e0 = e[0], e1 = e[1], ge = g_end;
+        const float e0 = e[0], e1 = e[1], to0 = t_own[0], to1 = t_own[1], po0 = p_own[0], po1 = p_own[1], ge = g_end;
+        const int n_last = min(C, hi - lo - j * C) - 1;
         if (j + 1 < n_chunks) ask(j + 1);
         bool any = bar_any(bad);
         if (any) remember(x);
@@ -514,9 +524,13 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
                 float r[4], re[4];
                 #pragma unroll
                 for (int c = 0; c < 4; c++) {
-                    x[mt][c] = hi4[mt][c] + lo4[mt][c];
+                    x[mt][c] = fmaf((c & 1) ? to1 : to0, x[mt][c], hi4[mt][c] + lo4[mt][c]);
                     r[c] = finite(x[mt][c]);
                     re[c] = __fmul_rn((c & 1) ? e1 : e0, r[c]);
+                    if (8 * w + pair + (c & 1) == n_last) {
+                        last[column(mt, c) - col0] = re[c];
+                        re[c] = 0.f;
+                    }
                 }
                 leave<MT>(sb + W::U, w, mt, lane, r);
                 leave<MT>(sb + W::E, w, mt, lane, re);
@@ -546,7 +560,7 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
             for (int mt = 0; mt < MT; mt++)
                 #pragma unroll
                 for (int c = 0; c < 4; c++) {
-                    float o = qs[mt][c] + (hi4[mt][c] + lo4[mt][c]);
+                    float o = fmaf((c & 1) ? po1 : po0, x[mt][c], qs[mt][c] + (hi4[mt][c] + lo4[mt][c]));
                     if (any && 8 * w + pair + (c & 1) >= first[column(mt, c) - col0]) o = CUDART_NAN_F;
                     if (t0 + (c & 1) < hi && column(mt, c) < dv) out[(size_t)(t0 + (c & 1)) * H * dv + (size_t)h * dv + column(mt, c)] = o;
                 }
@@ -566,6 +580,19 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
                     mma_planes<MT>(hi4[i], lo4[i], a, kb);
                 }
             }
+            float k_last[NT][2], u_last[MT][2];              // the last token's key (its planes' sum is the float) and (G_end / G) U
+            #pragma unroll
+            for (int i = 0; i < NT; i++) {
+                const char* at = sb + W::K + (n_last * W::LDK + 8 * (w * NT + i) + pair) * 2;
+                const unsigned h = *reinterpret_cast<const unsigned*>(at), m = *reinterpret_cast<const unsigned*>(at + C * W::LDK * 2),
+                               l = *reinterpret_cast<const unsigned*>(at + 2 * C * W::LDK * 2);
+                k_last[i][0] = __uint_as_float(h << 16) + (__uint_as_float(m << 16) + __uint_as_float(l << 16));
+                k_last[i][1] = __uint_as_float(h & 0xffff0000u) + (__uint_as_float(m & 0xffff0000u) + __uint_as_float(l & 0xffff0000u));
+            }
+            #pragma unroll
+            for (int mt = 0; mt < MT; mt++)
+                #pragma unroll
+                for (int c = 0; c < 2; c++) u_last[mt][c] = last[16 * mt + row + 8 * c];
             if (j + 1 < n_chunks) bar_arrive(5);
             #pragma unroll
             for (int i = 0; i < NT; i++)
@@ -573,7 +600,7 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
                 for (int mt = 0; mt < MT; mt++)
                     #pragma unroll
                     for (int c = 0; c < 4; c++) {
-                        S[i][mt][c] = fmaf(ge, S[i][mt][c], hi4[i][mt][c] + lo4[i][mt][c]);
+                        S[i][mt][c] = fmaf(k_last[i][c & 1], u_last[mt][c >> 1], fmaf(ge, S[i][mt][c], hi4[i][mt][c] + lo4[i][mt][c]));
                         if (any && first[column(mt, c) - col0] < C) S[i][mt][c] = CUDART_NAN_F;
                     }
         }

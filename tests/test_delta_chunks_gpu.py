@@ -102,3 +102,25 @@ def test_columns_beside_one_that_is_not_finite(H, G, dk, dv):
     assert not torch.isfinite(state1[slots[0], p, H - 1, 19]).any()
     state1[slots[0], p, H - 1, 19] = state[slots[0], p, H - 1, 19]
     assert torch.equal(state1, state)
+
+
+@pytest.mark.parametrize("decay", [0.01, 0.1])
+def test_strong_decays(decay):
+    """A state that is a few tokens' products is not further from 64 bits than token by token."""
+    from ithaca_b200.csrc import ops
+    H, G, dk, dv, T = 4, 2, 128, 128, 360
+    u, bg, before, ctx, cu, slots = make(H, G, dk, dv, [T], [0], 7, "usual")
+    bg[:, 1] = decay * (0.8 + 0.4 * torch.rand((T, H), generator=torch.Generator(device=DEV).manual_seed(1), device=DEV))
+    made = []
+    for chunks in (True, False):
+        state = before.clone()
+        ops.delta_rule(u, 4, 4 + G * dk, 4 + 2 * G * dk, bg, state, ctx, H, G, dk, dv, chunks=chunks)
+        made.append(state[slots[0], 1])
+    S = torch.zeros(H, dv, dk, dtype=torch.float64, device=DEV)
+    for t in range(T):
+        k = u[t, 4 + G * dk:4 + 2 * G * dk].double().view(G, dk).repeat_interleave(H // G, 0)
+        S = S * bg[t, 1].double()[:, None, None]
+        x = bg[t, 0].double()[:, None] * (u[t, 4 + 2 * G * dk:].double().view(H, dv) - torch.einsum("hvk,hk->hv", S, k))
+        S = S + x[:, :, None] * k[:, None, :]
+    # about four roundings to nearest of terms that are hardly ever as large as the sum: 2 * 2^-24 / sqrt(3)
+    assert far(made[0], S) < 6e-8 and far(made[0], S) < far(made[1], S)
