@@ -228,7 +228,7 @@ struct Walk {
     static constexpr int K = 0, Q = K + 3 * C * LDK * 2, T = Q + 3 * C * LDK * 2, P = T + 3 * C * LDT * 2;
     static constexpr int S = P + 3 * C * LDT * 2;        // first operands: [step][plane][MT][lane] 16 bytes
     static constexpr int R = S + KS * 3 * MT * 512, U = R + 4 * 3 * MT * 512, E = U + 4 * 3 * MT * 512;
-    static constexpr int FIRST = E + 4 * 3 * MT * 512;   // [16 MT] the first token of a chunk that is not finite in a column
+    static constexpr int FIRST = E + 4 * 3 * MT * 512;   // [16 MT] the first token of a chunk that is not finite in a column (C: none)
     static constexpr int LAST = FIRST + 16 * MT * 4;     // [16 MT] (G_end / G) U of the chunk's last token
     static constexpr int BYTES = LAST + 16 * MT * 4;
 };
@@ -472,8 +472,8 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
                 for (int c = 0; c < 4; c++) { ks[mt][c] += klo[mt][c]; qs[mt][c] = __fmul_rn(g[c & 1], qs[mt][c] + qlo[mt][c]); }
             if (j + 1 < n_chunks) bar_arrive(6);
         }
-        // V - G (K S).  What is not finite must not meet the zeros of earlier tokens' rows in a product: it goes in as 0, and from its token on the
-        // column's results, and its state, are NaN.
+        // V - G (K S).  What is not finite must not meet the zeros of earlier tokens' rows in a product: it goes in as 0.  Its own token's results, and
+        // the state if that is the last token, have its terms apart; behind its token the column's results and its state are NaN.
         bool bad = false;
         float x[MT][4];
         auto finite = [&](float& r) {
@@ -528,7 +528,7 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
                     r[c] = finite(x[mt][c]);
                     re[c] = __fmul_rn((c & 1) ? e1 : e0, r[c]);
                     if (8 * w + pair + (c & 1) == n_last) {
-                        last[column(mt, c) - col0] = re[c];
+                        last[column(mt, c) - col0] = __fmul_rn((c & 1) ? e1 : e0, x[mt][c]);
                         re[c] = 0.f;
                     }
                 }
@@ -561,7 +561,7 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
                 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     float o = fmaf((c & 1) ? po1 : po0, x[mt][c], qs[mt][c] + (hi4[mt][c] + lo4[mt][c]));
-                    if (any && 8 * w + pair + (c & 1) >= first[column(mt, c) - col0]) o = CUDART_NAN_F;
+                    if (any && 8 * w + pair + (c & 1) > first[column(mt, c) - col0]) o = CUDART_NAN_F;
                     if (t0 + (c & 1) < hi && column(mt, c) < dv) out[(size_t)(t0 + (c & 1)) * H * dv + (size_t)h * dv + column(mt, c)] = o;
                 }
         }
@@ -601,7 +601,7 @@ delta_chunk_kernel(const float* __restrict__ u, int ldu, int q_off, int k_off, i
                     #pragma unroll
                     for (int c = 0; c < 4; c++) {
                         S[i][mt][c] = fmaf(k_last[i][c & 1], u_last[mt][c >> 1], fmaf(ge, S[i][mt][c], hi4[i][mt][c] + lo4[i][mt][c]));
-                        if (any && first[column(mt, c) - col0] < C) S[i][mt][c] = CUDART_NAN_F;
+                        if (any && first[column(mt, c) - col0] < n_last) S[i][mt][c] = CUDART_NAN_F;
                     }
         }
         if (j + 1 < n_chunks) {

@@ -104,6 +104,25 @@ def test_columns_beside_one_that_is_not_finite(H, G, dk, dv):
     assert torch.equal(state1, state)
 
 
+@pytest.mark.parametrize("at", [77, 127, 149])                    # within a chunk, a chunk's last token, the prompt's
+@pytest.mark.parametrize("what", [float("inf"), float("-inf"), float("nan")])
+def test_an_infinity_is_what_it_is_token_by_token(at, what):
+    """Its own token's results, and the state behind the last token, stay infinite; later ones are NaN."""
+    from ithaca_b200.csrc import ops
+    H, G, dk, dv = 2, 1, 128, 64
+    u, bg, before, ctx, cu, slots = make(H, G, dk, dv, [150], [0], 3, "usual")
+    col = dv + 5
+    u[at, 4 + 2 * G * dk + col] = what
+    made = []
+    for chunks in (True, False):
+        state = before.clone()
+        o = ops.delta_rule(u, 4, 4 + G * dk, 4 + 2 * G * dk, bg, state, ctx, H, G, dk, dv, chunks=chunks)
+        made.append((o[at:, col], state[slots[0], 1, 1, 5]))
+    for got, want in zip(*made):
+        assert not torch.isfinite(want).any()
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got == float("inf"), want == float("inf")) and torch.equal(got.isinf(), want.isinf())
+
+
 @pytest.mark.parametrize("decay", [0.01, 0.1])
 def test_strong_decays(decay):
     """A state that is a few tokens' products is not further from 64 bits than token by token."""
