@@ -405,8 +405,9 @@ def split_takes(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch
 def gemm_split(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False,
                status: Optional[torch.Tensor] = None, tile: int = 0, side_by_side: bool = False) -> torch.Tensor:
     """out[M, N] (+)= x[M, K] @ w[N, K]^T, x and out float32, w bfloat16: x as three bfloat16 numbers on the tensor cores, sums of
-    128 products there, the rest in float registers.  ``tile``: tokens of a tile (32, 64, 128; 0 = chosen, with whether the slices of K run
-    ``side_by_side``): the same bits every way."""
+    64 k there, the rest in float registers.  ``tile``: tokens of a tile (32, 64, 128, 256; 0 = chosen, with whether the slices of K run
+    ``side_by_side``): the same bits every way.  The first tiles of ``w`` are asked for before x's planes are there, but
+    after every kernel before the call has finished (the kernel that forms the planes has waited for it)."""
     _need(x, "x", torch.float32, contiguous=False)
     _need(w, "w", torch.bfloat16, contiguous=False)
     M, K = x.shape
@@ -520,7 +521,9 @@ def tcgen05_splits(M: int, N: int, K: int) -> int:
     -n = clusters of n blocks per tile, each a slice of K, summed in shared memory (no scratch, one kernel).
     Measured on B200 with 2048 x 2048 .. 28672 x 4096 weights (``bench.py --only products --tokens ...``): with
     fewer tiles than half the SMs, K is sliced: by clusters of 2 or 4 where that busies at least half the SMs (clusters
-    of 3 measured far slower), else by a second kernel; stream-K wins when whole tiles would leave more than a
+    of 3 measured far slower), else by a second kernel.  (The shapes for which clusters were the best way all go to gemm_batch.cu now, which does the same
+    on pairs of SMs and shares the epilogue out: of what is left to this rule on 148 SMs none gets them, and they run only where a caller asks for
+    them.)  Stream-K wins when whole tiles would leave more than a
     tenth of the SMs' time unused and there is one token tile of at most 128 tokens (bandwidth-bound); beyond that
     whole tiles win."""
     N_SM = sm_count()
@@ -546,7 +549,7 @@ def wide_takes(M: int, N: int, K: int) -> bool:
     the pairs busy with its narrowest tiles of 256 tokens x 128 features.  Measured on B200, other kernel / this one
     (us): 36 tiles' worth and more: 4096 x 4096 at 300 tokens 20.0 / 19.1, 28672 x 4096 at 200 80 / 60, 16384 x 2048 at
     130 29 / 23, 4096 x 14336 at 512 67 / 58, 2048 x 8192 at 768 34 / 32; below: 6144 x 4096 at 130 17.5 / 20.1, 4096 x 14336 at 256
-    49 / 57, 2048 x 8192 at 512 27.5 / 30.5.  Up to 128 tokens the other kernel's slices of K win.  With few K steps a tile is mostly
+    49 / 57, 2048 x 8192 at 512 27.5 / 30.5.  Up to 128 tokens see ``batch_takes``.  With few K steps a tile is mostly
     its start and its epilogue, and a second tile of 256 tokens for a few of them does not pay: 8192 x 256 at 192 tokens 6.6 / 7.8, at 257
     7.4 / 8.5, at 400 8.7 / 8.0; 8192 x 512 at 257 8.7 / 9.3, at 400 10.0 / 9.4."""
     return M > 128 and M * N >= 36 * 256 * 128 and (K >= 1024 or M > 300)
@@ -575,15 +578,25 @@ def pairs_lib():
 
 def batch_takes(M: int, N: int, K: int) -> bool:
     """Whether a product of up to 128 tokens runs on gemm_batch.cu (no scratch, one kernel) rather than in one of the ways of gemm_tcgen05.cu (``tcgen05_splits``).
-    Two kinds of matrix stay behind (us on B200, those ways / this): few features with a long K, which nine slices and a second kernel keep
-    more SMs busy on (2048 x 8192 for 17 tokens 11.4 / 13.6, 48 12.8 / 13.7, 64 13.9 / 13.7, 65 14.5 / 15.9, 100 17.1 / 15.9), and a few tokens by very many features, where equal
-    shares of K steps spare the last of several rounds (128256 x 2048 for 24 tokens 82.7 / 84.4, 64 86.7 / 87.6, 100 94 / 90)."""
+    Two kinds of matrix stay behind.  Few features with a long K: seven or more slices of it and a second kernel keep more SMs busy than four slices do, as long as the
+    slices' sums (tokens x features x slices) are few.  Both times are estimated in us, from K steps a block, sums and tiles, fitted on B200 to 26 matrices (128
+    to 2,560 features, K of 4,096 to 16,384) at up to 17 numbers of tokens each: the estimate picks the faster way to 0.2 % on average, 6 % at worst.  Those ways /
+    this: 2048 x 8192 for 17 tokens 11.8 / 14.0, 56 13.9 / 14.1, 64 14.2 / 14.1, 65 14.9 / 16.4, 96 16.9 / 16.4; 768 x 16384 17 13.5 / 19.5, 128 17.9 / 22.6;
+    1024 x 4096 24 9.7 / 9.0, 65 12.3 / 11.0.  And up to 64 tokens by very many features with a short K: whole tiles, one an SM, where they fill the last round too (128256 x
+    2048 for 24 tokens 84.6 / 88.1, 64 88.9 / 90.0, 65 90.8 / 89.0; 128256 x 4096 165.7 / 165.2, 179 / 175; 96000 x 2048, which leaves a sixth of its rounds idle, 69.8 / 68.6, 75 / 69)."""
     if M > 128:
         return False
     n_sm = sm_count()
-    if K >= 4096 and K >= 3 * N and 8 * -(-N // 128) <= n_sm and (M <= 48 or 64 < M <= 80):
-        return False
-    return not (M <= 64 and -(-N // 256) >= 4 * (n_sm // 2))
+    tiles, steps = -(-N // 128), -(-K // 64)
+    slices = min(n_sm // tiles, steps // 4)
+    if steps >= 64 and slices >= (8 if M <= 64 else 7):
+        own, four, sums = -(-steps // slices), -(-steps // 4), M * tiles * slices
+        if M <= 64:
+            other, here = 3.89 + 0.37 * own + 1.78e-4 * sums + 0.17 * slices + 0.029 * M, 4.64 + 0.228 * four + 0.13 * tiles
+        else:
+            other, here = 3.9 + 0.43 * own + 0.88e-4 * sums + 0.13 * slices + 0.044 * M, 5.94 + 0.262 * four + 0.142 * tiles
+        return here <= other
+    return not (M <= 64 and steps < 64 and tiles >= 8 * (n_sm // 2) and tiles >= 0.9 * n_sm * -(-tiles // n_sm))
 
 
 def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, out_dtype=torch.float32,

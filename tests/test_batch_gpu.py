@@ -98,7 +98,10 @@ def test_what_it_refuses():
 # measured on B200: tokens, features, K, us in the ways of gemm_tcgen05.cu, us here
 @pytest.mark.parametrize("M,N,K,other,here", [(17, 28672, 4096, 43.5, 41.2), (64, 4096, 4096, 17.0, 11.5), (128, 6144, 4096, 26.6, 15.8), (17, 2048, 8192, 11.4, 13.6),
                                               (48, 2048, 8192, 12.8, 13.7), (100, 2048, 8192, 17.1, 15.9), (24, 1536, 6144, 9.7, 11.1), (24, 128256, 2048, 82.7, 84.4),
-                                              (100, 128256, 2048, 94.1, 90.3), (65, 1024, 512, 8.8, 5.1)])
+                                              (100, 128256, 2048, 94.1, 90.3), (65, 1024, 512, 8.8, 5.1),
+                                              (80, 2048, 8192, 16.0, 16.4), (104, 2048, 8192, 17.7, 16.4), (96, 768, 16384, 16.4, 22.5), (64, 2048, 16384, 20.1, 21.8), (17, 2304, 6144, 10.9, 12.6),
+                                              (104, 1280, 10240, 16.0, 17.4), (40, 1024, 4096, 10.7, 9.0), (80, 512, 4096, 11.3, 11.0), (65, 2560, 16384, 25.0, 26.9), (65, 3072, 16384, 28.5, 28.1),
+                                              (48, 2560, 10240, 20.2, 16.7), (64, 128256, 4096, 179.2, 174.6), (32, 96000, 2048, 69.9, 66.2)])
 def test_products_take_the_faster_way(M, N, K, other, here, monkeypatch):
     from ithaca_b200.csrc import ops
     monkeypatch.setattr(ops, "sm_count", lambda: 148)
