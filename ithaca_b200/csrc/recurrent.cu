@@ -581,9 +581,10 @@ selective_scan_stream_kernel(const __nv_bfloat16* __restrict__ u, const float* _
             float* tile = sm + (j & 3) * Tile::FLOATS;       // (free: the results of tile j - 4 have been read, by this team)
             if (mine) {
                 const bool there = lo + j * TT + tt < hi;
+                if (!there) r.u = make_uint2(0u, 0u);
                 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    const float x = there ? __uint_as_float(((i & 1) ? (i < 2 ? r.u.x : r.u.y) & 0xffff0000u : (i < 2 ? r.u.x : r.u.y) << 16)) : 0.f;
+                    const float x = __uint_as_float(((i & 1) ? (i < 2 ? r.u.x : r.u.y) & 0xffff0000u : (i < 2 ? r.u.x : r.u.y) << 16));
                     const float dt = there ? ik_softplus_as<true>((&r.d.x)[i] + bias[i]) : 0.f;
                     *reinterpret_cast<float2*>(tile + Tile::place(tt, tid % QC, i)) = make_float2(dt, dt * x);
                     *reinterpret_cast<float2*>(tile + Tile::XG + Tile::place(tt, tid % QC, i)) = make_float2(x, ik_silu_as<true>((&r.z.x)[i]));
@@ -614,10 +615,8 @@ selective_scan_stream_kernel(const __nv_bfloat16* __restrict__ u, const float* _
             #pragma unroll
             for (int i = 0; i < 2; i++) {
                 const int n = 4 * l + 2 * r + i;
-                e[i] = n < N ? A[(size_t)cc * N + n] * 1.44269504f : 0.f;
-                // (an infinite A: a step size of 0 still leaves the state alone; NaN stays)
-                asm("max.NaN.f32 %0, %0, %1;" : "+f"(e[i]) : "f"(-3.4e38f));
-                asm("min.NaN.f32 %0, %0, %1;" : "+f"(e[i]) : "f"(3.4e38f));
+                const float p = n < N ? A[(size_t)cc * N + n] * 1.44269504f : 0.f;
+                e[i] = p < -3.4e38f ? -3.4e38f : p;          // (an A of minus infinity: a step size of 0 still leaves the state alone; NaN stays)
                 s[i] = n < N && start > 0 ? st_in[n] : 0.f;
             }
             S[r] = ik_pack2(s[0], s[1]);
