@@ -36,6 +36,12 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k_p
     int* const row_pos = (int*)(factor + ROWS);               // [ROWS] position, -1: a row that is not there
     size_t* const place = (size_t*)(row_pos + ROWS);          // [TILE] row of key j in the pages (page, kv head, place)
     ik_pdl_wait();
+    IK_AFTER_WAIT(q);
+    IK_AFTER_WAIT(k_pages);
+    IK_AFTER_WAIT(v_pages);
+    IK_AFTER_WAIT(token_seq);
+    IK_AFTER_WAIT(token_pos);
+    IK_AFTER_WAIT(table);
     ik_pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tx = tid & 15, ty = tid >> 4;
     const int tokens = ROWS / heads, t0 = blockIdx.x * tokens, h0 = blockIdx.y * heads, kvh = h0 / (nh / nkv);

@@ -135,16 +135,16 @@ __device__ __forceinline__ float ik_block_max(float v, float* scratch) {
 //     the bandwidth-bound products, the first batch of WEIGHTS, which no kernel writes.  So a product launched
 //     early has its first 128 KB per SM on the way while the kernel before it is still finishing.
 //   * ik_pdl_launch_dependents() comes AFTER the kernel's own wait (so at most two kernels are ever on the
-//     device: this one and the one after it) and as late as is useful: small kernels call it right after the
-//     wait (the product behind a norm starts at once and loads weights while the norm runs); the products and
-//     decode attention call it after their main loop (their successor takes the SM slots that their finishing
+//     device: this one and the one after it).  Small kernels and the tcgen05 products call it right after the wait (the
+//     product behind a norm starts at once and loads weights while the norm runs; a tcgen05 product's blocks fill their SMs, so its successor
+//     starts where they end whenever it is called: after the main loop instead, a layer's products of 32 to 128 tokens took the same to 0.3 %);
+//     the skinny products and decode attention call it after their main loop (their successor takes the SM slots that their finishing
 //     blocks free, and does not compete with blocks that have not started yet).
 //   * what the kernel before has written is read with ordinary loads AFTER the wait.  A read-only load
 //     (__ldg, or a plain load through a `const __restrict__` pointer) is not enough: the compiler takes it for a
-//     read of constant memory and may move it to before the wait.  The skinny product, the one family that is
-//     launched early by default, reads its tokens with an explicit ld.global for that reason (with __ldg its
-//     results were wrong under graph replay); the element-wise kernels pass their input pointers through
-//     IK_AFTER_WAIT.
+//     read of constant memory and may move it to before the wait.  The skinny product reads its tokens with an explicit
+//     ld.global for that reason (with __ldg its results were wrong under graph replay); the others pass their input
+//     pointers through IK_AFTER_WAIT, bring them by TMA, or are of a family that is not launched early.
 // IK_PDL=<mask of kernel families> chooses which launches get the attribute (0 = none: kernels start strictly
 // one after another and the device-side calls are no-ops).  Default: the products (skinny and tcgen05) and the
 // element-wise kernels.  Measured on the graph-replayed decode step of the 8B shape: skinny products 1.1 % faster,

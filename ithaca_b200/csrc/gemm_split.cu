@@ -389,7 +389,7 @@ void cut(int K, int& nkb, int& per, int& slices) {
 struct Plan { int bn, side_by_side; };
 
 // Tokens of a tile, and whether the slices of K run side by side (with a second kernel that adds them): what takes the least time in
-// whole rounds over the pairs of SMs.  Nanoseconds a K step, all SMs at work (measured): STEP_TIMES.
+// whole rounds over the pairs of SMs.  Nanoseconds a K step with all SMs at work, measured: 1,150 with 256 tokens a tile, 580 with 128, 365 with 64, 300 with 32.
 Plan plan(int M, int N, int K, int pairs) {
     int nkb, per, slices;
     cut(K, nkb, per, slices);
