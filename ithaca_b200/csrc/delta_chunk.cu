@@ -8,9 +8,9 @@
 // a slice of a head's columns per block: five small products a chunk in place of 64 dependent steps.  The tokens' chain is what
 // bounds the token-by-token kernel (0.37 to 0.4 us a token; which sequences of a step go which way: ops.delta_chunks_from); the chunks' chain is
 // bound by the walk's products and the latencies between them.
-// Measured on B200: a layer 2,048 wide with 16 heads of 128 over two prompts of 3,000 and 1,910 tokens 2,776 us token by token; T and P 78 us, and the walk
-// 505 us (10.7 us a chunk) with float products on the CUDA cores, which read half of 16 bytes from shared memory per four multiply-adds, against 329 us
-// (7 us a chunk) on the tensor cores.
+// Measured on B200, 16 heads of 128 over two prompts of 3,000 and 1,910 tokens: token by token 2,776 us (the layer), in chunks 624 us with the walk's float
+// products on the CUDA cores, which read half of 16 bytes from shared memory per four multiply-adds, and 450 us with these on the tensor cores: 82 us for T
+// and P, 7.8 us a chunk for the walk.
 #include <math_constants.h>
 #include "common.cuh"
 
@@ -215,12 +215,13 @@ delta_chunk_prepare_kernel(const float* __restrict__ u, int ldu, int q_off, int 
 // state (DK / 8 components each, floats in registers); its planes and those of V - G (K S) and of U pass through shared memory.  Four more
 // warps bring the next chunk's K, Q, T and P as planes: they hold them in registers until the place is free.
 //
-// One block per (16 MT columns of a head, value head, walked sequence).  Bound by the tensor pipe (mma.sync takes 940 multiply-adds a cycle and SM: 6,700
-// cycles a chunk with MT = 2) and by what its latencies leave between three barriers a chunk: 13,000 cycles a chunk with MT = 2, 9,700 with MT = 1 (eight warps to bring in place of four, or a matrix asked for
+// One block per (16 MT columns of a head, value head, walked sequence).  Bound by what its latencies leave between three barriers a chunk, then by the tensor
+// pipe: about 14,000 cycles a chunk with MT = 2, of which counters show the pipe at work for 5,600 (2 cycles an instruction and SM) and 31 % of the issue slots
+// taken; a quarter fewer with MT = 1 (eight warps to bring in place of four, or a matrix asked for
 // ahead, change nothing).  Distance to 64 bits over prompts of 1,000 and 1,500 tokens, 8 heads of 128 (2-norm, results and states, float products
 // on the CUDA cores / these): decays around 0.1 2.07e-7 3.7e-8 / 2.07e-7 3.7e-8, 0.5 2.09e-7 4.7e-8 / 2.09e-7 5.1e-8, 0.8 to 1 2.32e-7 1.01e-7 / 2.15e-7
 // 0.85e-7, 0.97 2.48e-7 1.28e-7 / 2.12e-7 0.92e-7, near one 4.39e-7 4.09e-7 / 1.93e-7 1.56e-7.  (With those terms in the sums too: 2.23e-7 9.3e-8 around 0.1,
-// and 1.5 % less time.)
+// and 1 % less time.)
 template <int DK, int MT>
 struct Walk {
     static constexpr int LDK = DK + 8, LDT = C + 8;      // row strides of the planes (rows on 16 bytes, 8 of them over all banks)

@@ -18,7 +18,8 @@
 // holds 128 rows of W (TMEM lanes) and half of the tokens' rows of the three planes.  A stage of 64 k brings 16 KB of W and 192 bytes a
 // token into a block for 12 products: W is read once for the three planes.  Lanes are features, so a warp stores 32
 // neighbouring features of a token at a time.
-// What bounds it: with many tokens the tensor pipe (three times the operations of a 16-bit product), with few the bytes of W and the start.
+// What bounds it: with many tokens the tensor pipe (three times the operations of a 16-bit product; at work 86 % of the cycles with 2,048 tokens x 16384 x
+// 2048), with few the bytes of W and the start.
 // Measured on B200 (us in replayed graphs, with the kernels that form the planes and add the slices; gemm_simt.cu / this): 2,048 tokens x 16384 x
 // 2048 2,446 / 276 (498 TFLOP/s), 2048 x 8192 1,443 / 179; 465 tokens 737 / 76, 475 / 47; 1 token 177 / 15, 302 / 17; 128256 x 2048 for 3 tokens 861 / 84.
 #include <type_traits>

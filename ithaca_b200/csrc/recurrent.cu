@@ -457,7 +457,7 @@ selective_scan_kernel(const TU* __restrict__ u, const float* __restrict__ dt_raw
 // results of the tile before; the four last warps do nothing but the recurrence, a thread four states of a channel, L lanes a channel, CH channels a
 // block, two states per instruction where the hardware has one (mul and fma of f32x2).  So neither waits for the other's latency: a token
 // takes 40 ns with a block to an SM, and with more the reads from shared memory (10 to 14 cycles a warp and token), the exponentials (four a
-// cycle and scheduler) and the issue slots bind about evenly.  Tokens that are not there have a step size and an
+// cycle and scheduler) and the issue slots bind about evenly (counters, 1,000 + 640 tokens, 4,096 channels of 16 states: 53, 61 and 54 %).  Tokens that are not there have a step size and an
 // input of 0: a factor of 1 and nothing added.
 // Measured on B200, 4,096 channels of 16 states (us, the kernel above / this): one prompt of 200 25 / 10, of 3,000 341 / 125, 3,000 + 1,910 399 / 193,
 // eight of 2,000 790 / 437.  One team alone took 231 for 3,000 + 1,910 (a tile's softplus, gates and stores are 225 instructions of one
