@@ -8,9 +8,9 @@
 // a slice of a head's columns per block: five small products a chunk in place of 64 dependent steps.  The tokens' chain is what
 // bounds the token-by-token kernel (0.37 to 0.4 us a token; which sequences of a step go which way: ops.delta_chunks_from); the chunks' chain is
 // bound by the walk's products and the latencies between them.
-// Measured on B200, 16 heads of 128 over two prompts of 3,000 and 1,910 tokens: token by token 2,776 us (the layer), in chunks 624 us with the walk's float
-// products on the CUDA cores, which read half of 16 bytes from shared memory per four multiply-adds, and 450 us with these on the tensor cores: 82 us for T
-// and P, 7.8 us a chunk for the walk.
+// Measured on B200, 16 heads of 128 over two prompts of 3,000 and 1,910 tokens: token by token 2,776 us (the layer), in chunks 594 us with the walk's float
+// products on the CUDA cores, which read half of 16 bytes from shared memory per four multiply-adds, and 424 us with these on the tensor cores: 80 us for T
+// and P, 7.4 us a chunk for the walk.
 #include <math_constants.h>
 #include "common.cuh"
 
